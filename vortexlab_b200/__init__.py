@@ -649,6 +649,8 @@ class Sim:
 
     @schedule.setter
     def schedule(self, name: str):
+        """Launches every step by this schedule. Until one is chosen (and after ``autotune``), calls of
+        a few steps and more on a small domain run in one kernel for all their steps instead."""
         check(lib.vl_sim_set_schedule(self._h, self.SCHEDULES[name]))
 
     def set_cells_per_thread(self, cells: int):

@@ -15,6 +15,7 @@
 #include "vl_host.hpp"
 #include "vl_internal.hpp"
 #include "vl_launch.hpp"
+#include "vl_resident.cuh"
 
 struct vl_builder {
   vl::DomainSpec spec;
@@ -49,6 +50,8 @@ vl_shape* wrap_shape(std::unique_ptr<vl::Shape> s) {
 
 constexpr int kGraphSteps = 32;  // steps per captured CUDA graph (even: buffer parity returns)
 constexpr int kReduceBlocks = 296;
+constexpr uint64_t kResidentMinSteps = 4;     // fewer steps: the start (outlet velocities, own populations) costs more than it saves
+constexpr uint64_t kResidentMaxSteps = 4096;  // per launch
 
 }  // namespace
 
@@ -98,6 +101,17 @@ struct vl_sim {
   // kernel on one stream, 2 bulk then link, 3 staged (link values, then the bulk kernel that also
   // updates boundary cells; one stream).
   int schedule = 0;
+  // Small domains (resident_setup): calls of at least kResidentMinSteps steps run in the resident
+  // kernel (vl_resident.cuh) unless a schedule was chosen by name.
+  bool resident_ok = false;        // the domain is one the kernel takes
+  bool resident = true;            // no schedule was chosen by name
+  int res_v = 0;                   // cells per thread that the segment table was made for
+  vl::ResidentParams RP{};
+  int32_t* d_res_seg = nullptr;    // one of them: the segment table
+  std::vector<int32_t> res_task_first, res_outlets;   // first task / outlet tasks of each block
+  // device tables and buffers of the kernel (ResidentParams), one allocation each
+  std::vector<void*> d_res;
+  unsigned res_arrived = 0;        // arrivals of every launch so far
   uint64_t t_host = 0;
   uint64_t rec_start = 0, rec_cap = 0;
   bool timed = false;
@@ -109,6 +123,7 @@ struct vl_sim {
     if (gexec) cudaGraphExecDestroy(gexec);
     void* ptrs[] = {buf[0], buf[1], d_flag, d_bidx, d_bfirst, d_links, d_pidx, d_pn, d_ctl,
                     d_partials, d_hist, d_sched, d_red, d_cells, d_gather, d_bdesc, d_wbfirst, d_lb, d_ownc, d_lnode};
+    for (void* p : d_res) cudaFree(p);
     for (void* p : ptrs)
       if (p) cudaFree(p);
     for (cudaEvent_t e : pev) cudaEventDestroy(e);
@@ -131,6 +146,7 @@ struct vl_sim {
   int pull_ctl() {
     VL_CUDA(cudaMemcpyAsync(&hctl, d_ctl, sizeof(vl::Ctl), cudaMemcpyDeviceToHost, stream));
     VL_CUDA(cudaStreamSynchronize(stream));
+    if (hctl.stalled) return fail(VL_ECUDA, "resident step kernel: a block gave up waiting for the others");
     return VL_OK;
   }
 
@@ -237,6 +253,7 @@ struct vl_sim {
   }
 
   int set_schedule(int sc) {
+    resident = false;
     if (sc < 0 || sc >= VL_SCHEDULE_COUNT) return fail(VL_EINVAL, "schedule must be 0, 1, 2 or 3");
     if (sc != schedule && gexec) {
       VL_CUDA(cudaStreamSynchronize(stream));
@@ -283,7 +300,9 @@ struct vl_sim {
     hctl.dry = 0;
     if ((rc = push_ctl())) return rc;
     schedule = -1;
-    return set_schedule(best_sc);
+    rc = set_schedule(best_sc);
+    resident = true;
+    return rc;
   }
 
   // The pressure probe of step t is evaluated during step t + 1; the last step of a batch gets
@@ -339,8 +358,82 @@ struct vl_sim {
     return VL_OK;
   }
 
+  // The row segments of each block of the resident kernel. A block's boundary tasks and the last
+  // block's force sums keep some of its warps busy; they are counted in segments, so that all blocks
+  // finish a step together.
+  int resident_tables() {
+    const int v = L->resident_width(P, ck);
+    if (res_v == v) return VL_OK;
+    int sms = 0;
+    VL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    const int per_row = (P.nx + 32 * v - 1) / (32 * v);
+    const long long nseg = (long long)per_row * P.ny;
+    const int G = RP.grid;
+    if (L->resident_blocks(P, RP, ck, sms) < G || nseg > 0x7fffffff) { resident_ok = false; return VL_OK; }
+    // Segments that a task, an outlet node's place in the serial sum, the force sums and a chunk of them
+    // stand for (a segment is about 150 cycles of a block). Half and twice these move a step by 3 % at
+    // most on tunnels of D = 24, 37 and 60 and the rig at 20 and 80 cells per diameter.
+    const double task_segs = 3.0, outlet_segs = 0.1, sum_segs = 16.0, chunk_segs = 2.0;
+    std::vector<double> duty(G, 0.0);
+    for (int g = 0; g < G; ++g) duty[g] = task_segs * (res_task_first[g + 1] - res_task_first[g]);
+    for (int g = 0; g < G; ++g)
+      if (res_outlets[g] > 0) duty[g] += outlet_segs * P.np;
+    duty[G - 1] += sum_segs + chunk_segs * RP.nforce;
+    // the common number of segments' time T: sum of max(0, T - duty) = nseg
+    double lo = 0.0, hi = (double)nseg;
+    for (double d : duty) hi += d;
+    for (int it = 0; it < 80; ++it) {
+      const double T = 0.5 * (lo + hi);
+      double sum = 0.0;
+      for (double d : duty) sum += std::max(0.0, T - d);
+      (sum >= (double)nseg ? hi : lo) = T;
+    }
+    std::vector<int32_t> first(G + 1, 0);
+    double at = 0.0;
+    for (int g = 0; g < G; ++g) {
+      at += std::max(0.0, hi - duty[g]);
+      first[g + 1] = (int32_t)std::min<double>((double)nseg, std::floor(at + 0.5));
+    }
+    first[G] = (int32_t)nseg;
+    VL_CUDA(cudaStreamSynchronize(stream));
+    VL_CUDA(cudaMemcpy(d_res_seg, first.data(), first.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+    RP.segs_per_row = per_row;
+    res_v = v;
+    return VL_OK;
+  }
+
+  // Steps in the resident kernel, a bounded number per launch. `done`: false when it cannot run here.
+  int step_resident(uint64_t steps, bool& done) {
+    done = false;
+    if (int rc = resident_tables()) return rc;
+    if (!resident_ok) return VL_OK;
+    VL_CUDA(cudaEventRecord(ev0, stream));
+    uint64_t left = steps;
+    while (left > 0) {
+      RP.steps = (int)std::min<uint64_t>(left, kResidentMaxSteps);
+      RP.arrived0 = res_arrived;
+      cudaError_t e = L->resident(P, RP, ck, buf[cur], buf[cur ^ 1], stream);
+      if (e != cudaSuccess) return cuda_fail(e, "resident step kernel");
+      res_arrived += (unsigned)(RP.steps + 1) * (unsigned)RP.grid;
+      launches += 1;
+      cur ^= RP.steps & 1;
+      left -= (uint64_t)RP.steps;
+    }
+    VL_CUDA(cudaEventRecord(ev1, stream));
+    timed = true;
+    t_host += steps;
+    own_ok = false;
+    done = true;
+    return VL_OK;
+  }
+
   int step(uint64_t steps) {
     VL_CUDA(cudaSetDevice(device));
+    if (resident && resident_ok && !P.stream && steps >= (uint64_t)kResidentMinSteps) {
+      bool done = false;
+      if (int rc = step_resident(steps, done)) return rc;
+      if (done) return VL_OK;
+    }
     if (int rc = prepare_steps()) return rc;
     VL_CUDA(cudaEventRecord(ev0, stream));
     uint64_t left = steps;
@@ -531,6 +624,160 @@ void staged_split(const vl::CompiledDomain& d, const std::vector<int32_t>& lnode
   }
 }
 
+// Whether the resident step kernel takes this domain, and its tables. The rule on size, us per step of
+// the resident kernel / of the fastest schedule of two kernels (B200):
+//   towing tanks and rigs (an absorbing outlet: the two-kernel step waits for its serial outlet sum)
+//     FP64  442 x 84 5.3 / 12.7, 742 x 372 9.2 / 17.2, 1202 x 602 21.6 / 29.0, 1762 x 330 15.0 / 21.3
+//     FP32  302 x 152 5.6 / 13.7, 1042 x 522 10.9 / 21.0, 1802 x 902 27.8 / 35.4
+//     16-bit fixed point 1202 x 602 12.6 / 23.5
+//   boxes without an outlet
+//     FP64  300 x 200 4.9 / 9.9, 700 x 450 9.4 / 13.2, 1000 x 600 16.5 / 17.6, 1200 x 700 26.9 / 25.4
+//     FP32  700 x 450 7.9 / 12.1, 1001 x 600 11.9 / 14.4, 1600 x 900 29.3 / 21.0
+//     16-bit 1000 x 600 11.3 / 13.7 (fixed point), 13.0 / 13.4 (custom), 2002 x 1200 41.0 / 25.7
+// so: the two population buffers within the L2 (128 MB) and at most 1.7 M cells with an outlet, 0.64 M
+// without. Besides, no outlet node may have a link with a force group (its task forms no force terms), at
+// most kBlock chunks of boundary nodes (the force sums' shared memory).
+int resident_setup(vl_sim& s) {
+  const vl::CompiledDomain& d = s.dom;
+  const size_t bytes = 2 * 9 * (size_t)s.ns * s.L->elem;
+  if (bytes > ((size_t)128 << 20) || d.n > (d.pnode_idx.empty() ? (size_t)640000 : (size_t)1700000) || s.P.nlink > vl::kBlock)
+    return VL_OK;
+  const size_t nb = d.bnode_idx.size(), np = d.pnode_idx.size();
+  std::vector<int32_t> outlet_of(nb, -1);
+  std::vector<size_t> order, open, outlet_nodes(np);
+  for (size_t k = 0; k < np; ++k) {
+    const size_t g = (size_t)(std::lower_bound(d.bnode_idx.begin(), d.bnode_idx.end(), d.pnode_idx[k]) - d.bnode_idx.begin());
+    outlet_of[g] = (int32_t)k;
+    outlet_nodes[k] = g;
+    for (int l = d.bnode_first[g]; l < d.bnode_first[g + 1]; ++l)
+      if (d.links[(size_t)l].fgroup >= 0) return VL_OK;
+  }
+  for (size_t g = 0; g < nb; ++g) {
+    if (outlet_of[g] >= 0) continue;
+    bool any = false;
+    for (int l = d.bnode_first[g]; l < d.bnode_first[g + 1]; ++l) any = any || (d.links[(size_t)l].flags & 1);
+    (any ? open : order).push_back(g);
+  }
+  int sms = 0;
+  VL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s.device));
+  if (sms < 2) return VL_OK;
+  // Tasks: about one per block, of 8 to 32 nodes with like links; the last block has none (it sums the
+  // forces). The outlet tasks come first, one to a block as far as there are blocks.
+  const size_t per = std::min<size_t>(32, std::max<size_t>(8, (nb + (size_t)sms - 2) / (size_t)(sms - 1)));
+  // A small domain takes fewer blocks, of 16 segments and the outlet tasks' own (rig of 442 x 84 cells,
+  // FP64: 5.3 us per step on 86 blocks as on 148, 6.0 on 49): another sim's kernel may then run beside it.
+  const size_t need = ((d.nx + 31) / 32) * d.ny / 16 + (np + per - 1) / per + 2;
+  const int G = (int)std::min<size_t>((size_t)sms, std::max<size_t>(2, need));
+  std::vector<std::vector<size_t>> tasks;       // boundary-node ranks
+  std::vector<int> kind;
+  auto cut = [&](const std::vector<size_t>& v, int k) {
+    for (size_t i = 0; i < v.size(); i += per) {
+      tasks.emplace_back(v.begin() + (long)i, v.begin() + (long)std::min(v.size(), i + per));
+      kind.push_back(k);
+    }
+  };
+  cut(outlet_nodes, vl::TASK_OUTLET);
+  const size_t nout = tasks.size();
+  cut(open, vl::TASK_OPEN);
+  cut(order, vl::TASK_WALL);
+  if (nout > (size_t)vl::kResidentTaskWarps * (size_t)(G - 1)) return VL_OK;  // an outlet task has a warp of its own
+  std::vector<int32_t> block_outlets((size_t)G, 0);
+  for (size_t t = 0; t < nout; ++t) ++block_outlets[t % (size_t)(G - 1)];
+  s.res_task_first.assign((size_t)G + 1, 0);
+  std::vector<int4> nodes;
+  std::vector<vl::WallRec> walls;
+  std::vector<int4> trec;
+  std::vector<uint8_t> chunk_force((size_t)s.P.nlink, 0);
+  size_t most = 0;
+  for (int g = 0; g < G; ++g) {
+    size_t count = 0;
+    for (size_t t = (size_t)g; g < G - 1 && t < tasks.size(); t += (size_t)(G - 1), ++count) {
+      const int w0 = (int)walls.size();
+      for (size_t at = 0; at < 32; ++at) {
+        if (at >= tasks[t].size()) {
+          nodes.push_back(make_int4(-1, 0, 0, 0));
+          continue;
+        }
+        const size_t b = tasks[t][at];
+        const unsigned cell = (unsigned)d.bnode_idx[b];
+        const size_t x = (size_t)cell % d.nx, y = (size_t)cell / d.nx;
+        int mask = (x == 0 ? 1 << 27 : 0) | (x == d.nx - 1 ? 1 << 28 : 0) | (y == 0 ? 1 << 29 : 0) | (y == d.ny - 1 ? 1 << 30 : 0);
+        for (int l = d.bnode_first[b]; l < d.bnode_first[b + 1]; ++l) {
+          const vl::LinkRec& h = d.links[(size_t)l];
+          const int j = h.dir;
+          if (h.flags & 1) {
+            mask |= 1 << (j + 9);
+            if (kind[t] == vl::TASK_OUTLET && !(h.flags & 2)) mask |= 1 << (j + 18);
+            continue;
+          }
+          mask |= 1 << j;
+          if (h.fgroup >= 0) {
+            mask |= 1 << (j + 18);
+            chunk_force[b / (size_t)vl::kBlock] = 1;
+          }
+          vl::WallRec w;
+          std::memset(&w, 0, sizeof w);
+          w.slot = (unsigned)((size_t)(j - 1) * 32 + at);
+          // link_back's branches and coefficients, in the arithmetic type
+          unsigned type;
+          if (s.prec == VL_F64) {
+            const double q = h.q, kq = 0.5 / q;
+            type = q >= 0.5 ? vl::WALL_FAR : (h.behind >= 0 ? vl::WALL_NEAR : vl::WALL_HALF);
+            w.c1 = type == vl::WALL_FAR ? kq : 2.0 * q;
+            w.c2 = type == vl::WALL_FAR ? 1.0 - kq : 1.0 - 2.0 * q;
+          } else {
+            const float q = (float)h.q, kq = 0.5f / q;
+            type = q >= 0.5f ? vl::WALL_FAR : (h.behind >= 0 ? vl::WALL_NEAR : vl::WALL_HALF);
+            w.c1 = type == vl::WALL_FAR ? kq : 2.0f * q;
+            w.c2 = type == vl::WALL_FAR ? 1.0f - kq : 1.0f - 2.0f * q;
+          }
+          w.behind = type == vl::WALL_NEAR ? (unsigned)j * s.ns + (unsigned)h.behind : 0u;
+          w.meta = type | ((unsigned)h.vgroup << 2);
+          w.cu6 = h.cu6;
+          walls.push_back(w);
+        }
+        nodes.push_back(make_int4((int)cell, mask, d.bnode_first[b], kind[t] == vl::TASK_OUTLET ? outlet_of[b] : (int)b));
+      }
+      const int w1 = (int)walls.size();
+      trec.push_back(make_int4(w0, w1, kind[t], 0));
+    }
+    s.res_task_first[(size_t)g + 1] = s.res_task_first[(size_t)g] + (int)count;
+    most = std::max(most, count);
+  }
+  std::vector<int32_t> force_chunks;
+  for (size_t c = 0; c < chunk_force.size(); ++c)
+    if (chunk_force[c]) force_chunks.push_back((int32_t)c);
+  vl::ResidentParams& RP = s.RP;
+  RP.grid = G;
+  RP.max_tasks = (int)most;
+  RP.nforce = (int)force_chunks.size();
+  bool ok = true;
+  auto put = [&](auto** dst, const void* src, size_t bytes, bool zero) {
+    void* q = nullptr;
+    if (!ok || alloc_copy(&q, src, bytes) != VL_OK) { ok = false; return; }
+    s.d_res.push_back(q);
+    if (zero && cudaMemset(q, 0, bytes ? bytes : 16) != cudaSuccess) { fail(VL_ECUDA, "resident tables"); ok = false; }
+    *dst = (std::remove_pointer_t<decltype(dst)>)q;
+  };
+  const size_t f8 = sizeof(double);
+  put(&s.d_res_seg, nullptr, ((size_t)G + 1) * 4, true);
+  put(&RP.task_first, s.res_task_first.data(), s.res_task_first.size() * 4, false);
+  put(&RP.nodes, nodes.data(), nodes.size() * sizeof(int4), false);
+  put(&RP.walls, walls.data(), walls.size() * sizeof(vl::WallRec), false);
+  put(&RP.tasks, trec.data(), trec.size() * sizeof(int4), false);
+  s.res_outlets = block_outlets;
+  put(&RP.block_outlets, block_outlets.data(), block_outlets.size() * 4, false);
+  put(&RP.force_chunks, force_chunks.data(), force_chunks.size() * 4, false);
+  put(&RP.arrived, nullptr, sizeof(unsigned), true);
+  put(&RP.node_force, nullptr, 3 * (size_t)2 * d.ngroups * s.P.nbs * f8, true);
+  put(&RP.un, nullptr, 2 * np * f8, true);
+  put(&RP.drho, nullptr, 3 * f8, true);
+  if (!ok) return VL_ENOMEM;
+  RP.seg_first = s.d_res_seg;
+  s.resident_ok = true;
+  return VL_OK;
+}
+
 vl_sim* make_sim(vl::CompiledDomain&& dom, int precision) {
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
@@ -677,6 +924,7 @@ vl_sim* make_sim(vl::CompiledDomain&& dom, int precision) {
   P.warp_bfirst = s->d_wbfirst;
   P.lb = s->d_lb;
   P.ownc = s->d_ownc;
+  if (resident_setup(*s) != VL_OK) return nullptr;
   // Control block: vscale = 1, no outflow target (src/sim.rs:344-347).
   std::memset(&s->hctl, 0, sizeof(vl::Ctl));
   for (int g = 0; g < 4; ++g) s->hctl.vscale[g] = 1.0;

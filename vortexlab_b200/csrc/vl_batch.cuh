@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kBlock) k_batch_bulk(const __grid_constant__ B
   if (STAGED && in) gfirst = __ldg(p.seg_bfirst + T.seg_off + y * T.segs + (x >> 5));
   const uint8_t fl = in ? __ldg(p.flag + T.cell_off + idx) : (uint8_t)2;
   R f[9];
-  if (in) pull(a, T.ns, nx, ny, x, y, f);
+  if (in) pull<S>(a, T.ns, nx, ny, x, y, f);
   int g = -1;
   if (STAGED) {
     const unsigned bal = __ballot_sync(0xffffffffu, fl == 1);
@@ -309,7 +309,8 @@ __global__ void __launch_bounds__(kBlock) k_batch_links(const __grid_constant__ 
     for (int i = 0; i < 9; ++i) Store<S>::st(b + (unsigned)i * T.ns + idx, i, f[i]);
   }
   __syncthreads();
-  block_force_partial(s_acc, 2, p.partials + 2 * (size_t)cd.w);
+  __shared__ double s_red[2][kBlock / 32];
+  block_force_partial(s_acc, 2, p.partials + 2 * (size_t)cd.w, s_red);
   // The last chunk of this tunnel reduces the tunnel's partials and advances its step.
   __syncthreads();
   if (tid == 0) {

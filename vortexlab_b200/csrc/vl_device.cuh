@@ -63,6 +63,7 @@ struct Ctl {
   int dry;                     // timing runs: the epilogue commits nothing (no t, force or history)
   int absorbing;
   int dp_on;
+  int stalled;                 // set when a wait of the resident step kernel ran out
   double u_ref;
   unsigned long long sched_len;
   const double* sched;         // [sched_len][2] = (inlet ramp, body kick) per step
@@ -161,6 +162,7 @@ struct Store<double> {
   static __device__ __forceinline__ double ld(const double* p, int) { return __ldg(p); }
   static __device__ __forceinline__ double ld_cg(const double* p, int) { return __ldcg(p); }
   static __device__ __forceinline__ void st(double* p, int, double v) { *p = v; }
+  static __device__ __forceinline__ double rt(int, double v) { return v; }   // v as a load returns it
 };
 
 template <>
@@ -169,6 +171,7 @@ struct Store<float> {
   static __device__ __forceinline__ float ld(const float* p, int) { return __ldg(p); }
   static __device__ __forceinline__ float ld_cg(const float* p, int) { return __ldcg(p); }
   static __device__ __forceinline__ void st(float* p, int, float v) { *p = v; }
+  static __device__ __forceinline__ float rt(int, float v) { return v; }
 };
 
 template <>
@@ -181,6 +184,9 @@ struct Store<__half> {
     return wgt<float>(i) + __half2float(__ldcg(p));
   }
   static __device__ __forceinline__ void st(__half* p, int i, float v) { *p = __float2half_rn(v - wgt<float>(i)); }
+  static __device__ __forceinline__ float rt(int i, float v) {
+    return wgt<float>(i) + __half2float(__float2half_rn(v - wgt<float>(i)));
+  }
 };
 
 // 16-bit storage of f_i - w_i with more precision where the shifted populations live: sign, a
@@ -232,6 +238,7 @@ struct Store<c16> {
   static __device__ __forceinline__ void st(c16* p, int i, float v) {
     reinterpret_cast<unsigned short*>(p)[0] = (unsigned short)c16f::enc(v, i);
   }
+  static __device__ __forceinline__ float rt(int i, float v) { return c16f::dec(c16f::enc(v, i) & 0xffffu, i); }
 };
 
 // 16-bit fixed point of f_i - w_i: the shifted value in steps of 2^-19 for the rest population and
@@ -265,6 +272,7 @@ struct Store<q16> {
   static __device__ __forceinline__ void st(q16* p, int i, float v) {
     reinterpret_cast<short*>(p)[0] = (short)q16f::enc(v, i);
   }
+  static __device__ __forceinline__ float rt(int i, float v) { return q16f::dec(q16f::enc(v, i), i); }
 };
 
 // Storage formats that saturate instead of carrying a non-finite value.
@@ -328,6 +336,13 @@ template <>
 __device__ __forceinline__ void collide_s<q16>(float* f, int ck, float op, float om, float gx, float gy) {
   collide_s<float>(f, ck, op, om, gx, gy);
 }
+// A population load: through the read-only path (CG = 0), or straight from the L2 (CG = 1) where the
+// running kernel's own blocks have written the buffer since it started (vl_resident.cuh).
+template <class S, int CG>
+__device__ __forceinline__ typename Store<S>::R ldp(const S* p, int i) {
+  return CG ? Store<S>::ld_cg(p, i) : Store<S>::ld(p, i);
+}
+
 template <class R>
 __device__ __forceinline__ R pick(const R* f, int i) {
   R v = f[0];
@@ -352,9 +367,8 @@ struct Controls {
   int has_target;
 };
 
-__device__ __forceinline__ Controls read_controls(const Ctl* c) {
+__device__ __forceinline__ Controls read_controls(const Ctl* c, unsigned long long t) {
   Controls k;
-  const unsigned long long t = c->t;
 #pragma unroll
   for (int g = 0; g < 4; ++g) k.vs[g] = c->vscale[g];
   k.target = c->target;
@@ -369,18 +383,26 @@ __device__ __forceinline__ Controls read_controls(const Ctl* c) {
   }
   return k;
 }
+__device__ __forceinline__ Controls read_controls(const Ctl* c) { return read_controls(c, c->t); }
 
 // ------------------------------------------------------------------ epilogue
+// Who a block-wide helper runs on: the whole block of kBlock threads, or (vl_resident.cuh) one of
+// the kBlock-thread parts of a larger block, which has its own named barrier.
+struct WholeBlock {
+  __device__ __forceinline__ int tid() const { return (int)threadIdx.x; }
+  __device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+
 // Pressure-drop probe (src/cases/cylinder.rs:54-59) of the state `a` recorded as step `tstep`
 // of the history: probe_density (src/sim.rs:624-644) at distances 1, 2, 3 from each wall point,
 // extrapolated to the wall (src/sim.rs:648-651). Block-wide; every thread must call it.
-template <class S>
-__device__ void record_probe(const StepParams& p, const S* __restrict__ a, long long tstep) {
+template <class S, class Part = WholeBlock>
+__device__ void record_probe(const StepParams& p, const S* a, long long tstep, Part part = Part()) {
   __shared__ double rho_c[kProbeCorners];
   Ctl* c = p.ctl;
   const long long rs = (long long)c->rec_start;
   if (!c->dp_on || !c->rec_cap || tstep < rs || tstep - rs >= (long long)c->rec_cap) return;
-  const int tid = threadIdx.x;
+  const int tid = part.tid();
   if (tid < kProbeCorners) {
     const int idx = c->probe_idx[tid];
     double r = 0.0;
@@ -393,7 +415,7 @@ __device__ void record_probe(const StepParams& p, const S* __restrict__ a, long 
     }
     rho_c[tid] = r;
   }
-  __syncthreads();
+  part.sync();
   if (tid == 0) {
     double wall[2];
     for (int side = 0; side < 2; ++side) {
@@ -412,23 +434,24 @@ __device__ void record_probe(const StepParams& p, const S* __restrict__ a, long 
     }
     c->hist[(size_t)(tstep - rs) * kRec + 9] = (1.0 / 3.0) * (wall[0] - wall[1]) / (c->u_ref * c->u_ref);
   }
-  __syncthreads();
+  part.sync();
 }
 
 // Block-wide sum of `count` values spaced `stride` apart: thread t adds values t, t + kBlock, ...
 // in order, then a fixed shared-memory tree. The result is valid in thread 0. Every thread calls it.
-__device__ __forceinline__ double sum_partials(const double* v, int count, int stride, double* red) {
-  const int tid = threadIdx.x;
+template <class Part = WholeBlock>
+__device__ __forceinline__ double sum_partials(const double* v, int count, int stride, double* red, Part part = Part()) {
+  const int tid = part.tid();
   double acc = 0.0;
   for (int k = tid; k < count; k += kBlock) acc += __ldcg(v + (size_t)k * stride);
   red[tid] = acc;
-  __syncthreads();
+  part.sync();
   for (int s = kBlock / 2; s > 0; s >>= 1) {
     if (tid < s) red[tid] += red[tid + s];
-    __syncthreads();
+    part.sync();
   }
   const double out = red[0];
-  __syncthreads();
+  part.sync();
   return out;
 }
 
@@ -511,23 +534,23 @@ __global__ void __launch_bounds__(kBlock) k_probe(const __grid_constant__ StepPa
 // of row y. The nine population loads are issued together with the flag load, for every cell of the
 // tile (wrap keeps every neighbour index inside the grid), so no load waits for the flag; only
 // interior cells (flag 0) store. Boundary cells are written by the link kernel, solid cells never.
-template <class S>
-__device__ __forceinline__ void pull(const S* __restrict__ a, unsigned ns, int nx, int ny, int x, int y,
+template <class S, int CG = 0>
+__device__ __forceinline__ void pull(const S* a, unsigned ns, int nx, int ny, int x, int y,
                                      typename Store<S>::R* f) {
   const int ym = y == 0 ? ny - 1 : y - 1;
   const int yp = y == ny - 1 ? 0 : y + 1;
   const int xm = x == 0 ? nx - 1 : x - 1;
   const int xp = x == nx - 1 ? 0 : x + 1;
   const unsigned rc = (unsigned)(y * nx), rm = (unsigned)(ym * nx), rp = (unsigned)(yp * nx);
-  f[0] = Store<S>::ld(a + rc + x, 0);
-  f[1] = Store<S>::ld(a + 1u * ns + rc + xm, 1);
-  f[2] = Store<S>::ld(a + 2u * ns + rm + x, 2);
-  f[3] = Store<S>::ld(a + 3u * ns + rc + xp, 3);
-  f[4] = Store<S>::ld(a + 4u * ns + rp + x, 4);
-  f[5] = Store<S>::ld(a + 5u * ns + rm + xm, 5);
-  f[6] = Store<S>::ld(a + 6u * ns + rm + xp, 6);
-  f[7] = Store<S>::ld(a + 7u * ns + rp + xp, 7);
-  f[8] = Store<S>::ld(a + 8u * ns + rp + xm, 8);
+  f[0] = ldp<S, CG>(a + rc + x, 0);
+  f[1] = ldp<S, CG>(a + 1u * ns + rc + xm, 1);
+  f[2] = ldp<S, CG>(a + 2u * ns + rm + x, 2);
+  f[3] = ldp<S, CG>(a + 3u * ns + rc + xp, 3);
+  f[4] = ldp<S, CG>(a + 4u * ns + rp + x, 4);
+  f[5] = ldp<S, CG>(a + 5u * ns + rm + xm, 5);
+  f[6] = ldp<S, CG>(a + 6u * ns + rm + xp, 6);
+  f[7] = ldp<S, CG>(a + 7u * ns + rp + xp, 7);
+  f[8] = ldp<S, CG>(a + 8u * ns + rp + xm, 8);
 }
 
 //
@@ -557,7 +580,7 @@ __global__ void __launch_bounds__(kBlock) k_bulk(const __grid_constant__ StepPar
   if (STAGED) wfirst = __ldg(p.warp_bfirst + (size_t)tile * (kBlock / 32) + (threadIdx.x >> 5));
   const uint8_t fl = in ? __ldg(p.flag + idx) : (uint8_t)2;
   R f[9];
-  if (in) pull(a, p.ns, nx, ny, x, y, f);
+  if (in) pull<S>(a, p.ns, nx, ny, x, y, f);
   int k = -1;
   if (STAGED) {
     const unsigned bal = __ballot_sync(0xffffffffu, fl == 1);
@@ -716,8 +739,8 @@ __device__ __forceinline__ void force_terms(const LinkView& L, double o, double 
   ty = (double)cy_of(L.dir) * (o + bk) - wuy * (o - bk);
 }
 
-template <class S, class Put>
-__device__ __forceinline__ void link_rules(const S* __restrict__ a, unsigned ns, const typename Store<S>::R* own,
+template <class S, int CG = 0, class Put>
+__device__ __forceinline__ void link_rules(const S* a, unsigned ns, const typename Store<S>::R* own,
                                            int first, int last, const LinkRecDev* __restrict__ links,
                                            const double* vs, double drho, double gx_, double gy_, double sqrt_cs2,
                                            double* acc, Put put) {
@@ -728,7 +751,7 @@ __device__ __forceinline__ void link_rules(const S* __restrict__ a, unsigned ns,
   for (int l = first; l < last; ++l) {
     const LinkView L = load_link(links, l);
     R out, scale;
-    const R bval = uses_behind(L) ? Store<S>::ld(a + (unsigned)L.dir * ns + (unsigned)L.behind, L.dir) : R(0);
+    const R bval = uses_behind(L) ? ldp<S, CG>(a + (unsigned)L.dir * ns + (unsigned)L.behind, L.dir) : R(0);
     const R back = link_back<S>(bval, L, own, vs, drho, gx, gy, sqrt_cs2, have_u, ux, uy, out, scale);
     put(l, opp_of(L.dir), back);
     if (L.fgroup >= 0) {
@@ -743,8 +766,8 @@ __device__ __forceinline__ void link_rules(const S* __restrict__ a, unsigned ns,
 // The link pass for one boundary node (src/sim.rs:456-503): the incoming populations pulled from
 // the neighbours, each one that would come out of the boundary replaced by its link's rule, then
 // the collision. `f` returns the post-collision populations.
-template <class S>
-__device__ __forceinline__ void link_node(const S* __restrict__ a, unsigned ns, int nx, int ny, int idx, int first,
+template <class S, int CG = 0>
+__device__ __forceinline__ void link_node(const S* a, unsigned ns, int nx, int ny, int idx, int first,
                                           int last, const LinkRecDev* __restrict__ links, const double* vs,
                                           double drho, int ck, double op_, double om_, double gx_, double gy_,
                                           double sqrt_cs2, double* acc, typename Store<S>::R* f) {
@@ -752,26 +775,27 @@ __device__ __forceinline__ void link_node(const S* __restrict__ a, unsigned ns, 
   const R op = (R)op_, om = (R)om_, gx = (R)gx_, gy = (R)gy_;
   const int y = idx / nx, x = idx - y * nx;
   R own[9];
-  pull(a, ns, nx, ny, x, y, f);
+  pull<S, CG>(a, ns, nx, ny, x, y, f);
 #pragma unroll
-  for (int d = 0; d < 9; ++d) own[d] = Store<S>::ld(a + (unsigned)d * ns + idx, d);
-  link_rules<S>(a, ns, own, first, last, links, vs, drho, gx_, gy_, sqrt_cs2, acc,
+  for (int d = 0; d < 9; ++d) own[d] = ldp<S, CG>(a + (unsigned)d * ns + idx, d);
+  link_rules<S, CG>(a, ns, own, first, last, links, vs, drho, gx_, gy_, sqrt_cs2, acc,
                 [&](int, int i, R back) { set_dir(f, i, back); });
   collide_s<S>(f, ck, op, om, gx, gy);
 }
 
 // Block partial of the first `ncomp` force components: fixed shuffle tree within each warp, then
 // the warps in order. Written by threads 0..ncomp-1 to out[c]. Every thread calls it.
-__device__ __forceinline__ void block_force_partial(const double (*s_acc)[kBlock], int ncomp, double* out) {
-  __shared__ double s_red[2 * kMaxGroups][kBlock / 32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+template <class Part = WholeBlock>
+__device__ __forceinline__ void block_force_partial(const double (*s_acc)[kBlock], int ncomp, double* out,
+                                                    double (*s_red)[kBlock / 32], Part part = Part()) {
+  const int tid = part.tid(), lane = tid & 31, warp = tid >> 5;
   for (int c = 0; c < ncomp; ++c) {
     double v = s_acc[c][tid];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
     if (lane == 0) s_red[c][warp] = v;
   }
-  __syncthreads();
+  part.sync();
   if (tid < ncomp) {
     double v = 0.0;
     for (int w = 0; w < kBlock / 32; ++w) v += s_red[tid][w];
@@ -807,7 +831,8 @@ __global__ void __launch_bounds__(kBlock, VL_LINK_MIN_BLOCKS) k_links(const __gr
   }
   if (ncomp > 0) {
     __syncthreads();
-    block_force_partial(s_acc, ncomp, p.partials + (size_t)blockIdx.x * (2 * kMaxGroups));
+    __shared__ double s_red[2 * kMaxGroups][kBlock / 32];
+    block_force_partial(s_acc, ncomp, p.partials + (size_t)blockIdx.x * (2 * kMaxGroups), s_red);
   }
   arrive<S>(p, a, p.nlink);
 }
@@ -894,7 +919,8 @@ __global__ void __launch_bounds__(kBlock) k_links_stage(const __grid_constant__ 
   }
   if (ncomp > 0) {
     __syncthreads();
-    block_force_partial(s_acc, ncomp, p.partials + (size_t)blk * (2 * kMaxGroups));
+    __shared__ double s_red[2 * kMaxGroups][kBlock / 32];
+    block_force_partial(s_acc, ncomp, p.partials + (size_t)blk * (2 * kMaxGroups), s_red);
   }
   arrive<S>(p, a, p.nlinkblk);
 }

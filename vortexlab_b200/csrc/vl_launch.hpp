@@ -11,6 +11,7 @@ namespace vl {
 
 struct StepParams;
 struct BatchParams;
+struct ResidentParams;
 
 struct Launchers {
   size_t elem;  // bytes per stored population value
@@ -30,6 +31,11 @@ struct Launchers {
   cudaError_t (*reduce)(int n, unsigned ns, const uint8_t* flag, double gx, double gy, const void* a,
                         double* out, int blocks, cudaStream_t s);
   cudaError_t (*gather)(int m, unsigned ns, const int32_t* cells, const void* a, double* out, cudaStream_t s);
+  // Many steps in one cooperative launch (k_resident), from buffer `a`; the cells of a row one of its
+  // threads updates, and the blocks that fit the device at once (0: it cannot run).
+  cudaError_t (*resident)(const StepParams& p, const ResidentParams& r, int ck, void* a, void* b, cudaStream_t s);
+  int (*resident_width)(const StepParams& p, int ck);
+  int (*resident_blocks)(const StepParams& p, const ResidentParams& r, int ck, int sms);
   // Records the pressure probe of the last step of a batch (one block).
   cudaError_t (*probe)(const StepParams& p, const void* a, cudaStream_t s);
   // One step of a batch of tunnels: which = 1 link kernel, 2 bulk kernel, 3 both; + 4 the staged

@@ -7,6 +7,7 @@
 #include "vl_device.cuh"
 #include "vl_launch.hpp"
 #include "vl_pair.cuh"
+#include "vl_resident.cuh"
 #include "vl_stream.cuh"
 
 namespace vl {
@@ -111,6 +112,43 @@ struct LaunchImpl {
       default: return step_ck<1>(p, A, B, s, which, staged);
     }
   }
+  // ---- resident step kernel
+  using ResidentFn = void (*)(const StepParams, const ResidentParams, S*, S*);
+  static ResidentFn resident_fn(const StepParams& p, int ck) {
+    const int v = resident_width(p, ck);
+    if constexpr (!std::is_same<S, double>::value) {
+      if (v == 2) return ck == 0 ? k_resident<S, 2, 0> : k_resident<S, 2, 1>;
+    }
+    return ck == 0 ? k_resident<S, 1, 0> : (ck == 1 ? k_resident<S, 1, 1> : k_resident<S, 1, 2>);
+  }
+  // (at most two: four cells per thread do not fit the 64 registers of its narrow threads)
+  static int resident_width(const StepParams& p, int ck) {
+    const int v = ck == 0 ? group_width<0>(p) : (ck == 1 ? group_width<1>(p) : group_width<2>(p));
+    return v < 2 ? v : 2;
+  }
+  static size_t resident_bytes(const StepParams& p, const ResidentParams& r) {
+    return (size_t)((p.np + 1) / 2 * 2) * sizeof(double) + (size_t)r.max_tasks * sizeof(TaskScratch<typename Store<S>::R>);
+  }
+  // Blocks of the kernel that fit the device at once (0: it cannot run).
+  static int resident_blocks(const StepParams& p, const ResidentParams& r, int ck, int sms) {
+    const void* fn = (const void*)resident_fn(p, ck);
+    int per = 0;
+    if (resident_bytes(p, r) > (size_t)kResidentSmem ||
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidentSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kResidentThreads, resident_bytes(p, r)) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return per * sms;
+  }
+  static cudaError_t resident(const StepParams& p, const ResidentParams& r, int ck, void* a, void* b, cudaStream_t s) {
+    StepParams pp = p;
+    ResidentParams rr = r;
+    S *A = (S*)a, *B = (S*)b;
+    void* args[] = {&pp, &rr, &A, &B};
+    const void* fn = (const void*)resident_fn(p, ck);
+    return cudaLaunchCooperativeKernel(fn, dim3((unsigned)r.grid), dim3(kResidentThreads), args, resident_bytes(p, r), s);
+  }
   static int grid_for(int n) { return n <= 0 ? 1 : (n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16; }
   static cudaError_t init(int n, unsigned ns, const uint8_t* flag, const double* rho, const double* ux,
                           const double* uy, double rho0, double ux0, double uy0, void* a, void* b, cudaStream_t s) {
@@ -185,7 +223,7 @@ struct LaunchImpl {
     return cudaGetLastError();
   }
   static const Launchers& table() {
-    static const Launchers t = {sizeof(S), &step, &init, &init_grid, &to_f64, &from_f64, &macros, &reduce, &gather, &probe, &batch_step,
+    static const Launchers t = {sizeof(S), &step, &init, &init_grid, &to_f64, &from_f64, &macros, &reduce, &gather, &resident, &resident_width, &resident_blocks, &probe, &batch_step,
                                 &gather_own, &batch_gather_own};
     return t;
   }

@@ -86,6 +86,12 @@ struct Codec16<q16> {
 };
 
 // ------------------------------------------------------------------ vector access per format
+// A plane's values are read through the read-only path (CG = 0), or from the L2 (CG = 1) where the
+// running kernel's own blocks write the buffer (vl_resident.cuh).
+template <int CG, class T>
+__device__ __forceinline__ T ld_word(const T* p) {
+  return CG ? __ldcg(p) : __ldg(p);
+}
 // `Word` holds a thread's V stored values; dec / left / right give the V / 2 FP32 pairs of the
 // aligned group, of the group shifted one cell left (x0 - 1 ..) and one cell right (x0 + 1 ..);
 // `edge` selects the value at `ep` instead of the neighbouring lane's.
@@ -95,27 +101,29 @@ struct GroupIO;
 template <>
 struct GroupIO<float, 2> {
   using Word = float2;
-  template <bool SM>
+  template <int CG>
   static __device__ __forceinline__ Word ld(const float* p) {
 #ifdef VL_LD_L2_256B
-    if (!SM) {
+    if (!CG) {
       float2 w;
       asm("ld.global.nc.L2::256B.v2.f32 {%0, %1}, [%2];" : "=f"(w.x), "=f"(w.y) : "l"(p));
       return w;
     }
 #endif
-    return SM ? *reinterpret_cast<const float2*>(p) : __ldg(reinterpret_cast<const float2*>(p));
+    return ld_word<CG>(reinterpret_cast<const float2*>(p));
   }
   static __device__ __forceinline__ void st(float* p, Word w) { *reinterpret_cast<float2*>(p) = w; }
   static __device__ __forceinline__ void dec(int, Word w, float2* o) { o[0] = w; }
+  template <int CG>
   static __device__ __forceinline__ void left(int, Word v, bool edge, const float* ep, float2* o) {
     float up = __shfl_up_sync(0xffffffffu, v.y, 1);
-    if (edge) up = *ep;
+    if (edge) up = CG ? __ldcg(ep) : *ep;
     o[0] = make_float2(up, v.x);
   }
+  template <int CG>
   static __device__ __forceinline__ void right(int, Word v, bool edge, const float* ep, float2* o) {
     float dn = __shfl_down_sync(0xffffffffu, v.x, 1);
-    if (edge) dn = *ep;
+    if (edge) dn = CG ? __ldcg(ep) : *ep;
     o[0] = make_float2(v.y, dn);
   }
   static __device__ __forceinline__ Word enc(int, const float2* f) { return f[0]; }
@@ -124,56 +132,61 @@ struct GroupIO<float, 2> {
 template <>
 struct GroupIO<float, 4> {
   using Word = float4;
-  template <bool SM>
+  template <int CG>
   static __device__ __forceinline__ Word ld(const float* p) {
-    return SM ? *reinterpret_cast<const float4*>(p) : __ldg(reinterpret_cast<const float4*>(p));
+    return ld_word<CG>(reinterpret_cast<const float4*>(p));
   }
   static __device__ __forceinline__ void st(float* p, Word w) { *reinterpret_cast<float4*>(p) = w; }
   static __device__ __forceinline__ void dec(int, Word w, float2* o) {
     o[0] = make_float2(w.x, w.y);
     o[1] = make_float2(w.z, w.w);
   }
+  template <int CG>
   static __device__ __forceinline__ void left(int, Word v, bool edge, const float* ep, float2* o) {
     float up = __shfl_up_sync(0xffffffffu, v.w, 1);
-    if (edge) up = *ep;
+    if (edge) up = CG ? __ldcg(ep) : *ep;
     o[0] = make_float2(up, v.x);
     o[1] = make_float2(v.y, v.z);
   }
+  template <int CG>
   static __device__ __forceinline__ void right(int, Word v, bool edge, const float* ep, float2* o) {
     float dn = __shfl_down_sync(0xffffffffu, v.x, 1);
-    if (edge) dn = *ep;
+    if (edge) dn = CG ? __ldcg(ep) : *ep;
     o[0] = make_float2(v.y, v.z);
     o[1] = make_float2(v.w, dn);
   }
   static __device__ __forceinline__ Word enc(int, const float2* f) { return make_float4(f[0].x, f[0].y, f[1].x, f[1].y); }
 };
 
-// One stored 16-bit value (a generic load: the pointer may be in global or shared memory).
-template <class S>
+// One stored 16-bit value.
+template <int CG, class S>
 __device__ __forceinline__ unsigned ld16(const S* p) {
-  return (unsigned)*reinterpret_cast<const unsigned short*>(p);
+  const unsigned short* q = reinterpret_cast<const unsigned short*>(p);
+  return (unsigned)(CG ? __ldcg(q) : *q);
 }
 
 template <class S>
 struct GroupIO<S, 2> {
   using Word = unsigned;
   using C = Codec16<S>;
-  template <bool SM>
+  template <int CG>
   static __device__ __forceinline__ Word ld(const S* p) {
-    return SM ? *reinterpret_cast<const unsigned*>(p) : __ldg(reinterpret_cast<const unsigned*>(p));
+    return ld_word<CG>(reinterpret_cast<const unsigned*>(p));
   }
   static __device__ __forceinline__ void st(S* p, Word w) { *reinterpret_cast<unsigned*>(p) = w; }
   static __device__ __forceinline__ void dec(int i, Word w, float2* o) { o[0] = C::dec(i, w); }
   // low half: the previous lane's high half (or the value at `ep`); high half: the own low half
+  template <int CG>
   static __device__ __forceinline__ void left(int i, Word v, bool edge, const S* ep, float2* o) {
     unsigned up = __shfl_up_sync(0xffffffffu, v, 1);
-    if (edge) up = ld16(ep) << 16;
+    if (edge) up = ld16<CG>(ep) << 16;
     o[0] = C::dec(i, __byte_perm(up, v, 0x5432));
   }
   // low half: the own high half; high half: the next lane's low half (or the value at `ep`)
+  template <int CG>
   static __device__ __forceinline__ void right(int i, Word v, bool edge, const S* ep, float2* o) {
     unsigned dn = __shfl_down_sync(0xffffffffu, v, 1);
-    if (edge) dn = ld16(ep);
+    if (edge) dn = ld16<CG>(ep);
     o[0] = C::dec(i, __byte_perm(v, dn, 0x5432));
   }
   static __device__ __forceinline__ Word enc(int i, const float2* f) { return C::enc(i, f[0]); }
@@ -183,24 +196,26 @@ template <class S>
 struct GroupIO<S, 4> {
   using Word = uint2;
   using C = Codec16<S>;
-  template <bool SM>
+  template <int CG>
   static __device__ __forceinline__ Word ld(const S* p) {
-    return SM ? *reinterpret_cast<const uint2*>(p) : __ldg(reinterpret_cast<const uint2*>(p));
+    return ld_word<CG>(reinterpret_cast<const uint2*>(p));
   }
   static __device__ __forceinline__ void st(S* p, Word w) { *reinterpret_cast<uint2*>(p) = w; }
   static __device__ __forceinline__ void dec(int i, Word w, float2* o) {
     o[0] = C::dec(i, w.x);
     o[1] = C::dec(i, w.y);
   }
+  template <int CG>
   static __device__ __forceinline__ void left(int i, Word v, bool edge, const S* ep, float2* o) {
     unsigned up = __shfl_up_sync(0xffffffffu, v.y, 1);
-    if (edge) up = ld16(ep) << 16;
+    if (edge) up = ld16<CG>(ep) << 16;
     o[0] = C::dec(i, __byte_perm(up, v.x, 0x5432));
     o[1] = C::dec(i, __byte_perm(v.x, v.y, 0x5432));
   }
+  template <int CG>
   static __device__ __forceinline__ void right(int i, Word v, bool edge, const S* ep, float2* o) {
     unsigned dn = __shfl_down_sync(0xffffffffu, v.x, 1);
-    if (edge) dn = ld16(ep);
+    if (edge) dn = ld16<CG>(ep);
     o[0] = C::dec(i, __byte_perm(v.x, v.y, 0x5432));
     o[1] = C::dec(i, __byte_perm(v.y, dn, 0x5432));
   }
@@ -239,21 +254,19 @@ struct PairTask {
   int seg, x0t, halo;
 };
 
-// The pull of plane i for the thread's group: `src` is where the source row's values are read
-// (global memory, or a shared-memory copy indexed by the same x), `grow` the source row in global
-// memory (read at the periodic wrap).
-template <class S, int V, int SHIFT, bool SM>
-__device__ __forceinline__ void pull_group(const S* __restrict__ src, const S* __restrict__ grow, int i, int x0, int xl,
+// The pull of plane i for the thread's group from the source row `src`.
+template <class S, int V, int SHIFT, int CG>
+__device__ __forceinline__ void pull_group(const S* src, int i, int x0, int xl,
                                            int nx, int lane, bool in, float2 (*f)[9]) {
   using IO = GroupIO<S, V>;
   float2 o[V / 2];
-  const typename IO::Word v = IO::template ld<SM>(src + xl);
+  const typename IO::Word v = IO::template ld<CG>(src + xl);
   if (SHIFT == 0)
     IO::dec(i, v, o);
   else if (SHIFT < 0)
-    IO::left(i, v, lane == 0, x0 == 0 ? grow + (nx - 1) : src + (x0 - 1), o);
+    IO::template left<CG>(i, v, lane == 0, x0 == 0 ? src + (nx - 1) : src + (x0 - 1), o);
   else
-    IO::right(i, v, in && (lane == 31 || x0 + V >= nx), x0 + V >= nx ? grow : src + (x0 + V), o);
+    IO::template right<CG>(i, v, in && (lane == 31 || x0 + V >= nx), x0 + V >= nx ? src : src + (x0 + V), o);
 #pragma unroll
   for (int p = 0; p < V / 2; ++p) f[p][i] = o[p];
 }
@@ -262,8 +275,8 @@ __device__ __forceinline__ float& cell_of(float2 (*f)[9], int c, int i) {
   return (c & 1) ? f[c >> 1][i].y : f[c >> 1][i].x;
 }
 
-template <class S, int V, int STAGED, bool SM = false>
-__device__ __forceinline__ void group_update(const PairTask& t, const S* __restrict__ a, S* __restrict__ b) {
+template <class S, int V, int STAGED, int CG = 0>
+__device__ __forceinline__ void group_update(const PairTask& t, const S* a, S* b) {
   using IO = GroupIO<S, V>;
   const int nx = t.nx, ny = t.ny, y = t.y;
   const int lane = (int)(threadIdx.x & 31u);
@@ -281,19 +294,15 @@ __device__ __forceinline__ void group_update(const PairTask& t, const S* __restr
   float2 f[V / 2][9];
   const S* g[9] = {a + rc, a + 1u * ns + rc, a + 2u * ns + rm, a + 3u * ns + rc, a + 4u * ns + rp,
                    a + 5u * ns + rm, a + 6u * ns + rm, a + 7u * ns + rp, a + 8u * ns + rp};
-  const S* sr[9];
-#pragma unroll
-  for (int i = 0; i < 9; ++i)
-    sr[i] = SM ? (const S*)t.stage + (i * t.seg + t.halo - t.x0t) : g[i];
-  pull_group<S, V, 0, SM>(sr[0], g[0], 0, x0, xl, nx, lane, in, f);
-  pull_group<S, V, -1, SM>(sr[1], g[1], 1, x0, xl, nx, lane, in, f);
-  pull_group<S, V, 0, SM>(sr[2], g[2], 2, x0, xl, nx, lane, in, f);
-  pull_group<S, V, 1, SM>(sr[3], g[3], 3, x0, xl, nx, lane, in, f);
-  pull_group<S, V, 0, SM>(sr[4], g[4], 4, x0, xl, nx, lane, in, f);
-  pull_group<S, V, -1, SM>(sr[5], g[5], 5, x0, xl, nx, lane, in, f);
-  pull_group<S, V, 1, SM>(sr[6], g[6], 6, x0, xl, nx, lane, in, f);
-  pull_group<S, V, 1, SM>(sr[7], g[7], 7, x0, xl, nx, lane, in, f);
-  pull_group<S, V, -1, SM>(sr[8], g[8], 8, x0, xl, nx, lane, in, f);
+  pull_group<S, V, 0, CG>(g[0], 0, x0, xl, nx, lane, in, f);
+  pull_group<S, V, -1, CG>(g[1], 1, x0, xl, nx, lane, in, f);
+  pull_group<S, V, 0, CG>(g[2], 2, x0, xl, nx, lane, in, f);
+  pull_group<S, V, 1, CG>(g[3], 3, x0, xl, nx, lane, in, f);
+  pull_group<S, V, 0, CG>(g[4], 4, x0, xl, nx, lane, in, f);
+  pull_group<S, V, -1, CG>(g[5], 5, x0, xl, nx, lane, in, f);
+  pull_group<S, V, 1, CG>(g[6], 6, x0, xl, nx, lane, in, f);
+  pull_group<S, V, 1, CG>(g[7], 7, x0, xl, nx, lane, in, f);
+  pull_group<S, V, -1, CG>(g[8], 8, x0, xl, nx, lane, in, f);
   int k[V];
   if (STAGED) {
     const unsigned lt = (1u << lane) - 1u;

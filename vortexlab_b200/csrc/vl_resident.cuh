@@ -1,0 +1,575 @@
+// The resident step kernel: many steps of one sim in one cooperative launch.
+//
+// A domain whose two population buffers stay in the L2 takes a few microseconds of memory traffic
+// per step, less than the launches, the fork / join and the serial outlet sum of the two-kernel
+// step cost. Here one block per SM stays on the chip for all the steps of a call and a grid-wide
+// arrival counter separates them. Per step:
+//
+//   boundary tasks  8 to 32 boundary nodes with like links, a warp each, dealt out over the blocks: the
+//                   loads of a column's nodes are a transaction each. The wall links of a task run one
+//                   per lane from records whose coefficients the host has worked out (WallRec); then one
+//                   lane per node takes the returning populations, collides and stores. The nodes' own
+//                   populations stay in shared memory, and the part of the open-boundary rules that
+//                   needs only them is worked out after the block has arrived. The outlet nodes have
+//                   tasks and blocks of their own; there one warp sums the outlet velocities that the
+//                   previous step left (sequentially, src/sim.rs:444-455) beside the tasks.
+//   bulk            segments of 32 V cells of a row, taken by the block's other warps in turn.
+//   one part        (kBlock threads of the last block) the force sums and history record of the step
+//                   before the previous one, and the pressure probe of the previous step.
+//
+// The force terms of a task are formed after the block has arrived, per node in link order; that
+// part sums them by the tree of k_links over the same chunks of kBlock nodes.
+//
+// Populations are read from the L2 (ld.global.cg: another block wrote them a step before). The
+// counter is polled with relaxed loads, which leave the L1 alone, so the tables (read-only path) stay
+// in it from step to step; a block's stores are ordered before its arrival by the release, and no
+// population load is issued before the poll has returned. Every value is computed by the functions of
+// the two-kernel step in their order, so states, forces and records are bit-identical to it.
+//
+// Every wait is bounded (kWaitPolls polls); a block that gives up sets Ctl::stalled and leaves, and
+// so do the blocks that wait for it. The launch is cooperative: all blocks are on the chip at once.
+#pragma once
+
+#include "vl_device.cuh"
+#include "vl_pair.cuh"
+
+namespace vl {
+
+constexpr unsigned kWaitPolls = 1u << 22;   // seconds
+constexpr int kResidentThreads = 1024;      // 32 warps of 64 registers: enough loads in flight for the L2
+constexpr int kResidentWarps = kResidentThreads / 32;
+constexpr int kResidentTaskWarps = 16;      // the warps that take boundary tasks
+constexpr int kResidentSumPart = 2;         // the part of the last block that sums the forces
+constexpr int kResidentSmem = 160 * 1024;   // most dynamic shared memory of a block
+
+// A wall link of a task: c1, c2 are the coefficients of its rule (link_back: 0.5 / q and 1 - 0.5 / q, or
+// 2 q and 1 - 2 q), worked out in the arithmetic type; `behind` the population a[j][behind] of the near
+// rule.
+enum : unsigned { WALL_FAR = 0, WALL_NEAR = 1, WALL_HALF = 2 };   // q >= 1/2; q < 1/2; no node behind
+struct alignas(16) WallRec {
+  unsigned behind;
+  unsigned slot;                // (j - 1) * 32 + lane of its node
+  unsigned meta;                // type | vgroup << 2
+  unsigned pad0;
+  double c1, c2;
+  double cu6, pad1;
+};
+
+enum : int { TASK_WALL = 0, TASK_OPEN = 1, TASK_OUTLET = 2 };   // nodes with wall links only; with open links
+
+struct ResidentParams {
+  int steps;
+  int grid;
+  const int32_t* seg_first;     // [grid + 1] first row segment of each block
+  const int32_t* task_first;    // [grid + 1] first task of each block
+  int segs_per_row;             // segments of 32 V cells
+  // Per task and lane {cell or -1; link directions j: wall 1 << j, open 1 << (j + 9), and with force or (an
+  // outlet node) pressure 1 << (j + 18); first link; rank in the boundary-node list, or index in the outlet list}.
+  const int4* nodes;
+  // with a cell at the grid's edge: x = 0 1 << 27, x = nx - 1 1 << 28, y = 0 1 << 29, y = ny - 1 1 << 30
+  const WallRec* walls;
+  const int4* tasks;            // {first wall record, end, kind, -}
+  const int32_t* block_outlets; // outlet tasks of each block
+  int max_tasks;                // most tasks of a block
+  const int32_t* force_chunks;  // chunks that hold a node with force
+  int nforce;
+  unsigned* arrived;            // arrivals since the sim was built
+  unsigned arrived0;            // arrivals before this launch
+  double* node_force;           // three sets of [2 * ngroups][nbs], zero for nodes without force
+  double* un;                   // two sets of the outlet nodes' normal velocities
+  double* drho;                 // [3]
+};
+
+// Dynamic shared memory: the outlet velocities, then per task of the block (by lane of the node) the
+// returning populations of the links by direction j - 1, for an open link the part of it that needs no
+// outlet offset, and the nodes' own populations before and after the step (by its parity).
+template <class R>
+struct TaskScratch {
+  R back[8][32];
+  R open[8][32];
+  R own[2][9][32];
+};
+
+// One part of a block.
+struct PartOf {
+  int part;
+  __device__ __forceinline__ int tid() const { return (int)threadIdx.x & (kBlock - 1); }
+  __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(1 + part), "r"(kBlock) : "memory"); }
+};
+
+__device__ __forceinline__ void grid_arrive(unsigned* counter) {
+  __syncthreads();
+  if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+}
+
+// Waits (thread 0 of the block) until `target` arrivals have been counted.
+__device__ __forceinline__ bool poll_arrived(const unsigned* counter, unsigned target) {
+  for (unsigned k = 0; k < kWaitPolls; ++k) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
+    if ((int)(v - target) >= 0) return true;
+  }
+  return false;
+}
+
+// The sequential sum of n values in shared memory (the order of the reference); the next eight
+// are loaded during the chain of additions (9 cycles each).
+__device__ __forceinline__ double serial_sum(const double* v, int n) {
+  double s = 0.0;
+  int k = 0;
+  if (n >= 8) {
+    double x[8], y[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = v[i];
+    for (; k + 24 <= n; k += 16) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) y[i] = v[k + 8 + i];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s += x[i];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = v[k + 16 + i];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s += y[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += x[i];
+    k += 8;
+  }
+  for (; k < n; ++k) s += v[k];
+  return s;
+}
+
+// The named barrier between a block's summing warp and its outlet tasks' warps.
+__device__ __forceinline__ void outlet_sum_ready(int tasks) {
+  asm volatile("bar.arrive 8, %0;" ::"r"(32 * (1 + tasks)) : "memory");
+}
+__device__ __forceinline__ void outlet_sum_wait(int tasks) {
+  asm volatile("bar.sync 8, %0;" ::"r"(32 * (1 + tasks)) : "memory");
+}
+
+// The pull of a boundary node (pull) with its wraps from the node's flags.
+template <class S>
+__device__ __forceinline__ void pull_node(const S* a, unsigned ns, int nx, int ny, unsigned cell, int flags,
+                                          typename Store<S>::R* f) {
+  const unsigned up = (flags >> 29) & 1 ? (unsigned)((ny - 1) * nx) : (unsigned)-nx;         // row y - 1
+  const unsigned dn = (flags >> 30) & 1 ? (unsigned)-((ny - 1) * nx) : (unsigned)nx;         // row y + 1
+  const unsigned xm = (flags >> 27) & 1 ? (unsigned)(nx - 1) : (unsigned)-1;
+  const unsigned xp = (flags >> 28) & 1 ? (unsigned)(1 - nx) : 1u;
+  f[0] = Store<S>::ld_cg(a + cell, 0);
+  f[1] = Store<S>::ld_cg(a + 1u * ns + (cell + xm), 1);
+  f[2] = Store<S>::ld_cg(a + 2u * ns + (cell + up), 2);
+  f[3] = Store<S>::ld_cg(a + 3u * ns + (cell + xp), 3);
+  f[4] = Store<S>::ld_cg(a + 4u * ns + (cell + dn), 4);
+  f[5] = Store<S>::ld_cg(a + 5u * ns + (cell + up + xm), 5);
+  f[6] = Store<S>::ld_cg(a + 6u * ns + (cell + up + xp), 6);
+  f[7] = Store<S>::ld_cg(a + 7u * ns + (cell + dn + xp), 7);
+  f[8] = Store<S>::ld_cg(a + 8u * ns + (cell + dn + xm), 8);
+}
+
+// Normal velocity of an outlet node from its populations as stored (outlet_offset).
+__device__ __forceinline__ double outlet_velocity(const double* f, const StepParams& p, int k) {
+  double rho, jx, jy;
+  moments(f, rho, jx, jy);
+  const double ux = jx / rho - 0.5 * p.gx, uy = jy / rho - 0.5 * p.gy;
+  return (double)p.pnode_n[2 * k] * ux + (double)p.pnode_n[2 * k + 1] * uy;
+}
+
+// What a task's open links return, as far as it follows from the nodes' own populations (link_back): of
+// a radiating link everything, of a pressure link the factor 1 + cu^2 / 2 - 1.5 u^2 and the link's density.
+template <class S>
+__device__ __forceinline__ void open_prepare(const StepParams& p, const int4& nd, int kind, int parity,
+                                             TaskScratch<typename Store<S>::R>& t) {
+  using R = typename Store<S>::R;
+  const int lane = (int)(threadIdx.x & 31u);
+  if (nd.x < 0 || !((nd.y >> 9) & 0x1ff)) return;
+  R own[9];
+#pragma unroll
+  for (int d = 0; d < 9; ++d) own[d] = t.own[parity][d][lane];
+  R rho, jx, jy;
+  moments(own, rho, jx, jy);
+  const R ux = jx / rho - R(0.5) * (R)p.gx, uy = jy / rho - R(0.5) * (R)p.gy;
+  const unsigned all = ((unsigned)nd.y | ((unsigned)nd.y >> 9)) & 0x1ffu;
+#pragma unroll
+  for (int j = 1; j < 9; ++j) {
+    if (!((nd.y >> (j + 9)) & 1)) continue;
+    const R cu = R(3.0) * ((R)cx_of(j) * ux + (R)cy_of(j) * uy);
+    R g = R(1.0) + R(0.5) * cu * cu - R(1.5) * (ux * ux + uy * uy);
+    const int4 w = __ldg(reinterpret_cast<const int4*>((const LinkRecDev*)p.links + nd.z + __popc(all & ((1u << j) - 1u))) + 2);
+    const R lrho = (R)__hiloint2double(w.y, w.x);
+    if (kind == TASK_OUTLET && ((nd.y >> (j + 18)) & 1)) {
+      t.back[j - 1][lane] = lrho;
+    } else {
+      const int flags = (int)(((unsigned)w.w >> 8) & 0xffu);
+      const R nxv = (R)((int)((flags >> 2) & 3) - 1), nyv = (R)((int)((flags >> 4) & 3) - 1);
+      const R rho_w = lrho + (nxv * ux + nyv * uy) / (R)p.sqrt_cs2;
+      g = -own[j] + R(2.0) * (R)w_of(j) * rho_w * g;
+    }
+    t.open[j - 1][lane] = g;
+  }
+}
+
+// One task of a warp: its boundary nodes updated. vs: the step's wall speeds; parity: the step's; outlets:
+// the outlet tasks of the block that wait for *s_drho (an outlet task; 0: no target); un_new: the
+// outlet velocities after the step.
+template <class S, int CK>
+__device__ __forceinline__ void boundary_task(const StepParams& p, const ResidentParams& r, const int4& nd, const int4& td,
+                                              const S* a, S* b, const double* vs, int parity, int outlets,
+                                              const double* s_drho, double* un_new, TaskScratch<typename Store<S>::R>& t) {
+  using R = typename Store<S>::R;
+  const int lane = (int)(threadIdx.x & 31u);
+  const unsigned cell = (unsigned)nd.x;
+  R f[9];
+  if (nd.x >= 0) pull_node(a, p.ns, p.nx, p.ny, cell, nd.y, f);
+  const R* own = &t.own[parity][0][0];
+  constexpr int U = 3;                                          // links of a lane in flight
+  for (int base = td.x + lane; base < td.y; base += U * 32) {
+    R bval[U];
+    unsigned slot[U], meta[U];
+#pragma unroll
+    for (int m = 0; m < U; ++m) {
+      const int l = base + m * 32;
+      if (l < td.y) {
+        const uint4 w = __ldg(reinterpret_cast<const uint4*>(r.walls + l));
+        slot[m] = w.y;
+        meta[m] = w.z;
+        if ((w.z & 3u) == WALL_NEAR) bval[m] = Store<S>::ld_cg(a + w.x, (int)(w.y / 32) + 1);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < U; ++m) {
+      const int l = base + m * 32;
+      if (l < td.y) {
+        const double2 cc = __ldg(reinterpret_cast<const double2*>(r.walls + l) + 1);
+        const R corr = (R)__ldg(&r.walls[l].cu6) * (R)vs[(meta[m] >> 2) & 3u];
+        const unsigned type = meta[m] & 3u;
+        const int j = (int)(slot[m] / 32) + 1, node = (int)(slot[m] & 31u);
+        const R out = own[j * 32 + node];
+        const R x3 = type == WALL_NEAR ? bval[m] : own[opp_of(j) * 32 + node];
+        R back = type == WALL_NEAR ? out : out - corr;
+        if (type != WALL_HALF) back = (R)cc.x * back + (R)cc.y * x3;
+        if (type == WALL_NEAR) back = back - corr;
+        t.back[j - 1][node] = back;
+      }
+    }
+  }
+  double drho = 0.0;
+  __syncwarp();
+  if (outlets > 0) {
+    outlet_sum_wait(outlets);
+    drho = *s_drho;
+  }
+  if (nd.x < 0) return;
+  if (td.z != TASK_WALL) {
+#pragma unroll
+    for (int j = 1; j < 9; ++j) {
+      if ((nd.y >> (j + 9)) & 1) {
+        R back = t.open[j - 1][lane];
+        if (td.z == TASK_OUTLET && ((nd.y >> (j + 18)) & 1)) {
+          const R rho_w = t.back[j - 1][lane] + (R)drho;        // (open_prepare left the link's density here)
+          back = -own[j * 32 + lane] + R(2.0) * (R)w_of(j) * rho_w * back;
+        }
+        f[opp_of(j)] = back;
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 1; j < 9; ++j)
+    if ((nd.y >> j) & 1) f[opp_of(j)] = t.back[j - 1][lane];
+  collide_s<S>(f, CK, (R)p.op, (R)p.om, (R)p.gx, (R)p.gy);
+#pragma unroll
+  for (int i = 0; i < 9; ++i) Store<S>::st(b + (unsigned)i * p.ns + cell, i, f[i]);
+#pragma unroll
+  for (int i = 0; i < 9; ++i) f[i] = Store<S>::rt(i, f[i]);
+  if (td.z == TASK_OUTLET) {
+    double fd[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) fd[i] = (double)f[i];
+    __stcg(un_new + nd.w, outlet_velocity(fd, p, nd.w));
+  }
+#pragma unroll
+  for (int i = 0; i < 9; ++i) t.own[parity ^ 1][i][lane] = f[i];
+}
+
+// The force terms of a task's nodes, per node in link order (after boundary_task).
+template <class S>
+__device__ __forceinline__ void task_force(const StepParams& p, const int4& nd, const double* vs, int parity,
+                                           double* node_force, const TaskScratch<typename Store<S>::R>& t) {
+  using R = typename Store<S>::R;
+  const int lane = (int)(threadIdx.x & 31u);
+  const unsigned fm = ((unsigned)nd.y >> 18) & 0x1ffu;
+  if (nd.x < 0 || !fm) return;
+  const unsigned all = ((unsigned)nd.y | ((unsigned)nd.y >> 9)) & 0x1ffu;
+  double acc[2 * kMaxGroups];
+#pragma unroll
+  for (int k = 0; k < 2 * kMaxGroups; ++k) acc[k] = 0.0;
+  for (int j = 1; j < 9; ++j) {
+    if (!((fm >> j) & 1u)) continue;
+    const LinkView L = load_link((const LinkRecDev*)p.links, nd.z + __popc(all & ((1u << j) - 1u)));
+    double tx, ty;
+    force_terms(L, (double)t.own[parity][j][lane], (double)t.back[j - 1][lane], (double)(R)vs[L.vgroup], tx, ty);
+#pragma unroll
+    for (int g = 0; g < kMaxGroups; ++g) {
+      if (g == L.fgroup) {
+        acc[2 * g] += tx;
+        acc[2 * g + 1] += ty;
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 2 * kMaxGroups; ++k)
+    if (k < 2 * p.ngroups) __stcg(node_force + (size_t)k * p.nbs + nd.w, acc[k]);
+}
+
+// Force sums and history record of step t by one part: per chunk with force the tree of
+// block_force_partial (a warp per chunk: kBlock / 32 groups of 32 nodes, then the groups in order), then
+// the tree of sum_partials by one warp per component (at most kBlock chunks). s_part[component][chunk] is
+// zero for the other chunks.
+template <class S>
+__device__ __forceinline__ void resident_epilogue(const StepParams& p, const ResidentParams& r, unsigned long long t,
+                                                  int slot, bool final_step, double (*s_part)[kBlock], double* s_force,
+                                                  const PartOf& me) {
+  Ctl* c = p.ctl;
+  const int tid = me.tid(), lane = tid & 31, warp = tid >> 5;
+  const int ncomp = 2 * p.ngroups;
+  const double* nf = r.node_force + (size_t)slot * ncomp * p.nbs;
+  for (int q = warp; q < r.nforce * ncomp; q += kBlock / 32) {
+    const int ch = __ldg(r.force_chunks + q / ncomp), k = q % ncomp;
+    double v[kBlock / 32];
+#pragma unroll
+    for (int w = 0; w < kBlock / 32; ++w) {
+      const int g = ch * kBlock + w * 32 + lane;
+      v[w] = g < p.nb ? __ldcg(nf + (size_t)k * p.nbs + g) : 0.0;
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+      for (int w = 0; w < kBlock / 32; ++w) v[w] += __shfl_down_sync(0xffffffffu, v[w], off);
+    }
+    double sum = 0.0;
+#pragma unroll
+    for (int w = 0; w < kBlock / 32; ++w) sum += v[w];
+    if (lane == 0) s_part[k][ch] = sum;
+  }
+  me.sync();
+  if (warp < ncomp) {
+    double v[kBlock / 32];
+#pragma unroll
+    for (int w = 0; w < kBlock / 32; ++w) v[w] = s_part[warp][w * 32 + lane];
+#pragma unroll
+    for (int h = kBlock / 64; h > 0; h >>= 1) {
+#pragma unroll
+      for (int w = 0; w < h; ++w) v[w] += v[w + h];
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v[0] += __shfl_down_sync(0xffffffffu, v[0], off);
+    if (lane == 0) s_force[warp] = v[0];
+  }
+  me.sync();
+  if (tid == 0) {
+    const int has_target = c->sched_on ? c->absorbing : c->has_target;
+    const double drho = p.np > 0 && has_target ? __ldcg(r.drho + slot) : 0.0;
+    bool finite = true;
+    for (int k = 0; k < ncomp; ++k) finite = finite && isfinite(s_force[k]);
+    if (!finite && !c->nonfinite) {
+      c->nonfinite = 1;
+      c->nonfinite_t = t;
+    }
+    if (c->rec_cap && t >= c->rec_start && t - c->rec_start < c->rec_cap) {
+      double* h = c->hist + (size_t)(t - c->rec_start) * kRec;
+      for (int k = 0; k < 2 * kMaxGroups; ++k) h[k] = k < ncomp ? s_force[k] : 0.0;
+      h[8] = drho;
+      if (!c->dp_on) h[9] = 0.0;                                // else the probe, one step before this
+    }
+    if (final_step) {
+      for (int k = 0; k < 2 * kMaxGroups; ++k) c->force[k] = k < ncomp ? s_force[k] : 0.0;
+      c->drho = drho;
+      if (c->sched_on) {
+        const Controls k = read_controls(c, t);
+        c->vscale[1] = k.vs[1];
+        c->vscale[2] = k.vs[2];
+        c->target = k.target;
+        c->has_target = k.has_target;
+      }
+      c->t = t + 1;
+    }
+  }
+  me.sync();
+}
+
+template <class S, int V, int CK>
+__global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_constant__ StepParams p,
+                                                                  const __grid_constant__ ResidentParams r, S* buf0,
+                                                                  S* buf1) {
+  using R = typename Store<S>::R;
+  __shared__ double s_part[2 * kMaxGroups][kBlock];             // the last part's chunk sums
+  __shared__ double s_force[2 * kMaxGroups];
+  __shared__ double s_vs[2][4];                                 // by parity of the step
+  __shared__ double s_target[2];
+  __shared__ unsigned long long s_t;
+  __shared__ int s_next[2];                                     // next segment of the block, by parity
+  __shared__ int s_go;
+  __shared__ double s_drho;
+  extern __shared__ double s_dyn[];
+  const int bid = (int)blockIdx.x, lane = (int)(threadIdx.x & 31u), warp = (int)threadIdx.x >> 5;
+  Ctl* c = p.ctl;
+  const unsigned long long t0 = c->t;
+  const int seg0 = __ldg(r.seg_first + bid), seg1 = __ldg(r.seg_first + bid + 1);
+  const int task0 = __ldg(r.task_first + bid), task1 = __ldg(r.task_first + bid + 1);
+  const PartOf me{(int)threadIdx.x / kBlock};
+  const bool last = bid == r.grid - 1 && me.part == kResidentSumPart;
+  const int has_target = c->sched_on ? c->absorbing : c->has_target;
+  double* s_un = s_dyn;                                         // the summing warp's outlet velocities
+  TaskScratch<R>* scratch = (TaskScratch<R>*)(s_dyn + (p.np + 1) / 2 * 2);
+  const int outlets = has_target ? __ldg(r.block_outlets + bid) : 0;
+  const size_t force_set = (size_t)2 * p.ngroups * p.nbs;
+
+  // controls of step s into shared memory (one thread)
+  auto controls = [&](int s) {
+    const Controls k = read_controls(c, t0 + (unsigned long long)s);
+#pragma unroll
+    for (int g = 0; g < 4; ++g) s_vs[s & 1][g] = k.vs[g];
+    s_target[s & 1] = k.target;
+    s_t = t0 + (unsigned long long)s;
+    s_next[s & 1] = seg0;
+  };
+
+  if (threadIdx.x == 0) controls(0);
+  for (int k = (int)threadIdx.x; k < 2 * kMaxGroups * kBlock; k += kResidentThreads) (&s_part[0][0])[k] = 0.0;
+  // Outlet velocities of the start state; every block computes all of them into the same values, so
+  // no grid-wide wait is needed before the first step.
+  for (int k = (int)threadIdx.x; k < p.np; k += kResidentThreads) {
+    const int idx = __ldg(p.pnode_idx + k);
+    double f[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) f[i] = (double)Store<S>::ld_cg(buf0 + (size_t)i * p.ns + idx, i);
+    __stcg(r.un + k, outlet_velocity(f, p, k));
+  }
+  __threadfence();
+  // The nodes' own populations in the start state.
+  if (warp < kResidentTaskWarps) {
+    for (int task = task0 + warp; task < task1; task += kResidentTaskWarps) {
+      const int4 nd = __ldg(r.nodes + (size_t)task * 32 + lane);
+      TaskScratch<R>& t = scratch[task - task0];
+      if (nd.x >= 0) {
+#pragma unroll
+        for (int d = 0; d < 9; ++d) t.own[0][d][lane] = Store<S>::ld_cg(buf0 + (unsigned)d * p.ns + (unsigned)nd.x, d);
+      }
+      open_prepare<S>(p, nd, __ldg(r.tasks + task).z, 0, t);
+    }
+  }
+  __syncthreads();
+
+  unsigned target = r.arrived0;
+  int slot = 0;                                                 // step s: slot s % 3
+  for (int s = 0; s < r.steps; ++s) {
+    const S* a = (s & 1) ? buf1 : buf0;
+    S* b = (s & 1) ? buf0 : buf1;
+    const int slot2 = slot == 2 ? 0 : slot + 1;                 // (s - 2) % 3
+
+    if (last) {
+      if (s > 0) record_probe<S>(p, a, (long long)(t0 + s) - 1, me);
+      if (s > 1) resident_epilogue<S>(p, r, t0 + s - 2, slot2, false, s_part, s_force, me);
+    } else if (warp < kResidentTaskWarps) {
+      for (int task = task0 + warp; task < task1; task += kResidentTaskWarps) {
+        const int4 nd = __ldg(r.nodes + (size_t)task * 32 + lane), td = __ldg(r.tasks + task);
+        boundary_task<S, CK>(p, r, nd, td, a, b, s_vs[s & 1], s & 1, td.z == TASK_OUTLET ? outlets : 0, &s_drho,
+                             r.un + ((s & 1) ^ 1) * p.np, scratch[task - task0]);
+        __syncwarp();
+      }
+    } else if (outlets > 0 && warp == kResidentWarps - 1) {
+      const double* un = r.un + (s & 1) * p.np;
+      for (int base = 0; base < p.np; base += 16 * 32) {        // 16 loads of a lane in flight
+        double v[16];
+#pragma unroll
+        for (int m = 0; m < 16; ++m)
+          if (base + m * 32 + lane < p.np) v[m] = __ldcg(un + base + m * 32 + lane);
+#pragma unroll
+        for (int m = 0; m < 16; ++m)
+          if (base + m * 32 + lane < p.np) s_un[base + m * 32 + lane] = v[m];
+      }
+      __syncwarp();
+      const double drho = (serial_sum(s_un, p.np) / (double)p.np - s_target[s & 1]) / p.sqrt_cs2;
+      if (lane == 0) {
+        s_drho = drho;
+        __stcg(r.drho + slot, drho);                            // (every block with outlet tasks writes this value)
+      }
+      __syncwarp();
+      outlet_sum_ready(outlets);
+    }
+
+    while (true) {
+      int sg = 0;
+      if (lane == 0) sg = atomicAdd(&s_next[s & 1], 1);
+      sg = __shfl_sync(0xffffffffu, sg, 0);
+      if (sg >= seg1) break;
+      const int y = sg / r.segs_per_row;
+      const int xw = (sg - y * r.segs_per_row) * (32 * V);
+      if constexpr (V > 1) {
+        PairTask q;
+        q.nx = p.nx;
+        q.ny = p.ny;
+        q.y = y;
+        q.xw = xw;
+        q.ns = p.ns;
+        q.flag = p.flag;
+        q.ck = CK;
+        q.op = (float)p.op;
+        q.om = (float)p.om;
+        q.bad = &c->nonfinite;
+        q.bad_t = &c->nonfinite_t;
+        q.t_now = &s_t;
+        group_update<S, V, 0, 1>(q, a, b);
+      } else {
+        const int x = xw + lane;
+        if (x < p.nx) {
+          const unsigned idx = (unsigned)(y * p.nx + x);
+          const uint8_t fl = __ldg(p.flag + idx);
+          R f[9];
+          pull<S, 1>(a, p.ns, p.nx, p.ny, x, y, f);
+          if (fl == 0) {
+            collide_s<S>(f, CK, (R)p.op, (R)p.om, (R)p.gx, (R)p.gy);
+            if (Saturates<S>::value && !density_plausible(f)) mark_diverged(&c->nonfinite, &c->nonfinite_t, &s_t);
+#pragma unroll
+            for (int i = 0; i < 9; ++i) Store<S>::st(b + (unsigned)i * p.ns + idx, i, f[i]);
+          }
+        }
+      }
+    }
+
+    grid_arrive(r.arrived);
+    target += (unsigned)r.grid;
+    // After the arrival (the block has synchronised: the step's controls and counter are free).
+    if (warp < kResidentTaskWarps) {
+      for (int task = task0 + warp; task < task1; task += kResidentTaskWarps) {
+        const int4 nd = __ldg(r.nodes + (size_t)task * 32 + lane);
+        const int kind = __ldg(r.tasks + task).z;
+        TaskScratch<R>& t = scratch[task - task0];
+        if (kind == TASK_OUTLET || kind == TASK_OPEN) open_prepare<S>(p, nd, kind, (s & 1) ^ 1, t);
+        if (kind != TASK_OUTLET) task_force<S>(p, nd, s_vs[s & 1], s & 1, r.node_force + slot * force_set, t);
+      }
+    }
+    if (threadIdx.x == kResidentThreads - 32) controls(s + 1);
+    if (threadIdx.x == kResidentThreads - 64) {
+      s_go = poll_arrived(r.arrived, target);
+      if (!s_go) c->stalled = 1;
+    }
+    __syncthreads();
+    if (!s_go) return;
+    slot = slot2;
+  }
+  // The force terms of the last step are complete after one more arrival.
+  grid_arrive(r.arrived);
+  target += (unsigned)r.grid;
+  if (bid != r.grid - 1) return;
+  if (threadIdx.x == 0) {
+    s_go = poll_arrived(r.arrived, target);
+    if (!s_go) c->stalled = 1;
+  }
+  __syncthreads();
+  if (!s_go || !last) return;
+  record_probe<S>(p, (r.steps & 1) ? buf1 : buf0, (long long)(t0 + r.steps) - 1, me);
+  if (r.steps > 1) resident_epilogue<S>(p, r, t0 + r.steps - 2, slot == 2 ? 0 : slot + 1, false, s_part, s_force, me);
+  resident_epilogue<S>(p, r, t0 + r.steps - 1, slot == 0 ? 2 : slot - 1, true, s_part, s_force, me);
+}
+
+}  // namespace vl
