@@ -1,0 +1,470 @@
+// Convolutions of the warm-start network as implicit GEMMs on tcgen05 (3x3, padding 1, stride 1 or 2,
+// or 1x1; NHWC BF16 activations, FP32 accumulation): the operand that im2col would write out is loaded
+// tap by tap with TMA boxes of the activation tensor itself (4-D map C, W, H, B; the box of a tile is
+// shifted by the tap, and what lies outside the image reads as zero, which is the padding).
+//
+// The K order is that of the im2col matrix, (tap, channel), in tensor-core steps of 16: every product
+// is accumulated in the order in which the GEMM over the materialised matrix accumulates it, so the
+// results are the same bit for bit.
+//
+//   k_conv    y[pixel, n] = epilogue(sum over (tap, c) of x[pixel + tap, c] w[n, (tap, c)]): the forward
+//             pass, and the input gradient of a stride-1 layer (dz with mirrored weights). Persistent:
+//             a block takes tiles of 128 pixels (bw x bh of one image) x bn channels in turn; warp 0
+//             loads, warp 1 issues the MMAs, warps 2-5 read the accumulator of one tile while the next
+//             is computed in the other (two accumulators in TMEM).
+//   k_wgrad   gw[(tap, c), n] = sum over pixels of x[pixel + tap, c] dz[pixel, n]: both operands MN-major,
+//             64 pixels of K at a time in row order, split over K as the plain GEMM splits it.
+//
+// Bound: the tile loads (x nine times through the L2, one box a tap) instead of the HBM round trip of the
+// nine-fold matrix. B200, batch 16, us of im2col + GEMM -> k_conv: 128 x 256 pixels 32 -> 32 channels 129 +
+// 76 -> 56, 96 -> 32 340 + 185 -> 144; 64 x 128 64 -> 64 63 + 55 -> 23, 192 -> 64 170 + 103 -> 53; 32 x 64
+// 128 -> 128 35 + 41 -> 19; 16 x 32 256 -> 256 21 + 39 -> 23. Weight gradients, GEMM over the matrix -> k_wgrad:
+// 32 x 32 87 -> 67, 96 x 32 215 -> 164, 64 x 64 42 -> 27, 128 x 128 45 -> 25.
+// Every wait on an mbarrier is bounded, as in vl_gemm.cuh.
+#pragma once
+
+#include "vl_gemm.cuh"
+
+namespace vl {
+namespace gemm {
+
+constexpr int kConvThreads = 192;
+constexpr int kConvMaxStages = 8;
+
+struct ConvParams {
+  int tiles, tiles_x, tiles_y;   // 128-pixel tiles: all, per row of tiles, per image
+  int bw, bh, log2_bw;           // pixels of a tile (bw * bh = 128)
+  int Ho, Wo, stride;
+  int taps, chunks;              // 9 or 1; KC-channel chunks of C
+  int pad;
+  int stages, bn, tmem_cols;     // tmem_cols: columns of one accumulator (a power of two)
+  int kb_split;                  // K blocks accumulated before the partial sum is added to `out` (all: kblocks)
+  EpiParams ep;
+};
+
+__device__ __forceinline__ void tma_load_4d(const CUtensorMap* map, uint64_t* bar, void* dst, int c, int x, int y, int b) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(
+          smem_u32(dst)),
+      "l"(map), "r"(smem_u32(bar)), "r"(c), "r"(x), "r"(y), "r"(b)
+      : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// K-major tile of 32-channel rows with 64-byte swizzle: rows of 64 bytes, 8-row (512-byte) atoms.
+__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((addr >> 4) & 0x3FFFu);
+  d |= (uint64_t)1u << 16;
+  d |= (uint64_t)(512u >> 4) << 32;
+  d |= (uint64_t)1u << 46;
+  d |= (uint64_t)4u << 61;   // SWIZZLE_64B
+  return d;
+}
+
+// MN-major tile of 32-wide column blocks with 64-byte swizzle: 8 K rows of 64 bytes form a 512-byte atom;
+// the next 8 K rows follow it, the next 32 columns are 64 K rows = 4096 bytes on.
+__device__ __forceinline__ uint64_t smem_desc_sw64_mn(uint32_t addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((addr >> 4) & 0x3FFFu);
+  d |= (uint64_t)(4096u >> 4) << 16;
+  d |= (uint64_t)(512u >> 4) << 32;
+  d |= (uint64_t)1u << 46;
+  d |= (uint64_t)4u << 61;
+  return d;
+}
+
+__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+      "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
+}
+
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)));
+}
+
+__device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t* v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+        "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+      : "r"(addr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+template <int KC>
+__host__ __device__ constexpr int conv_stage_bytes(int bn) {
+  return (BM + bn) * KC * 2;
+}
+
+template <int KC>
+__global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant__ CUtensorMap tmA,
+                                                          const __grid_constant__ CUtensorMap tmB,
+                                                          const __grid_constant__ ConvParams p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t full[kConvMaxStages], empty[kConvMaxStages], tfull[2], tempty[2];
+  __shared__ uint32_t tmem_base;
+  __shared__ int failed, issued_loads;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = (int)blockIdx.y * p.bn;
+  const int kblocks = p.taps * p.chunks;
+  const int stage_bytes = conv_stage_bytes<KC>(p.bn);
+  const EpiParams& ep = p.ep;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&tfull[i], 1);
+      mbar_init(&tempty[i], 4);
+    }
+    failed = 0;
+    issued_loads = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
+                 "r"((uint32_t)(2 * p.tmem_cols)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = tmem_base;
+
+  if (threadIdx.x == 0) {
+    // loads: the stages of the ring in turn, in tile and K order (the counters are kept, not divided: a
+    // division in this loop costs as much as the load it issues)
+    int s = 0, issued = 0;
+    uint32_t phase = 1;                         // of the empty barriers: the first round passes at once
+    bool ok = true;
+    for (int t = (int)blockIdx.x; t < p.tiles && ok; t += (int)gridDim.x) {
+      const int per = p.tiles_x * p.tiles_y;
+      const int b = t / per, q = t - b * per, ty = q / p.tiles_x, tx = q - ty * p.tiles_x;
+      const int x0 = tx * p.bw * p.stride - p.pad, y0 = ty * p.bh * p.stride - p.pad;
+      int ky = 0, kx = 0, c0 = 0;
+      for (int kb = 0; kb < kblocks; ++kb) {
+        if (!mbar_wait(&empty[s], phase, ep.spin_limit)) {
+          atomicExch(&failed, 1);
+          ok = false;
+          break;
+        }
+        uint8_t* sa = smem + s * stage_bytes;
+        mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
+        tma_load_4d(&tmA, &full[s], sa, c0, x0 + kx, y0 + ky, b);
+        tma_load_2d(&tmB, &full[s], sa + BM * KC * 2, kb * KC, n0);
+        ++issued;
+        if (++s == p.stages) {
+          s = 0;
+          phase ^= 1;
+        }
+        c0 += KC;
+        if (c0 == p.chunks * KC) {
+          c0 = 0;
+          if (++kx == 3) {
+            kx = 0;
+            ++ky;
+          }
+        }
+      }
+    }
+    issued_loads = issued;
+  } else if (threadIdx.x == 32) {
+    const uint32_t idesc = instr_desc_bf16(p.bn);
+    int s = 0, n = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = (int)blockIdx.x; t < p.tiles && ok; t += (int)gridDim.x) {
+      int left = 0, buf = 0;
+      uint32_t acc = 0;
+      for (int kb = 0; kb < kblocks; ++kb) {
+        const bool fresh = left == 0;
+        if (fresh) {                            // the next accumulator, once it has been read
+          buf = n & 1;
+          if (!mbar_wait(&tempty[buf], ((uint32_t)(n >> 1) & 1u) ^ 1u, ep.spin_limit)) {
+            atomicExch(&failed, 1);
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;");
+          acc = tmem + (uint32_t)(buf * p.tmem_cols);
+          left = min(p.kb_split, kblocks - kb);
+          ++n;
+        }
+        if (!mbar_wait(&full[s], phase, ep.spin_limit)) {
+          atomicExch(&failed, 1);
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const uint32_t a_addr = smem_u32(smem + s * stage_bytes), b_addr = a_addr + BM * KC * 2;
+        const uint64_t da = KC == 64 ? smem_desc_sw128(a_addr) : smem_desc_sw64(a_addr);
+        const uint64_t db = KC == 64 ? smem_desc_sw128(b_addr) : smem_desc_sw64(b_addr);
+#pragma unroll
+        for (int k = 0; k < KC / 16; ++k) mma_bf16(acc, da + 2u * k, db + 2u * k, idesc, (!fresh || k > 0) ? 1u : 0u);
+        mma_commit(&empty[s]);
+        if (--left == 0) mma_commit(&tfull[buf]);
+        if (++s == p.stages) {
+          s = 0;
+          phase ^= 1;
+        }
+      }
+    }
+  } else if (warp >= 2) {
+    // epilogue: a warp reads the 32 rows of its TMEM lanes (its number modulo 4), a row per lane
+    const int rows = (warp & 3) * 32;
+    const int parts = (kblocks + p.kb_split - 1) / p.kb_split;
+    int n = 0;
+    bool ok = true;
+    for (int t = (int)blockIdx.x; t < p.tiles && ok; t += (int)gridDim.x)
+    for (int z = 0; z < parts; ++z, ++n) {
+      const int buf = n & 1;
+      const bool add = z > 0 || (ep.flags & EPI_ACCUM);
+      if (!mbar_wait(&tfull[buf], (uint32_t)(n >> 1) & 1u, ep.spin_limit)) {
+        atomicExch(&failed, 1);
+        ok = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const int per = p.tiles_x * p.tiles_y;
+      const int b = t / per, q = t - b * per, ty = q / p.tiles_x, tx = q - ty * p.tiles_x;
+      const int m = rows + lane;
+      const int x = tx * p.bw + (m & (p.bw - 1)), y = ty * p.bh + (m >> p.log2_bw);
+      const bool valid = x < p.Wo && y < p.Ho;
+      const size_t row = ((size_t)b * p.Ho + y) * p.Wo + x;
+      for (int c0 = 0; c0 < p.bn; c0 += 32) {
+        uint32_t v[32];
+        tmem_ld32(tmem + (uint32_t)(buf * p.tmem_cols + c0) + ((uint32_t)rows << 16), v);
+        if (valid) {
+          const int cols = min(32, ep.n_valid - (n0 + c0));
+#pragma unroll
+          for (int j = 0; j < 32; j += 4) {
+            float4 bv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if ((ep.flags & EPI_BIAS) && j < cols) bv = __ldg(reinterpret_cast<const float4*>(ep.bias + n0 + c0 + j));
+            const float bj[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              float f = __uint_as_float(v[j + i]) + bj[i];
+              if (ep.flags & EPI_RELU) f = fmaxf(f, 0.0f);
+              v[j + i] = __float_as_uint(f);
+            }
+          }
+          // 32 bytes a store: whole sectors, though a lane's row lies apart from its neighbours'
+          if (ep.flags & EPI_BF16) {
+            __nv_bfloat16* o = (__nv_bfloat16*)ep.out + row * ep.ldc + n0 + c0;
+#pragma unroll
+            for (int j = 0; j < 32; j += 8) {
+              if (j < cols) {                   // (the column count is a multiple of 8)
+                uint32_t u[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[j + 2 * i]), __uint_as_float(v[j + 2 * i + 1]));
+                  u[i] = *reinterpret_cast<const uint32_t*>(&h);
+                }
+                *reinterpret_cast<uint4*>(o + j) = make_uint4(u[0], u[1], u[2], u[3]);
+              }
+            }
+          } else {
+            float* o = (float*)ep.out + row * ep.ldc + n0 + c0;
+#pragma unroll
+            for (int j = 0; j < 32; j += 8) {
+              if (j < cols) {
+                if (add) {
+                  const float4 e0 = *reinterpret_cast<const float4*>(o + j), e1 = *reinterpret_cast<const float4*>(o + j + 4);
+                  const float e[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+#pragma unroll
+                  for (int i = 0; i < 8; ++i) v[j + i] = __float_as_uint(e[i] + __uint_as_float(v[j + i]));
+                }
+                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o + j), "r"(v[j]), "r"(v[j + 1]),
+                             "r"(v[j + 2]), "r"(v[j + 3]), "r"(v[j + 4]), "r"(v[j + 5]), "r"(v[j + 6]), "r"(v[j + 7])
+                             : "memory");
+              }
+            }
+          }
+        }
+        __syncwarp();
+      }
+      // the accumulator is read: the MMAs of the tile after the next may overwrite it
+      asm volatile("tcgen05.fence::before_thread_sync;");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty[buf]);
+    }
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (failed && threadIdx.x == 0) {
+    // drain (bounded): the copies that may still be landing in this block's shared memory
+    const int issued = issued_loads;
+    for (int it = issued > p.stages ? issued - p.stages : 0; it < issued; ++it)
+      mbar_wait(&full[it % p.stages], (uint32_t)(it / p.stages) & 1u, ep.spin_limit);
+    if (ep.err) atomicExch(ep.err, 1);
+  }
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(2 * p.tmem_cols)));
+}
+
+// ------------------------------------------------------------------ weight gradient
+struct WgradParams {
+  int Ho, Wo, stride, pad, taps;
+  int C;                         // channels; a K block is 64 pixels, of a row's part or of whole rows
+  int kblocks, kb_per, stages, bn;
+  EpiParams ep;                  // FP32 rows (tap, c) of `out`, split-K partial results split_stride apart
+};
+
+template <int KC>
+__host__ __device__ constexpr int wgrad_stage_bytes(int bn) {
+  return BM * 64 * 2 + bn * 64 * 2;
+}
+
+template <int KC>
+__global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtensorMap tmA,
+                                                  const __grid_constant__ CUtensorMap tmB,
+                                                  const __grid_constant__ WgradParams p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t full[kConvMaxStages], empty[kConvMaxStages], done;
+  __shared__ uint32_t tmem_base;
+  __shared__ int failed, issued_loads;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m0 = (int)blockIdx.x * BM, n0 = (int)blockIdx.y * p.bn;
+  const int kb_first = (int)blockIdx.z * p.kb_per;
+  const int kblocks = min(p.kblocks - kb_first, p.kb_per);
+  const int stage_bytes = wgrad_stage_bytes<KC>(p.bn);
+  const uint32_t tmem_cols = p.bn <= 32 ? 32u : (p.bn <= 64 ? 64u : (p.bn <= 128 ? 128u : 256u));
+  const EpiParams& ep = p.ep;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(&done, 1);
+    failed = 0;
+    issued_loads = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "r"(tmem_cols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = tmem_base;
+  if (threadIdx.x == 0) {
+    // the KC-wide column blocks of this tile: their tap and first channel (past the last: all zero)
+    constexpr int NB = BM / KC;
+    int kx[NB], ky[NB], c0[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int row = m0 + i * KC, tap = row / p.C;
+      c0[i] = row - tap * p.C;
+      ky[i] = tap < p.taps ? (p.taps == 9 ? tap / 3 : 0) : -(1 << 24);
+      kx[i] = p.taps == 9 ? tap % 3 : 0;
+    }
+    int issued = 0, s = 0;
+    uint32_t phase = 1;
+    int r0 = kb_first * 64;
+    int x = r0 % p.Wo, y = r0 / p.Wo, b = y / p.Ho;
+    y -= b * p.Ho;
+    for (int kb = 0; kb < kblocks; ++kb) {
+      if (!mbar_wait(&empty[s], phase, ep.spin_limit)) { atomicExch(&failed, 1); break; }
+      uint8_t* sa = smem + s * stage_bytes;
+      mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
+#pragma unroll
+      for (int i = 0; i < NB; ++i)
+        tma_load_4d(&tmA, &full[s], sa + i * (64 * KC * 2), c0[i], x * p.stride - p.pad + kx[i], y * p.stride - p.pad + ky[i], b);
+      for (int c = 0; c < p.bn / 64; ++c) tma_load_2d(&tmB, &full[s], sa + BM * 64 * 2 + 8192 * c, n0 + 64 * c, r0);
+      issued = kb + 1;
+      if (++s == p.stages) {
+        s = 0;
+        phase ^= 1;
+      }
+      r0 += 64;
+      if (p.Wo >= 64) {
+        x += 64;
+        if (x == p.Wo) {
+          x = 0;
+          ++y;
+        }
+      } else {
+        y += 64 / p.Wo;
+      }
+      if (y == p.Ho) {
+        y = 0;
+        ++b;
+      }
+    }
+    issued_loads = issued;
+  } else if (threadIdx.x == 32) {
+    const uint32_t idesc = instr_desc_bf16(p.bn, OP_A_MN | OP_B_MN);
+    int s = 0;
+    uint32_t phase = 0;
+    for (int kb = 0; kb < kblocks; ++kb) {
+      if (!mbar_wait(&full[s], phase, ep.spin_limit)) { atomicExch(&failed, 1); break; }
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const uint32_t a_addr = smem_u32(smem + s * stage_bytes), b_addr = a_addr + BM * 64 * 2;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        // 16 K rows further: two 8-row atoms
+        const uint64_t da = KC == 64 ? smem_desc_sw128_mn(a_addr + 2048u * k) : smem_desc_sw64_mn(a_addr + 1024u * k);
+        const uint64_t db = smem_desc_sw128_mn(b_addr + 2048u * k);
+        mma_bf16(tmem, da, db, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+      }
+      mma_commit(&empty[s]);
+      if (++s == p.stages) {
+        s = 0;
+        phase ^= 1;
+      }
+    }
+    mma_commit(&done);
+  }
+  __syncwarp();
+  const bool have = mbar_wait(&done, 0, ep.spin_limit);
+  if (!have) atomicExch(&failed, 1);
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  __syncthreads();
+  const bool good = !failed;
+  if (!good && threadIdx.x == 0) {
+    const int issued = issued_loads;
+    for (int kb = issued > p.stages ? issued - p.stages : 0; kb < issued; ++kb)
+      mbar_wait(&full[kb % p.stages], (uint32_t)(kb / p.stages) & 1u, ep.spin_limit);
+    if (ep.err) atomicExch(ep.err, 1);
+  }
+  if (good) {
+    const int row = m0 + warp * 32 + lane;
+    for (int c0 = 0; c0 < p.bn; c0 += 32) {
+      uint32_t v[32];
+      tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+      const int cols = min(32, ep.n_valid - (n0 + c0));
+      if (row < ep.m_valid) {
+        float* o = (float*)ep.out + (size_t)blockIdx.z * ep.split_stride + (size_t)row * ep.ldc + n0 + c0;
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+          if (j < cols)
+            *reinterpret_cast<float4*>(o + j) = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
+                                                            __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols));
+}
+
+}  // namespace gemm
+}  // namespace vl

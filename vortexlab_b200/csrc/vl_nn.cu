@@ -12,6 +12,7 @@
 #include <string>
 
 #include "../../include/vortexlab.h"
+#include "vl_conv.cuh"
 #include "vl_gemm.cuh"
 #include "vl_launch.hpp"
 
@@ -40,20 +41,45 @@ int encoder(PFN_cuTensorMapEncodeTiled_v12000* out) {
 
 // 2-D tensor map of a row-major BF16 matrix [rows][cols] with leading dimension ld (elements),
 // box = 64 columns x box_rows rows, 128-byte swizzle. Out-of-range boxes read zeros.
-int make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
+int make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows,
+             int box_cols = vl::gemm::BK) {
   PFN_cuTensorMapEncodeTiled_v12000 enc;
   int rc = encoder(&enc);
   if (rc) return rc;
   if (((uintptr_t)base & 15) || (ld * 2) % 16) return fail(VL_EINVAL, "GEMM operands need 16-byte aligned rows");
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {ld * 2};
-  cuuint32_t box[2] = {(cuuint32_t)vl::gemm::BK, box_rows};
+  cuuint32_t box[2] = {(cuuint32_t)box_cols, box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(VL_EINVAL, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
   return VL_OK;
+}
+
+// 4-D map (C, W, H, B) of NHWC BF16 activations; a box is kc channels x bw x bh pixels spaced `stride`
+// apart, rows of kc channels swizzled over their 128 or 64 bytes. Pixels outside the image read zero.
+int make_map_nhwc(CUtensorMap* map, const void* x, int B, int H, int W, int C, int stride, int kc, int bw, int bh) {
+  PFN_cuTensorMapEncodeTiled_v12000 enc;
+  int rc = encoder(&enc);
+  if (rc) return rc;
+  if (((uintptr_t)x & 15) || (C * 2) % 16) return fail(VL_EINVAL, "convolution operands need 16-byte aligned pixels");
+  cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
+  cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2};
+  cuuint32_t box[4] = {(cuuint32_t)kc, (cuuint32_t)(bw * stride), (cuuint32_t)(bh * stride), 1};
+  cuuint32_t estr[4] = {1, (cuuint32_t)stride, (cuuint32_t)stride, 1};
+  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(x), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, kc == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(VL_EINVAL, "cuTensorMapEncodeTiled (NHWC) failed (" + std::to_string((int)r) + ")");
+  return VL_OK;
+}
+
+int sm_count(int dev) {
+  int n = 0;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+  return n;
 }
 
 // Device workspace for split-K partial tiles, one per device, grown on demand. Split-K GEMMs of
@@ -83,15 +109,33 @@ int workspace(int dev, size_t bytes, void** out) {
 }
 
 // out[m, n] (leading dimension ldc) = (accumulate ? out : 0) + sum over z of ws[z][m][n], z in order.
+// Sixteen splits' values are loaded ahead of the additions: with few outputs (a thin layer: 2,048 values
+// of 296 splits) one thread's chain of loads was the time (53 us -> 9 us).
 __global__ void k_split_reduce(const float* __restrict__ ws, int splits, int M, int N, float* __restrict__ out,
                                int ldc, int accumulate) {
   const long long total = (long long)M * N;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     float s = 0.0f;
-    for (int z = 0; z < splits; ++z) s += ws[(long long)z * total + i];
+    int z = 0;
+    for (; z + 16 <= splits; z += 16) {
+      float v[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) v[k] = __ldcs(ws + (long long)(z + k) * total + i);
+#pragma unroll
+      for (int k = 0; k < 16; ++k) s += v[k];
+    }
+    for (; z < splits; ++z) s += ws[(long long)z * total + i];
     float* o = out + (i / N) * ldc + (i % N);
     *o = accumulate ? *o + s : s;
   }
+}
+
+int split_reduce(const float* ws, int splits, int M, int N, float* out, int ldc, int accumulate, cudaStream_t s) {
+  const long long total = (long long)M * N;
+  const int blocks = (int)std::min<long long>((total + 63) / 64, 148 * 32);
+  k_split_reduce<<<blocks, 64, 0, s>>>(ws, splits, M, N, out, ldc, accumulate);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? VL_OK : fail(VL_ECUDA, std::string("gemm split reduce: ") + cudaGetErrorString(e));
 }
 
 template <int BN>
@@ -140,13 +184,7 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int 
   vl::gemm::k_gemm_bf16<BN><<<grid, 128, vl::gemm::smem_bytes<BN>(stages), s>>>(ta, tb, kblocks, kb_per, stages, op, p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(VL_ECUDA, std::string("gemm launch: ") + cudaGetErrorString(e));
-  if (splits > 1) {
-    long long total = (long long)M * N;
-    int blocks = (int)std::min<long long>((total + 255) / 256, 148 * 8);
-    k_split_reduce<<<blocks, 256, 0, s>>>(ws, splits, M, N, (float*)ep.out, ep.ldc, ep.flags & vl::gemm::EPI_ACCUM);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return fail(VL_ECUDA, std::string("gemm split reduce: ") + cudaGetErrorString(e));
-  }
+  if (splits > 1) return split_reduce(ws, splits, M, N, (float*)ep.out, ep.ldc, ep.flags & vl::gemm::EPI_ACCUM, s);
   return VL_OK;
 }
 
@@ -184,6 +222,183 @@ int vl_nn_gemm_bf16(const void* a, int lda, const void* b, int ldb, int M, int N
     case 128: return launch_gemm<128>(ta, tb, M, N, K, op, ep, s);
     default: return launch_gemm<256>(ta, tb, M, N, K, op, ep, s);
   }
+}
+
+}  // extern "C"
+
+// ------------------------------------------------------------------ implicit convolutions
+namespace {
+
+template <int KC>
+int launch_conv(const CUtensorMap& ta, const CUtensorMap& tb, vl::gemm::ConvParams& p, int N, cudaStream_t s) {
+  using namespace vl::gemm;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const int stage = conv_stage_bytes<KC>(p.bn);
+  // Two blocks share an SM where their accumulators (2 x tmem_cols columns each) fit the 512 of its tensor
+  // memory: one's prologue and tail run beside the other's MMAs.
+  const int per_sm = 4 * p.tmem_cols <= 512 ? 2 : 1;
+  p.stages = std::min(kConvMaxStages, (per_sm == 2 ? 104 * 1024 : 208 * 1024) / stage);
+  const int smem = p.stages * stage + 1024;
+  static std::mutex m;
+  static bool configured[64] = {};
+  {
+    std::lock_guard<std::mutex> g(m);
+    if (dev >= 64 || !configured[dev]) {
+      cudaError_t e = cudaFuncSetAttribute(k_conv<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024);
+      if (e != cudaSuccess) return fail(VL_ECUDA, std::string("convolution smem attribute: ") + cudaGetErrorString(e));
+      if (dev < 64) configured[dev] = true;
+    }
+  }
+  const int gy = (N + p.bn - 1) / p.bn;
+  const int gx = std::max(1, std::min(p.tiles, per_sm * sm_count(dev) / gy));
+  k_conv<KC><<<dim3((unsigned)gx, (unsigned)gy), kConvThreads, smem, s>>>(ta, tb, p);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? VL_OK : fail(VL_ECUDA, std::string("convolution launch: ") + cudaGetErrorString(e));
+}
+
+template <int KC>
+int launch_wgrad(const CUtensorMap& ta, const CUtensorMap& tb, vl::gemm::WgradParams& p, int kp, int N, float* out,
+                 cudaStream_t s) {
+  using namespace vl::gemm;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const int gx = (kp + BM - 1) / BM, gy = (N + p.bn - 1) / p.bn;
+  // the split of launch_gemm for the same product, so that the partial sums are the same
+  int splits = 1;
+  const int tiles = gx * gy;
+  if (tiles < 148 && p.kblocks >= 16) splits = std::max(1, std::min(p.kblocks / 8, (296 + tiles - 1) / tiles));
+  p.kb_per = (p.kblocks + splits - 1) / splits;
+  splits = (p.kblocks + p.kb_per - 1) / p.kb_per;
+  p.ep.out = out;
+  p.ep.ldc = N;
+  p.ep.split_stride = 0;
+  if (splits > 1) {
+    void* w = nullptr;
+    int rc = workspace(dev, (size_t)splits * kp * N * sizeof(float), &w);
+    if (rc) return rc;
+    p.ep.out = w;
+    p.ep.split_stride = (long long)kp * N;
+  }
+  const int stage = wgrad_stage_bytes<KC>(p.bn);
+  p.stages = std::min(kConvMaxStages, 100 * 1024 / stage);
+  static std::mutex m;
+  static bool configured[64] = {};
+  {
+    std::lock_guard<std::mutex> g(m);
+    if (dev >= 64 || !configured[dev]) {
+      cudaError_t e = cudaFuncSetAttribute(k_wgrad<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 104 * 1024);
+      if (e != cudaSuccess) return fail(VL_ECUDA, std::string("weight gradient smem attribute: ") + cudaGetErrorString(e));
+      if (dev < 64) configured[dev] = true;
+    }
+  }
+  k_wgrad<KC><<<dim3((unsigned)gx, (unsigned)gy, (unsigned)splits), 128, p.stages * stage + 1024, s>>>(ta, tb, p);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return fail(VL_ECUDA, std::string("weight gradient launch: ") + cudaGetErrorString(e));
+  return splits > 1 ? split_reduce((const float*)p.ep.out, splits, kp, N, out, N, 0, s) : VL_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int vl_nn_conv_bf16(const void* x, int B, int H, int W, int C, int stride, int taps, const void* w, int kp, int N,
+                    void* out, int ldc, const float* bias, int flags, int* err, void* stream) {
+  using namespace vl::gemm;
+  if (!x || !w || !out || B < 1 || H < 1 || W < 1 || N < 1 || (stride != 1 && stride != 2) || (taps != 1 && taps != 9))
+    return fail(VL_EINVAL, "convolution: bad arguments");
+  if (C < 32 || C % 32 || kp % 8 || kp < taps * C || N % 8 || ldc % 8 || ((uintptr_t)out & 31) || ((uintptr_t)bias & 15))
+    return fail(VL_EINVAL, "convolution: channels in 32s, output channels in 8s, 32-byte aligned rows");
+  if ((flags & EPI_BIAS) && !bias) return fail(VL_EINVAL, "convolution: bias requested without a bias");
+  const int kc = C % 64 == 0 ? 64 : 32;
+  ConvParams p;
+  p.Ho = (H + stride - 1) / stride;
+  p.Wo = (W + stride - 1) / stride;
+  p.stride = stride;
+  p.taps = taps;
+  p.chunks = C / kc;
+  p.pad = taps == 9 ? 1 : 0;
+  // the tile shape with the fewest tiles (the widest of those)
+  long long best = 0;
+  for (int lw = 7; lw >= 3; --lw) {
+    const int bw = 1 << lw, bh = BM >> lw;
+    const long long n = (long long)((p.Wo + bw - 1) / bw) * ((p.Ho + bh - 1) / bh);
+    if (lw == 7 || n < best) {
+      best = n;
+      p.bw = bw;
+      p.bh = bh;
+      p.log2_bw = lw;
+    }
+  }
+  p.tiles_x = (p.Wo + p.bw - 1) / p.bw;
+  p.tiles_y = (p.Ho + p.bh - 1) / p.bh;
+  if (best * B > 0x7fffffffLL) return fail(VL_EINVAL, "convolution: too many pixels");
+  p.tiles = (int)(best * B);
+  // channels of a block: all of them up to 256, else equal parts in 32s; halves while the tiles are too few
+  // to give every SM one
+  int parts = (N + 255) / 256;
+  while (p.tiles * parts < 148 && N >= 64 * 2 * parts) parts *= 2;
+  p.bn = (N + parts - 1) / parts;
+  p.bn = p.bn <= 32 ? 32 : (p.bn + 63) / 64 * 64;
+  // FP32 results of few tiles: the K split of launch_gemm for the same product (there for more blocks),
+  // so that the sums are the same
+  p.kb_split = taps * p.chunks;
+  {
+    const int gbn = N <= 32 ? 32 : (N <= 64 ? 64 : (N <= 128 ? 128 : 256)), kb64 = (kp + BK - 1) / BK;
+    const long long gt = (((long long)B * p.Ho * p.Wo + BM - 1) / BM) * ((N + gbn - 1) / gbn);
+    if (gt < 148 && kb64 >= 16 && !(flags & (EPI_BIAS | EPI_RELU | EPI_BF16 | EPI_ACCUM))) {
+      const int splits = std::max(1, std::min(kb64 / 8, (int)((296 + gt - 1) / gt)));
+      p.kb_split = std::min(p.kb_split, (kb64 + splits - 1) / splits * (BK / kc));
+    }
+  }
+  p.tmem_cols = p.bn <= 32 ? 32 : (p.bn <= 64 ? 64 : (p.bn <= 128 ? 128 : 256));
+  p.ep = EpiParams{};
+  p.ep.out = out;
+  p.ep.ldc = ldc;
+  p.ep.bias = bias;
+  p.ep.n_valid = N;
+  p.ep.flags = flags & (EPI_ACCUM | EPI_BIAS | EPI_RELU | EPI_BF16);
+  p.ep.err = err;
+  p.ep.spin_limit = kSpinLimit;
+  CUtensorMap ta, tb;
+  int rc = make_map_nhwc(&ta, x, B, H, W, C, stride, kc, p.bw, p.bh);
+  if (rc) return rc;
+  rc = make_map(&tb, w, (uint64_t)N, (uint64_t)kp, (uint64_t)kp, (uint32_t)p.bn, kc);
+  if (rc) return rc;
+  return kc == 64 ? launch_conv<64>(ta, tb, p, N, (cudaStream_t)stream) : launch_conv<32>(ta, tb, p, N, (cudaStream_t)stream);
+}
+
+int vl_nn_wgrad_bf16(const void* x, int B, int H, int W, int C, int stride, const void* dz, int N, float* gwt, int kp,
+                     int* err, void* stream) {
+  using namespace vl::gemm;
+  if (!x || !dz || !gwt || B < 1 || H < 1 || W < 1 || N < 1 || (stride != 1 && stride != 2))
+    return fail(VL_EINVAL, "weight gradient: bad arguments");
+  const int Ho = (H + stride - 1) / stride, Wo = (W + stride - 1) / stride;
+  const int bw = Wo % 64 == 0 ? 64 : Wo;
+  if (C < 32 || C % 32 || kp < 9 * C || N % 8 || ((uintptr_t)gwt & 15) || bw > 64 || 64 % bw || Ho % (64 / bw))
+    return fail(VL_EINVAL, "weight gradient: channels in 32s, output rows that 64-pixel blocks divide");
+  const int kc = C % 64 == 0 ? 64 : 32;
+  WgradParams p;
+  p.Ho = Ho;
+  p.Wo = Wo;
+  p.stride = stride;
+  p.pad = 1;
+  p.taps = 9;
+  p.C = C;
+  p.kblocks = (int)((long long)B * Ho * Wo / 64);
+  p.bn = N <= 64 ? 64 : (N <= 128 ? 128 : 256);
+  p.ep = EpiParams{};
+  p.ep.m_valid = kp;
+  p.ep.n_valid = N;
+  p.ep.err = err;
+  p.ep.spin_limit = kSpinLimit;
+  CUtensorMap ta, tb;
+  int rc = make_map_nhwc(&ta, x, B, H, W, C, stride, kc, bw, 64 / bw);
+  if (rc) return rc;
+  rc = make_map(&tb, dz, (uint64_t)B * Ho * Wo, (uint64_t)N, (uint64_t)N, 64u);
+  if (rc) return rc;
+  return kc == 64 ? launch_wgrad<64>(ta, tb, p, kp, N, gwt, (cudaStream_t)stream)
+                  : launch_wgrad<32>(ta, tb, p, kp, N, gwt, (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -9,10 +9,12 @@ of a lower level has stride 2); the decoder upsamples 2x (nearest), concatenates
 level, and applies two 3x3 convolutions; a 1x1 convolution gives the output. With levels = 4 and
 c0 = 32 it has 1.95 M parameters.
 
-Every convolution is an im2col gather plus a BF16 GEMM on the tcgen05 tensor cores with FP32
-accumulation (vl_nn_gemm_bf16); its backward pass is two more GEMMs (weights: cols^T dz, with both
-operands read MN-major where they lie, no transposes; data: the im2col of dz times the mirrored
-weights for stride-1 layers, dz W^T then col2im for stride 2).
+Every convolution is a BF16 product on the tcgen05 tensor cores with FP32 accumulation, whose
+operand tiles are loaded tap by tap from the activations (vl_nn_conv_bf16; no im2col matrix); its
+backward pass is two more (weights: x^T dz, both operands read MN-major where they lie,
+vl_nn_wgrad_bf16; data: dz with the mirrored weights for stride-1 layers, dz W^T then col2im for
+stride 2). The 4-channel input layer, and weight gradients on grids that 64-pixel blocks do not
+divide, go through the materialised im2col matrix and vl_nn_gemm_bf16.
 Master weights and Adam moments are FP32. torch provides device memory only: every arithmetic
 operation on the device runs in this library's kernels.
 
@@ -135,11 +137,16 @@ class Conv:
         self.ho, self.wo = (h + self.stride - 1) // self.stride, (w + self.stride - 1) // self.stride
         self.rows = B * self.ho * self.wo
         bf = dict(dtype=torch.bfloat16, device="cuda")
-        self.cols = torch.zeros(self.rows, self.kp, **bf) if self.k == 3 else None
+        self.direct = self.cin % 32 == 0 and self.cout % 8 == 0
+        w64 = 64 if self.wo % 64 == 0 else self.wo
+        self.direct_w = self.direct and self.k == 3 and 64 % w64 == 0 and self.ho % (64 // w64) == 0
+        # the im2col matrix, where a product still goes through it
+        self.cols = torch.zeros(self.rows, self.kp, **bf) if self.k == 3 and not (self.direct and self.direct_w) else None
         self.flip = self.k == 3 and self.stride == 1
         if self.flip:       # input gradient as a convolution of dz with mirrored weights
             self.kpf = _kp(9 * self.cout)
-            self.dcols = torch.zeros(self.rows, self.kpf, **bf)
+            self.direct_x = self.cout % 32 == 0 and self.cin % 8 == 0
+            self.dcols = None if self.direct_x else torch.zeros(self.rows, self.kpf, **bf)
             self.wf = torch.zeros(self.cin, self.kpf, **bf)
         elif self.k == 3:   # stride 2: dz W^T, then col2im
             self.dcols = torch.zeros(self.rows, self.kp, dtype=torch.float32, device="cuda")
@@ -151,14 +158,25 @@ class Conv:
     def forward(self, x, err):
         """x: BF16 [B, h, w, cin] (contiguous). Returns y: BF16 (ReLU layers) or FP32 [rows, cout]."""
         self.x = x
-        if self.k == 3:
-            check(lib.vl_nn_im2col(_p(x), self.B, self.h, self.wd, self.cin, self.stride, self.kp, _p(self.cols), None))
-            a = self.cols
-        else:
-            a = x
+        self.has_cols = False
         flags = EPI_BIAS | ((EPI_RELU | EPI_BF16) if self.relu else 0)
-        gemm(a, self.kp, self.wb, self.kp, self.rows, self.cout, self.kp, self.y, self.cout, flags, self.b, err)
+        if self.direct:
+            check(lib.vl_nn_conv_bf16(_p(x), self.B, self.h, self.wd, self.cin, self.stride, self.k * self.k, _p(self.wb),
+                                      self.kp, self.cout, _p(self.y), self.cout, _fp(self.b), flags,
+                                      err.ptr() if err is not None else None, None))
+            return self.y
+        gemm(self._im2col(), self.kp, self.wb, self.kp, self.rows, self.cout, self.kp, self.y, self.cout, flags, self.b, err)
         return self.y
+
+    def _im2col(self):
+        """The left operand [rows, kp] of the layer's product: its im2col matrix, gathered once per
+        forward pass, or the input itself (1x1)."""
+        if self.k != 3:
+            return self.x
+        if not self.has_cols:
+            check(lib.vl_nn_im2col(_p(self.x), self.B, self.h, self.wd, self.cin, self.stride, self.kp, _p(self.cols), None))
+            self.has_cols = True
+        return self.cols
 
     def backward(self, dy, dx, accumulate, err, need_dx=True):
         """dy: FP32 [rows, cout], the gradient of the layer output. Writes (or, with `accumulate`,
@@ -167,12 +185,21 @@ class Conv:
                                 _p(self.dz), None, _p(self.colsum), None))
         check(lib.vl_nn_bias_grad(_p(self.colsum), self.rows, self.cout, _p(self.gb), None))
         # weight gradient gw^T [kp, cout] = cols^T dz: both operands read MN-major as they lie
-        a = self.cols if self.k == 3 else self.x
-        gemm(a, self.kp, self.dz, self.cout, self.kp, self.cout, self.rows, self.gwt, self.cout, A_MN | B_MN, None, err)
+        if self.direct_w:
+            check(lib.vl_nn_wgrad_bf16(_p(self.x), self.B, self.h, self.wd, self.cin, self.stride, _p(self.dz), self.cout,
+                                       _p(self.gwt), self.kp, err.ptr() if err is not None else None, None))
+        else:
+            gemm(self._im2col(), self.kp, self.dz, self.cout, self.kp, self.cout, self.rows, self.gwt, self.cout, A_MN | B_MN,
+                 None, err)
         if not need_dx:
             return
         if self.flip:
             check(lib.vl_nn_flip_weights(_p(self.wb), self.cout, self.cin, self.kp, self.kpf, _p(self.wf), None))
+            if self.direct_x:
+                check(lib.vl_nn_conv_bf16(_p(self.dz), self.B, self.ho, self.wo, self.cout, 1, 9, _p(self.wf), self.kpf,
+                                          self.cin, _p(dx), self.cin, None, EPI_ACCUM if accumulate else 0,
+                                          err.ptr() if err is not None else None, None))
+                return
             check(lib.vl_nn_im2col(_p(self.dz), self.B, self.ho, self.wo, self.cout, 1, self.kpf, _p(self.dcols), None))
             gemm(self.dcols, self.kpf, self.wf, self.kpf, self.rows, self.cin, self.kpf, dx, self.cin,
                  EPI_ACCUM if accumulate else 0, None, err)
