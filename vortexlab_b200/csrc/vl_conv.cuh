@@ -17,9 +17,9 @@
 //
 // Bound: the tile loads (x nine times through the L2, one box a tap) instead of the HBM round trip of the
 // nine-fold matrix. B200, batch 16, us of im2col + GEMM -> k_conv: 128 x 256 pixels 32 -> 32 channels 129 +
-// 76 -> 56, 96 -> 32 340 + 185 -> 144; 64 x 128 64 -> 64 63 + 55 -> 23, 192 -> 64 170 + 103 -> 53; 32 x 64
-// 128 -> 128 35 + 41 -> 19; 16 x 32 256 -> 256 21 + 39 -> 23. Weight gradients, GEMM over the matrix -> k_wgrad:
-// 32 x 32 87 -> 67, 96 x 32 215 -> 164, 64 x 64 42 -> 27, 128 x 128 45 -> 25.
+// 76 -> 56, 96 -> 32 340 + 185 -> 144 (k_conv_rows below: 24 and 61); 64 x 128 64 -> 64 63 + 55 -> 23, 192 -> 64
+// 170 + 103 -> 44; 32 x 64 128 -> 128 35 + 41 -> 17; 16 x 32 256 -> 256 21 + 39 -> 21. Weight gradients, GEMM over the matrix -> k_wgrad:
+// 32 x 32 87 -> 67, 96 x 32 215 -> 164 (k_wgrad_rows: 43 and 79), 64 x 64 42 -> 27, 128 x 128 45 -> 23.
 // Every wait on an mbarrier is bounded, as in vl_gemm.cuh.
 #pragma once
 
@@ -85,6 +85,14 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t da, uint64_t db
       "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
 }
 
+// One lane of the (converged) warp. The issuing loops run on the whole warp, so that descriptors and
+// counters are warp-uniform values (the MMA takes them from uniform registers), and this lane issues.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e != 0;
+}
+
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)));
 }
@@ -101,6 +109,64 @@ __device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t* v) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// The epilogue of one accumulator: this lane's row of it (TMEM address `acc`, bn columns from column n0 of the
+// output) to row `row` of `out`, if valid; `add`: onto the FP32 values there. By whole warps.
+__device__ __forceinline__ void store_tile(const EpiParams& ep, uint32_t acc, int bn, int n0, bool valid, size_t row, bool add,
+                                           void* out) {
+  for (int c0 = 0; c0 < bn; c0 += 32) {
+    uint32_t v[32];
+    tmem_ld32(acc + (uint32_t)c0, v);
+    if (valid) {
+      const int cols = min(32, ep.n_valid - (n0 + c0));
+#pragma unroll
+      for (int j = 0; j < 32; j += 4) {
+        float4 bv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if ((ep.flags & EPI_BIAS) && j < cols) bv = __ldg(reinterpret_cast<const float4*>(ep.bias + n0 + c0 + j));
+        const float bj[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float f = __uint_as_float(v[j + i]) + bj[i];
+          if (ep.flags & EPI_RELU) f = fmaxf(f, 0.0f);
+          v[j + i] = __float_as_uint(f);
+        }
+      }
+      // 32 bytes a store: whole sectors, though a lane's row lies apart from its neighbours'
+      if (ep.flags & EPI_BF16) {
+        __nv_bfloat16* o = (__nv_bfloat16*)out + row * ep.ldc + n0 + c0;
+#pragma unroll
+        for (int j = 0; j < 32; j += 8) {
+          if (j < cols) {                   // (the column count is a multiple of 8)
+            uint32_t u[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[j + 2 * i]), __uint_as_float(v[j + 2 * i + 1]));
+              u[i] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+            *reinterpret_cast<uint4*>(o + j) = make_uint4(u[0], u[1], u[2], u[3]);
+          }
+        }
+      } else {
+        float* o = (float*)out + row * ep.ldc + n0 + c0;
+#pragma unroll
+        for (int j = 0; j < 32; j += 8) {
+          if (j < cols) {
+            if (add) {
+              const float4 e0 = *reinterpret_cast<const float4*>(o + j), e1 = *reinterpret_cast<const float4*>(o + j + 4);
+              const float e[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+#pragma unroll
+              for (int i = 0; i < 8; ++i) v[j + i] = __float_as_uint(e[i] + __uint_as_float(v[j + i]));
+            }
+            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o + j), "r"(v[j]), "r"(v[j + 1]),
+                         "r"(v[j + 2]), "r"(v[j + 3]), "r"(v[j + 4]), "r"(v[j + 5]), "r"(v[j + 6]), "r"(v[j + 7])
+                         : "memory");
+          }
+        }
+      }
+    }
+    __syncwarp();
+  }
+}
+
 template <int KC>
 __host__ __device__ constexpr int conv_stage_bytes(int bn) {
   return (BM + bn) * KC * 2;
@@ -115,7 +181,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
   __shared__ __align__(8) uint64_t full[kConvMaxStages], empty[kConvMaxStages], tfull[2], tempty[2];
   __shared__ uint32_t tmem_base;
   __shared__ int failed, issued_loads;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int n0 = (int)blockIdx.y * p.bn;
   const int kblocks = p.taps * p.chunks;
   const int stage_bytes = conv_stage_bytes<KC>(p.bn);
@@ -181,7 +247,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
       }
     }
     issued_loads = issued;
-  } else if (threadIdx.x == 32) {
+  } else if (warp == 1) {
     const uint32_t idesc = instr_desc_bf16(p.bn);
     int s = 0, n = 0;
     uint32_t phase = 0;
@@ -212,10 +278,14 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
         const uint32_t a_addr = smem_u32(smem + s * stage_bytes), b_addr = a_addr + BM * KC * 2;
         const uint64_t da = KC == 64 ? smem_desc_sw128(a_addr) : smem_desc_sw64(a_addr);
         const uint64_t db = KC == 64 ? smem_desc_sw128(b_addr) : smem_desc_sw64(b_addr);
+        --left;
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < KC / 16; ++k) mma_bf16(acc, da + 2u * k, db + 2u * k, idesc, (!fresh || k > 0) ? 1u : 0u);
-        mma_commit(&empty[s]);
-        if (--left == 0) mma_commit(&tfull[buf]);
+          for (int k = 0; k < KC / 16; ++k) mma_bf16(acc, da + 2u * k, db + 2u * k, idesc, (!fresh || k > 0) ? 1u : 0u);
+          mma_commit(&empty[s]);
+          if (left == 0) mma_commit(&tfull[buf]);
+        }
+        __syncwarp();
         if (++s == p.stages) {
           s = 0;
           phase ^= 1;
@@ -244,58 +314,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
       const int x = tx * p.bw + (m & (p.bw - 1)), y = ty * p.bh + (m >> p.log2_bw);
       const bool valid = x < p.Wo && y < p.Ho;
       const size_t row = ((size_t)b * p.Ho + y) * p.Wo + x;
-      for (int c0 = 0; c0 < p.bn; c0 += 32) {
-        uint32_t v[32];
-        tmem_ld32(tmem + (uint32_t)(buf * p.tmem_cols + c0) + ((uint32_t)rows << 16), v);
-        if (valid) {
-          const int cols = min(32, ep.n_valid - (n0 + c0));
-#pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            float4 bv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if ((ep.flags & EPI_BIAS) && j < cols) bv = __ldg(reinterpret_cast<const float4*>(ep.bias + n0 + c0 + j));
-            const float bj[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              float f = __uint_as_float(v[j + i]) + bj[i];
-              if (ep.flags & EPI_RELU) f = fmaxf(f, 0.0f);
-              v[j + i] = __float_as_uint(f);
-            }
-          }
-          // 32 bytes a store: whole sectors, though a lane's row lies apart from its neighbours'
-          if (ep.flags & EPI_BF16) {
-            __nv_bfloat16* o = (__nv_bfloat16*)ep.out + row * ep.ldc + n0 + c0;
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (j < cols) {                   // (the column count is a multiple of 8)
-                uint32_t u[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[j + 2 * i]), __uint_as_float(v[j + 2 * i + 1]));
-                  u[i] = *reinterpret_cast<const uint32_t*>(&h);
-                }
-                *reinterpret_cast<uint4*>(o + j) = make_uint4(u[0], u[1], u[2], u[3]);
-              }
-            }
-          } else {
-            float* o = (float*)ep.out + row * ep.ldc + n0 + c0;
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (j < cols) {
-                if (add) {
-                  const float4 e0 = *reinterpret_cast<const float4*>(o + j), e1 = *reinterpret_cast<const float4*>(o + j + 4);
-                  const float e[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
-#pragma unroll
-                  for (int i = 0; i < 8; ++i) v[j + i] = __float_as_uint(e[i] + __uint_as_float(v[j + i]));
-                }
-                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o + j), "r"(v[j]), "r"(v[j + 1]),
-                             "r"(v[j + 2]), "r"(v[j + 3]), "r"(v[j + 4]), "r"(v[j + 5]), "r"(v[j + 6]), "r"(v[j + 7])
-                             : "memory");
-              }
-            }
-          }
-        }
-        __syncwarp();
-      }
+      store_tile(ep, tmem + (uint32_t)(buf * p.tmem_cols) + ((uint32_t)rows << 16), p.bn, n0, valid, row, add, ep.out);
       // the accumulator is read: the MMAs of the tile after the next may overwrite it
       asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
@@ -310,6 +329,212 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
     const int issued = issued_loads;
     for (int it = issued > p.stages ? issued - p.stages : 0; it < issued; ++it)
       mbar_wait(&full[it % p.stages], (uint32_t)(it / p.stages) & 1u, ep.spin_limit);
+    if (ep.err) atomicExch(ep.err, 1);
+  }
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(2 * p.tmem_cols)));
+}
+
+// ------------------------------------------------------------------ 3x3, stride 1, rows of 128 pixels
+// k_conv loads every activation nine times (once a tap) and the weights once a tile. Here a block walks down a
+// strip of 128-pixel rows: a ring of input rows (130 pixels, all channels) stays in shared memory, each
+// tile of one output row adds one row to it, and the three taps of a row are the same shared-memory
+// tile read 0, 1 or 2 pixels on (the swizzle is a function of the shared-memory address, so a descriptor
+// that starts at a later row of the swizzled tile is valid). The weights of the block's channels stay in
+// shared memory for all its tiles. K order and results as k_conv. Bound now by the issue and latency of its
+// narrow MMAs (about 80 cycles each). B200, batch 16, k_conv -> here: 128 x 256 pixels 32 -> 32 channels 56 -> 24 us,
+// 96 -> 32 144 -> 61, 32 -> 96 (FP32 result) 102 -> 59; 64 x 128 64 -> 64 23 -> 19.
+struct RowsParams {
+  int units, segs, tx, seg_rows;   // work units (image, column of tiles, segment of rows); rows of a segment
+  int Ho, Wo;
+  int chunks, bn, tmem_cols;       // KC-channel chunks of C
+  int ring;                        // rows of the ring
+  int box_bytes;                   // shared memory of one chunk of one row (130 pixels, 1024-byte aligned)
+  EpiParams ep;
+};
+constexpr int kRowsMaxRing = 16;
+constexpr int kRowPixels = BM + 2;
+
+template <int KC>
+__host__ __device__ constexpr int rows_box_bytes() {
+  return (kRowPixels * KC * 2 + 1023) / 1024 * 1024;
+}
+
+// CH: KC-channel chunks of C, known to the compiler where that is 1, 2 or 3: the issuing thread's loop is then
+// straight-line code of a few instructions an MMA (with a run-time loop over them it took 126 cycles an MMA of
+// 32 channels, and was the kernel's time).
+template <int KC, int CH>
+__global__ void __launch_bounds__(kConvThreads, 1) k_conv_rows(const __grid_constant__ CUtensorMap tmA,
+                                                               const __grid_constant__ CUtensorMap tmB,
+                                                               const __grid_constant__ RowsParams p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t full[kRowsMaxRing], empty[kRowsMaxRing], wfull, tfull[2], tempty[2];
+  __shared__ uint32_t tmem_base;
+  __shared__ int failed, issued_loads;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int n0 = (int)blockIdx.y * p.bn;
+  const int row_bytes = p.chunks * p.box_bytes, wtap_bytes = p.bn * KC * 2;
+  uint8_t* weights = smem;                                  // [tap][chunk] tiles of bn rows
+  uint8_t* rows = smem + (9 * p.chunks * wtap_bytes + 1023) / 1024 * 1024;
+  const EpiParams& ep = p.ep;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.ring; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&tfull[i], 1);
+      mbar_init(&tempty[i], 4);
+    }
+    mbar_init(&wfull, 1);
+    failed = 0;
+    issued_loads = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
+                 "r"((uint32_t)(2 * p.tmem_cols)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = tmem_base;
+
+  if (threadIdx.x == 0) {
+    mbar_expect_tx(&wfull, (uint32_t)(9 * p.chunks * wtap_bytes));
+    for (int k = 0; k < 9 * p.chunks; ++k) tma_load_2d(&tmB, &wfull, weights + k * wtap_bytes, k * KC, n0);
+    int s = 0, issued = 0;
+    uint32_t phase = 1;
+    bool ok = true;
+    for (int u = (int)blockIdx.x; u < p.units && ok; u += (int)gridDim.x) {
+      const int q = u / p.segs, seg = u - q * p.segs, b = q / p.tx, tx = q - b * p.tx;
+      const int y0 = seg * p.seg_rows, y1 = min(y0 + p.seg_rows, p.Ho);
+      for (int y = y0 - 1; y <= y1; ++y) {                  // (rows -1 and Ho read zero)
+        if (!mbar_wait(&empty[s], phase, ep.spin_limit)) {
+          atomicExch(&failed, 1);
+          ok = false;
+          break;
+        }
+        mbar_expect_tx(&full[s], (uint32_t)(p.chunks * kRowPixels * KC * 2));
+        for (int c = 0; c < p.chunks; ++c) tma_load_4d(&tmA, &full[s], rows + s * row_bytes + c * p.box_bytes, c * KC, tx * BM - 1, y, b);
+        ++issued;
+        if (++s == p.ring) {
+          s = 0;
+          phase ^= 1;
+        }
+      }
+    }
+    issued_loads = issued;
+  } else if (warp == 1) {
+    const uint32_t idesc = instr_desc_bf16(p.bn);
+    bool ok = mbar_wait(&wfull, 0, ep.spin_limit);
+    if (!ok) atomicExch(&failed, 1);
+    int s = 0, n = 0;                                       // s: ring slot of the row above the tile
+    uint32_t phase = 0;                                     // of that slot
+    for (int u = (int)blockIdx.x; u < p.units && ok; u += (int)gridDim.x) {
+      const int seg = u % p.segs;
+      const int y0 = seg * p.seg_rows, y1 = min(y0 + p.seg_rows, p.Ho);
+      for (int y = y0; y < y1 && ok; ++y, ++n) {
+        const int buf = n & 1;
+        if (!mbar_wait(&tempty[buf], ((uint32_t)(n >> 1) & 1u) ^ 1u, ep.spin_limit)) {
+          atomicExch(&failed, 1);
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const uint32_t acc = tmem + (uint32_t)(buf * p.tmem_cols);
+        const uint64_t wd = KC == 64 ? smem_desc_sw128(smem_u32(weights)) : smem_desc_sw64(smem_u32(weights));
+        const uint64_t rd = KC == 64 ? smem_desc_sw128(smem_u32(rows)) : smem_desc_sw64(smem_u32(rows));
+        const uint32_t wstep = (uint32_t)wtap_bytes >> 4, cstep = (uint32_t)p.box_bytes >> 4;   // in descriptor units
+        int slot = s;
+        uint32_t ph = phase;
+#pragma unroll
+        for (int ky = 0; ky < 3; ++ky) {
+          if (ok && !mbar_wait(&full[slot], ph, ep.spin_limit)) {
+            atomicExch(&failed, 1);
+            ok = false;
+          }
+          if (!ok) continue;
+          asm volatile("tcgen05.fence::after_thread_sync;");
+          const uint64_t ra = rd + (uint64_t)((uint32_t)(slot * row_bytes) >> 4);
+          if (elect_one()) {
+#pragma unroll
+            for (int kx = 0; kx < 3; ++kx) {
+              const int chunks = CH > 0 ? CH : p.chunks;
+#pragma unroll
+              for (int c = 0; c < (CH > 0 ? CH : chunks); ++c) {
+                const uint64_t da = ra + (uint64_t)((uint32_t)(kx * KC / 8) + (uint32_t)c * cstep);
+                const uint64_t db = wd + (uint64_t)((uint32_t)((ky * 3 + kx) * chunks + c) * wstep);
+#pragma unroll
+                for (int k = 0; k < KC / 16; ++k)
+                  mma_bf16(acc, da + 2u * k, db + 2u * k, idesc, (ky | kx | c | k) != 0 ? 1u : 0u);
+              }
+            }
+          }
+          __syncwarp();
+          if (++slot == p.ring) {
+            slot = 0;
+            ph ^= 1;
+          }
+        }
+        if (!ok) break;
+        if (elect_one()) {
+          mma_commit(&empty[s]);                            // the row above is done with
+          mma_commit(&tfull[buf]);
+        }
+        __syncwarp();
+        if (++s == p.ring) {
+          s = 0;
+          phase ^= 1;
+        }
+      }
+      // the last two rows of the segment
+      for (int i = 0; i < 2 && ok; ++i) {
+        if (elect_one()) mma_commit(&empty[s]);
+        __syncwarp();
+        if (++s == p.ring) {
+          s = 0;
+          phase ^= 1;
+        }
+      }
+    }
+  } else if (warp >= 2) {
+    const int prow = (warp & 3) * 32;
+    int n = 0;
+    bool ok = true;
+    for (int u = (int)blockIdx.x; u < p.units && ok; u += (int)gridDim.x) {
+      const int q = u / p.segs, seg = u - q * p.segs, b = q / p.tx, tx = q - b * p.tx;
+      const int y0 = seg * p.seg_rows, y1 = min(y0 + p.seg_rows, p.Ho);
+      const int x = tx * BM + prow + lane;
+      for (int y = y0; y < y1; ++y, ++n) {
+        const int buf = n & 1;
+        if (!mbar_wait(&tfull[buf], (uint32_t)(n >> 1) & 1u, ep.spin_limit)) {
+          atomicExch(&failed, 1);
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        store_tile(ep, tmem + (uint32_t)(buf * p.tmem_cols) + ((uint32_t)prow << 16), p.bn, n0, x < p.Wo,
+                   ((size_t)b * p.Ho + y) * p.Wo + x, (ep.flags & EPI_ACCUM) != 0, ep.out);
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tempty[buf]);
+      }
+    }
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (failed && threadIdx.x == 0) {
+    mbar_wait(&wfull, 0, ep.spin_limit);
+    const int issued = issued_loads;
+    for (int it = issued > p.ring ? issued - p.ring : 0; it < issued; ++it)
+      mbar_wait(&full[it % p.ring], (uint32_t)(it / p.ring) & 1u, ep.spin_limit);
     if (ep.err) atomicExch(ep.err, 1);
   }
   __syncthreads();
@@ -340,7 +565,7 @@ __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtens
   __shared__ __align__(8) uint64_t full[kConvMaxStages], empty[kConvMaxStages], done;
   __shared__ uint32_t tmem_base;
   __shared__ int failed, issued_loads;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int m0 = (int)blockIdx.x * BM, n0 = (int)blockIdx.y * p.bn;
   const int kb_first = (int)blockIdx.z * p.kb_per;
   const int kblocks = min(p.kblocks - kb_first, p.kb_per);
@@ -410,7 +635,7 @@ __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtens
       }
     }
     issued_loads = issued;
-  } else if (threadIdx.x == 32) {
+  } else if (warp == 1) {
     const uint32_t idesc = instr_desc_bf16(p.bn, OP_A_MN | OP_B_MN);
     int s = 0;
     uint32_t phase = 0;
@@ -418,20 +643,20 @@ __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtens
       if (!mbar_wait(&full[s], phase, ep.spin_limit)) { atomicExch(&failed, 1); break; }
       asm volatile("tcgen05.fence::after_thread_sync;");
       const uint32_t a_addr = smem_u32(smem + s * stage_bytes), b_addr = a_addr + BM * 64 * 2;
+      const uint64_t da = KC == 64 ? smem_desc_sw128_mn(a_addr) : smem_desc_sw64_mn(a_addr), db = smem_desc_sw128_mn(b_addr);
+      if (elect_one()) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        // 16 K rows further: two 8-row atoms
-        const uint64_t da = KC == 64 ? smem_desc_sw128_mn(a_addr + 2048u * k) : smem_desc_sw64_mn(a_addr + 1024u * k);
-        const uint64_t db = smem_desc_sw128_mn(b_addr + 2048u * k);
-        mma_bf16(tmem, da, db, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+        for (int k = 0; k < 4; ++k)                         // 16 K rows further: two 8-row atoms
+          mma_bf16(tmem, da + (uint64_t)((KC == 64 ? 128u : 64u) * k), db + 128u * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+        mma_commit(&empty[s]);
       }
-      mma_commit(&empty[s]);
+      __syncwarp();
       if (++s == p.stages) {
         s = 0;
         phase ^= 1;
       }
     }
-    mma_commit(&done);
+    if (elect_one()) mma_commit(&done);
   }
   __syncwarp();
   const bool have = mbar_wait(&done, 0, ep.spin_limit);
@@ -460,6 +685,148 @@ __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtens
                                                             __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
       }
     }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols));
+}
+
+// Weight gradient of a stride-1 3x3 layer whose output rows are whole 64-pixel blocks. k_wgrad loads the
+// pixels of a K block once per tap; here a block of the grid takes one kernel row ky and one KC-channel chunk, and
+// the three taps of the row are one operand: column block kx of the MN-major tile is the same shared memory
+// read kx pixels on (leading offset = one pixel's row), 128 / KC of them to an MMA; what lies past kx = 2 is
+// computed and dropped. K order, split and results as k_wgrad.
+struct WgradRowsParams {
+  int Ho, Wo, C, chunks;         // chunks: of KC channels
+  int kblocks, kb_per, stages, bn, stage_bytes, a_bytes;
+  int kp;
+  EpiParams ep;
+};
+constexpr int kWgradPixels = 64 + 4;
+
+template <int KC>
+__global__ void __launch_bounds__(128, 1) k_wgrad_rows(const __grid_constant__ CUtensorMap tmA,
+                                                       const __grid_constant__ CUtensorMap tmB,
+                                                       const __grid_constant__ WgradRowsParams p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t full[kConvMaxStages], empty[kConvMaxStages], done;
+  __shared__ uint32_t tmem_base;
+  __shared__ int failed, issued_loads;
+  constexpr int ACCS = KC == 64 ? 2 : 1;                    // taps 0-1 and 2, or all three
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int ky = (int)blockIdx.x % 3, c0 = (int)blockIdx.x / 3 * KC, n0 = (int)blockIdx.y * p.bn;
+  const int kb_first = (int)blockIdx.z * p.kb_per;
+  const int kblocks = min(p.kblocks - kb_first, p.kb_per);
+  const uint32_t acc_cols = p.bn <= 32 ? 32u : (p.bn <= 64 ? 64u : (p.bn <= 128 ? 128u : 256u));
+  const uint32_t tmem_cols = acc_cols * ACCS;
+  const EpiParams& ep = p.ep;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(&done, 1);
+    failed = 0;
+    issued_loads = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "r"(tmem_cols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = tmem_base;
+  if (threadIdx.x == 0) {
+    int issued = 0, s = 0;
+    uint32_t phase = 1;
+    int r0 = kb_first * 64;
+    int x = r0 % p.Wo, y = r0 / p.Wo, b = y / p.Ho;
+    y -= b * p.Ho;
+    const int boxes = (p.bn + 63) / 64;
+    const uint32_t bytes = (uint32_t)(kWgradPixels * KC * 2 + p.bn * 128);
+    for (int kb = 0; kb < kblocks; ++kb) {
+      if (!mbar_wait(&empty[s], phase, ep.spin_limit)) { atomicExch(&failed, 1); break; }
+      uint8_t* sa = smem + s * p.stage_bytes;
+      mbar_expect_tx(&full[s], bytes);
+      tma_load_4d(&tmA, &full[s], sa, c0, x - 1, y + ky - 1, b);
+      for (int c = 0; c < boxes; ++c) tma_load_2d(&tmB, &full[s], sa + p.a_bytes + 8192 * c, n0 + 64 * c, r0);
+      issued = kb + 1;
+      if (++s == p.stages) {
+        s = 0;
+        phase ^= 1;
+      }
+      r0 += 64;
+      x += 64;
+      if (x == p.Wo) {
+        x = 0;
+        if (++y == p.Ho) {
+          y = 0;
+          ++b;
+        }
+      }
+    }
+    issued_loads = issued;
+  } else if (warp == 1) {
+    const uint32_t idesc = instr_desc_bf16(p.bn, OP_A_MN | OP_B_MN);
+    const bool narrow = p.bn == 32;
+    int s = 0;
+    uint32_t phase = 0;
+    for (int kb = 0; kb < kblocks; ++kb) {
+      if (!mbar_wait(&full[s], phase, ep.spin_limit)) { atomicExch(&failed, 1); break; }
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const uint32_t a_addr = smem_u32(smem + s * p.stage_bytes), b_addr = a_addr + (uint32_t)p.a_bytes;
+      // the swizzled-tile descriptors with the leading offset of one pixel
+      uint64_t da = KC == 64 ? smem_desc_sw128_mn(a_addr) : smem_desc_sw64_mn(a_addr);
+      da = (da & ~((uint64_t)0x3FFFu << 16)) | ((uint64_t)(KC * 2 >> 4) << 16);
+      const uint64_t db = narrow ? smem_desc_sw64_mn(b_addr) : smem_desc_sw128_mn(b_addr);
+      const uint32_t bstep = narrow ? 64u : 128u;
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {                       // 16 pixels further
+#pragma unroll
+          for (int q = 0; q < ACCS; ++q)
+            mma_bf16(tmem + acc_cols * q, da + (uint64_t)((KC == 64 ? 128u : 64u) * k + q * 2u * (KC * 2u >> 4)),
+                     db + (uint64_t)(bstep * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+        }
+        mma_commit(&empty[s]);
+      }
+      __syncwarp();
+      if (++s == p.stages) {
+        s = 0;
+        phase ^= 1;
+      }
+    }
+    if (elect_one()) mma_commit(&done);
+  }
+  __syncwarp();
+  const bool have = mbar_wait(&done, 0, ep.spin_limit);
+  if (!have) atomicExch(&failed, 1);
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  __syncthreads();
+  const bool good = !failed;
+  if (!good && threadIdx.x == 0) {
+    const int issued = issued_loads;
+    for (int kb = issued > p.stages ? issued - p.stages : 0; kb < issued; ++kb)
+      mbar_wait(&full[kb % p.stages], (uint32_t)(kb / p.stages) & 1u, ep.spin_limit);
+    if (ep.err) atomicExch(ep.err, 1);
+  }
+  if (good) {
+    float* out = (float*)ep.out + (size_t)blockIdx.z * ep.split_stride;
+    const int m = warp * 32 + lane;
+#pragma unroll
+    for (int q = 0; q < ACCS; ++q) {
+      const int kx = 2 * q + m / KC, row = (ky * 3 + kx) * p.C + c0 + m % KC;
+      store_tile(ep, tmem + acc_cols * q + ((uint32_t)(warp * 32) << 16), p.bn, n0, kx < 3, (size_t)row, false, out);
+    }
+    // the rows past 9 C are zero
+    if (blockIdx.x == 0)
+      for (int i = (int)threadIdx.x; i < (p.kp - 9 * p.C) * p.bn; i += 128) {
+        const int n = n0 + i % p.bn;
+        if (n < ep.n_valid) out[(size_t)(9 * p.C + i / p.bn) * ep.ldc + n] = 0.0f;
+      }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();

@@ -257,6 +257,139 @@ int launch_conv(const CUtensorMap& ta, const CUtensorMap& tb, vl::gemm::ConvPara
   return e == cudaSuccess ? VL_OK : fail(VL_ECUDA, std::string("convolution launch: ") + cudaGetErrorString(e));
 }
 
+// k_conv_rows for a stride-1 3x3 convolution, where it applies: `done` false otherwise.
+template <int KC>
+int launch_rows(const void* x, int B, int H, int W, int C, const void* w, int kp, int N, const vl::gemm::EpiParams& ep,
+                bool& done, cudaStream_t s) {
+  using namespace vl::gemm;
+  done = false;
+  RowsParams p;
+  p.chunks = C / KC;
+  p.box_bytes = rows_box_bytes<KC>();
+  // All output channels in one block, their 9 C x bn weights and a ring of five rows in its shared memory;
+  // two blocks an SM where both fit. (In two or three parts, 192 -> 64 channels took 53 us as in k_conv, 64 -> 192
+  // 47 against 41.)
+  const int row_bytes = p.chunks * p.box_bytes;
+  const auto weight_bytes = [&](int bn) { return (9 * C * bn * 2 + 1023) / 1024 * 1024; };
+  constexpr int kMost = 220 * 1024;
+  if (N > 256) return VL_OK;
+  p.bn = N <= 32 ? 32 : (N + 63) / 64 * 64;
+  if (weight_bytes(p.bn) + 5 * row_bytes + 1024 > kMost) return VL_OK;
+  p.tmem_cols = p.bn <= 32 ? 32 : (p.bn <= 64 ? 64 : (p.bn <= 128 ? 128 : 256));
+  const int wb = weight_bytes(p.bn);
+  const int per_sm = 4 * p.tmem_cols <= 512 && wb + 5 * row_bytes + 1024 <= kMost / 2 ? 2 : 1;
+  p.ring = std::min(kRowsMaxRing, (kMost / per_sm - 1024 - wb) / row_bytes);
+  p.Ho = H;
+  p.Wo = W;
+  p.tx = (W + BM - 1) / BM;
+  p.ep = ep;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const int blocks = per_sm * sm_count(dev);
+  // the segment length with the shortest longest block (a segment loads two rows more than it has tiles)
+  long long best = 0;
+  for (int rows = 4; rows <= 64; ++rows) {
+    const long long units = (long long)B * p.tx * ((H + rows - 1) / rows);
+    const long long cost = ((units + blocks - 1) / blocks) * (rows + 1);
+    if (rows == 4 || cost < best) {
+      best = cost;
+      p.seg_rows = rows;
+    }
+  }
+  p.segs = (H + p.seg_rows - 1) / p.seg_rows;
+  const long long units = (long long)B * p.tx * p.segs;
+  if (units > 0x7fffffffLL) return VL_OK;
+  p.units = (int)units;
+  CUtensorMap ta, tb;
+  int rc = make_map_nhwc(&ta, x, B, H, W, C, 1, KC, kRowPixels, 1);
+  if (rc) return rc;
+  rc = make_map(&tb, w, (uint64_t)N, (uint64_t)kp, (uint64_t)kp, (uint32_t)p.bn, KC);
+  if (rc) return rc;
+  using Fn = void (*)(const CUtensorMap, const CUtensorMap, const RowsParams);
+  const Fn fns[4] = {k_conv_rows<KC, 0>, k_conv_rows<KC, 1>, k_conv_rows<KC, 2>, k_conv_rows<KC, 3>};
+  const int ch = p.chunks <= 3 ? p.chunks : 0;
+  static std::mutex m;
+  static bool configured[64][4] = {};
+  {
+    std::lock_guard<std::mutex> g(m);
+    if (dev >= 64 || !configured[dev][ch]) {
+      cudaError_t e = cudaFuncSetAttribute((const void*)fns[ch], cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
+      if (e != cudaSuccess) return fail(VL_ECUDA, std::string("convolution smem attribute: ") + cudaGetErrorString(e));
+      if (dev < 64) configured[dev][ch] = true;
+    }
+  }
+  const int smem = wb + p.ring * row_bytes + 1024;
+  fns[ch]<<<dim3((unsigned)std::min<long long>(units, blocks)), kConvThreads, smem, s>>>(ta, tb, p);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return fail(VL_ECUDA, std::string("convolution launch: ") + cudaGetErrorString(e));
+  done = true;
+  return VL_OK;
+}
+
+// The K split of launch_gemm for a weight gradient [kp, N] over `kblocks` 64-pixel blocks, so that the partial sums
+// are the same, and where the partial results go.
+int wgrad_split(int dev, int kp, int N, int bn, int kblocks, int* kb_per, int* splits, vl::gemm::EpiParams* ep, float* out) {
+  const int tiles = ((kp + vl::gemm::BM - 1) / vl::gemm::BM) * ((N + bn - 1) / bn);
+  int n = 1;
+  if (tiles < 148 && kblocks >= 16) n = std::max(1, std::min(kblocks / 8, (296 + tiles - 1) / tiles));
+  *kb_per = (kblocks + n - 1) / n;
+  *splits = (kblocks + *kb_per - 1) / *kb_per;
+  ep->out = out;
+  ep->ldc = N;
+  ep->split_stride = 0;
+  if (*splits > 1) {
+    void* w = nullptr;
+    int rc = workspace(dev, (size_t)*splits * kp * N * sizeof(float), &w);
+    if (rc) return rc;
+    ep->out = w;
+    ep->split_stride = (long long)kp * N;
+  }
+  return VL_OK;
+}
+
+template <int KC>
+int launch_wgrad_rows(const void* x, int B, int H, int W, int C, const void* dz, int N, int kp, float* out,
+                      const vl::gemm::EpiParams& ep, cudaStream_t s) {
+  using namespace vl::gemm;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  WgradRowsParams p;
+  p.Ho = H;
+  p.Wo = W;
+  p.C = C;
+  p.chunks = C / KC;
+  p.kp = kp;
+  p.kblocks = (int)((long long)B * H * W / 64);
+  p.bn = N <= 32 ? 32 : (N <= 64 ? 64 : (N <= 128 ? 128 : 256));
+  p.ep = ep;
+  int splits = 1;
+  int rc = wgrad_split(dev, kp, N, std::max(p.bn, 64), p.kblocks, &p.kb_per, &splits, &p.ep, out);
+  if (rc) return rc;
+  p.a_bytes = (kWgradPixels * KC * 2 + 1023) / 1024 * 1024;
+  p.stage_bytes = p.a_bytes + p.bn * 128;
+  p.stages = std::min(kConvMaxStages, 100 * 1024 / p.stage_bytes);
+  CUtensorMap ta, tb;
+  rc = make_map_nhwc(&ta, x, B, H, W, C, 1, KC, kWgradPixels, 1);
+  if (rc) return rc;
+  rc = make_map(&tb, dz, (uint64_t)B * H * W, (uint64_t)N, (uint64_t)N, 64u, p.bn == 32 ? 32 : 64);
+  if (rc) return rc;
+  static std::mutex m;
+  static bool configured[64] = {};
+  {
+    std::lock_guard<std::mutex> g(m);
+    if (dev >= 64 || !configured[dev]) {
+      cudaError_t e = cudaFuncSetAttribute(k_wgrad_rows<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 104 * 1024);
+      if (e != cudaSuccess) return fail(VL_ECUDA, std::string("weight gradient smem attribute: ") + cudaGetErrorString(e));
+      if (dev < 64) configured[dev] = true;
+    }
+  }
+  const int gy = (N + p.bn - 1) / p.bn;
+  k_wgrad_rows<KC><<<dim3((unsigned)(3 * p.chunks), (unsigned)gy, (unsigned)splits), 128, p.stages * p.stage_bytes + 1024, s>>>(ta, tb, p);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return fail(VL_ECUDA, std::string("weight gradient launch: ") + cudaGetErrorString(e));
+  return splits > 1 ? split_reduce((const float*)p.ep.out, splits, kp, N, out, N, 0, s) : VL_OK;
+}
+
 template <int KC>
 int launch_wgrad(const CUtensorMap& ta, const CUtensorMap& tb, vl::gemm::WgradParams& p, int kp, int N, float* out,
                  cudaStream_t s) {
@@ -264,22 +397,9 @@ int launch_wgrad(const CUtensorMap& ta, const CUtensorMap& tb, vl::gemm::WgradPa
   int dev = 0;
   cudaGetDevice(&dev);
   const int gx = (kp + BM - 1) / BM, gy = (N + p.bn - 1) / p.bn;
-  // the split of launch_gemm for the same product, so that the partial sums are the same
   int splits = 1;
-  const int tiles = gx * gy;
-  if (tiles < 148 && p.kblocks >= 16) splits = std::max(1, std::min(p.kblocks / 8, (296 + tiles - 1) / tiles));
-  p.kb_per = (p.kblocks + splits - 1) / splits;
-  splits = (p.kblocks + p.kb_per - 1) / p.kb_per;
-  p.ep.out = out;
-  p.ep.ldc = N;
-  p.ep.split_stride = 0;
-  if (splits > 1) {
-    void* w = nullptr;
-    int rc = workspace(dev, (size_t)splits * kp * N * sizeof(float), &w);
-    if (rc) return rc;
-    p.ep.out = w;
-    p.ep.split_stride = (long long)kp * N;
-  }
+  int rc = wgrad_split(dev, kp, N, p.bn, p.kblocks, &p.kb_per, &splits, &p.ep, out);
+  if (rc) return rc;
   const int stage = wgrad_stage_bytes<KC>(p.bn);
   p.stages = std::min(kConvMaxStages, 100 * 1024 / stage);
   static std::mutex m;
@@ -360,6 +480,13 @@ int vl_nn_conv_bf16(const void* x, int B, int H, int W, int C, int stride, int t
   p.ep.flags = flags & (EPI_ACCUM | EPI_BIAS | EPI_RELU | EPI_BF16);
   p.ep.err = err;
   p.ep.spin_limit = kSpinLimit;
+  // Rows of whole 128-pixel tiles (or nearly: at most a quarter more tiles than the best shape) without a K split
+  if (stride == 1 && taps == 9 && p.kb_split == taps * p.chunks && 4LL * ((W + BM - 1) / BM) * H <= 5 * best) {
+    bool done = false;
+    int rc = kc == 64 ? launch_rows<64>(x, B, H, W, C, w, kp, N, p.ep, done, (cudaStream_t)stream)
+                      : launch_rows<32>(x, B, H, W, C, w, kp, N, p.ep, done, (cudaStream_t)stream);
+    if (rc || done) return rc;
+  }
   CUtensorMap ta, tb;
   int rc = make_map_nhwc(&ta, x, B, H, W, C, stride, kc, p.bw, p.bh);
   if (rc) return rc;
@@ -392,6 +519,13 @@ int vl_nn_wgrad_bf16(const void* x, int B, int H, int W, int C, int stride, cons
   p.ep.n_valid = N;
   p.ep.err = err;
   p.ep.spin_limit = kSpinLimit;
+  // The three taps of a row as one operand: for chunks of 32 channels (batch 16, 128 x 256 pixels: 32 x 32
+  // 67 -> 43 us, 96 x 32 165 -> 79) and many chunks (64 x 128 192 x 64 77 -> 57, 32 x 64 384 x 128 57 -> 49); one or two
+  // 64-channel chunks leave it too few blocks (64 x 64 27 -> 30, 128 x 128 23 -> 27), wide N too many dropped products
+  // (64 x 192 51 -> 77).
+  if (stride == 1 && Wo % 64 == 0 && (kc == 32 || (C >= 192 && N <= 128)))
+    return kc == 64 ? launch_wgrad_rows<64>(x, B, H, W, C, dz, N, kp, gwt, p.ep, (cudaStream_t)stream)
+                    : launch_wgrad_rows<32>(x, B, H, W, C, dz, N, kp, gwt, p.ep, (cudaStream_t)stream);
   CUtensorMap ta, tb;
   int rc = make_map_nhwc(&ta, x, B, H, W, C, stride, kc, bw, 64 / bw);
   if (rc) return rc;
