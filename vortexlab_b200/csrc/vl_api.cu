@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -50,8 +51,35 @@ vl_shape* wrap_shape(std::unique_ptr<vl::Shape> s) {
 
 constexpr int kGraphSteps = 32;  // steps per captured CUDA graph (even: buffer parity returns)
 constexpr int kReduceBlocks = 296;
+constexpr size_t kScratchKeep = (size_t)64 << 20;
 constexpr uint64_t kResidentMinSteps = 4;     // fewer steps: the start (outlet velocities, own populations) costs more than it saves
 constexpr uint64_t kResidentMaxSteps = 4096;  // per launch
+
+// Sim::vorticity (src/sim.rs:582-620) from the velocity field of k_macros: central differences, one-sided next
+// to solids and at the domain's edge, FP64 rounded once to FP32. One thread a cell; bound by reading the two
+// fields (on the host, after copying them, a 482 x 242 frame took 1.0 ms; here 0.01 ms and the copy of the frame).
+__device__ __forceinline__ double one_sided(bool ahead, bool behind, double va, double v0, double vb) {
+  if (ahead && behind) return 0.5 * (va - vb);
+  if (ahead) return va - v0;
+  if (behind) return v0 - vb;
+  return 0.0;
+}
+__global__ void k_vorticity(int nx, int ny, const uint8_t* __restrict__ flag, const double* __restrict__ ux,
+                            const double* __restrict__ uy, float* __restrict__ out) {
+  const int n = nx * ny;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    float w = 0.0f;
+    if (flag[k] != 2) {
+      const int y = k / nx, x = k - y * nx;
+      const bool xp = x + 1 < nx && flag[k + 1] != 2, xm = x > 0 && flag[k - 1] != 2;
+      const bool yp = y + 1 < ny && flag[k + nx] != 2, ym = y > 0 && flag[k - nx] != 2;
+      const double dv = one_sided(xp, xm, xp ? uy[k + 1] : 0.0, uy[k], xm ? uy[k - 1] : 0.0);
+      const double du = one_sided(yp, ym, yp ? ux[k + nx] : 0.0, ux[k], ym ? ux[k - nx] : 0.0);
+      w = (float)(dv - du);
+    }
+    out[k] = w;
+  }
+}
 
 }  // namespace
 
@@ -124,6 +152,7 @@ struct vl_sim {
     void* ptrs[] = {buf[0], buf[1], d_flag, d_bidx, d_bfirst, d_links, d_pidx, d_pn, d_ctl,
                     d_partials, d_hist, d_sched, d_red, d_cells, d_gather, d_bdesc, d_wbfirst, d_lb, d_ownc, d_lnode};
     for (void* p : d_res) cudaFree(p);
+    if (d_scratch) cudaFree(d_scratch);
     for (void* p : ptrs)
       if (p) cudaFree(p);
     for (cudaEvent_t e : pev) cudaEventDestroy(e);
@@ -496,6 +525,30 @@ struct vl_sim {
     if (total_ms) *total_ms = tot;
     t_host += steps;
     return flush_probe();
+  }
+
+  // Device memory of the calls that read a field (observables, narrow downloads): kept between calls up to
+  // kScratchKeep bytes (an allocation and its release wait for the device, about 0.3 ms a call), larger
+  // ones released by scratch_done. Held under scratch_mutex from scratch() to the end of the copy.
+  std::mutex scratch_mutex;
+  void* d_scratch = nullptr;
+  size_t scratch_bytes = 0;
+  int scratch(size_t bytes, void** out) {
+    if (bytes > scratch_bytes) {
+      if (d_scratch) cudaFree(d_scratch);
+      d_scratch = nullptr;
+      scratch_bytes = 0;
+      VL_CUDA(cudaMalloc(&d_scratch, bytes));
+      scratch_bytes = bytes;
+    }
+    *out = d_scratch;
+    return VL_OK;
+  }
+  void scratch_done() {
+    if (scratch_bytes <= kScratchKeep) return;
+    cudaFree(d_scratch);
+    d_scratch = nullptr;
+    scratch_bytes = 0;
   }
 
   // 9 FP64 populations of each listed cell (reference order).
@@ -1321,11 +1374,12 @@ int vl_sim_download(vl_sim* s, double* out) {
     VL_CUDA(cudaMemcpy2DAsync(out, n * 8, s->a(), (size_t)s->ns * 8, n * 8, 9, cudaMemcpyDeviceToHost, s->stream));
   } else {
     double* tmp = nullptr;
-    VL_CUDA(cudaMalloc(&tmp, 9 * n * sizeof(double)));
+    std::lock_guard<std::mutex> guard(s->scratch_mutex);
+    if (int rc = s->scratch(9 * n * sizeof(double), (void**)&tmp)) return rc;
     cudaError_t e = s->L->to_f64((int)n, s->ns, s->a(), tmp, s->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, tmp, 9 * n * 8, cudaMemcpyDeviceToHost, s->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
-    cudaFree(tmp);
+    s->scratch_done();
     if (e != cudaSuccess) return cuda_fail(e, "download");
   }
   VL_CUDA(cudaStreamSynchronize(s->stream));
@@ -1363,14 +1417,15 @@ int vl_sim_macros_field(vl_sim* s, double* rho, double* ux, double* uy) {
   VL_CUDA(cudaSetDevice(s->device));
   const size_t n = s->n;
   double* tmp = nullptr;
-  VL_CUDA(cudaMalloc(&tmp, 3 * n * sizeof(double)));
+  std::lock_guard<std::mutex> guard(s->scratch_mutex);
+  if (int rc = s->scratch(3 * n * sizeof(double), (void**)&tmp)) return rc;
   cudaError_t e = s->L->macros((int)n, s->ns, s->d_flag, s->dom.accel[0], s->dom.accel[1], s->a(), tmp, tmp + n,
                                tmp + 2 * n, s->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(rho, tmp, n * 8, cudaMemcpyDeviceToHost, s->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(ux, tmp + n, n * 8, cudaMemcpyDeviceToHost, s->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(uy, tmp + 2 * n, n * 8, cudaMemcpyDeviceToHost, s->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
-  cudaFree(tmp);
+  s->scratch_done();
   if (e != cudaSuccess) return cuda_fail(e, "macros_field");
   return VL_OK;
 }
@@ -1437,34 +1492,24 @@ int vl_sim_max_speed(vl_sim* s, double* out) {
 // Sim::vorticity (src/sim.rs:582-620): central differences, one-sided next to solids.
 int vl_sim_vorticity(vl_sim* s, float* out) {
   if (!s || !out) return fail(VL_EINVAL, "null argument");
-  const size_t nx = s->dom.nx, ny = s->dom.ny, n = s->n;
-  std::vector<double> rho(n), ux(n), uy(n);
-  int rc = vl_sim_macros_field(s, rho.data(), ux.data(), uy.data());
+  VL_CUDA(cudaSetDevice(s->device));
+  const size_t n = s->n;
+  double* tmp = nullptr;
+  std::lock_guard<std::mutex> guard(s->scratch_mutex);
+  int rc = s->scratch(3 * n * sizeof(double) + n * sizeof(float), (void**)&tmp);
   if (rc) return rc;
-  for (size_t k = 0; k < n; ++k) {
-    out[k] = 0.0f;
-    if (s->dom.flag[k] == 2) { ux[k] = 0.0; uy[k] = 0.0; }
+  float* w = (float*)(tmp + 3 * n);
+  cudaError_t e = s->L->macros((int)n, s->ns, s->d_flag, s->dom.accel[0], s->dom.accel[1], s->a(), tmp, tmp + n,
+                               tmp + 2 * n, s->stream);
+  if (e == cudaSuccess) {
+    const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
+    k_vorticity<<<blocks, 256, 0, s->stream>>>((int)s->dom.nx, (int)s->dom.ny, s->d_flag, tmp + n, tmp + 2 * n, w);
+    e = cudaGetLastError();
   }
-  auto fluid = [&](long x, long y) {
-    return x >= 0 && y >= 0 && x < (long)nx && y < (long)ny && s->dom.flag[(size_t)y * nx + (size_t)x] != 2;
-  };
-  auto get = [&](long x, long y, int comp) {
-    const size_t k = (size_t)y * nx + (size_t)x;
-    return comp == 0 ? ux[k] : uy[k];
-  };
-  for (long y = 0; y < (long)ny; ++y) {
-    for (long x = 0; x < (long)nx; ++x) {
-      if (!fluid(x, y)) continue;
-      auto diff = [&](long dx, long dy, int comp) -> double {
-        const bool p = fluid(x + dx, y + dy), m = fluid(x - dx, y - dy);
-        if (p && m) return 0.5 * (get(x + dx, y + dy, comp) - get(x - dx, y - dy, comp));
-        if (p) return get(x + dx, y + dy, comp) - get(x, y, comp);
-        if (m) return get(x, y, comp) - get(x - dx, y - dy, comp);
-        return 0.0;
-      };
-      out[(size_t)y * nx + (size_t)x] = (float)(diff(1, 0, 1) - diff(0, 1, 0));
-    }
-  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(out, w, n * sizeof(float), cudaMemcpyDeviceToHost, s->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+  s->scratch_done();
+  if (e != cudaSuccess) return cuda_fail(e, "vorticity");
   return VL_OK;
 }
 
