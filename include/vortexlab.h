@@ -407,14 +407,15 @@ int vl_nn_gemm_bf16(const void* a, int lda, const void* b, int ldb, int M, int N
 /* Gathers and elementwise kernels around the GEMM. Activations are NHWC BF16 (row = pixel,
  * channels contiguous); a 3x3 convolution (padding 1, stride 1 or 2) is im2col + GEMM, with the
  * im2col row in (ky, kx, c) order zero-padded to kp (a multiple of 64) columns. */
-/* Convolution without the im2col matrix (x: NHWC BF16, C in multiples of 32; taps 9: 3x3 with padding 1 and
+/* Convolution without the im2col matrix (x: NHWC BF16, C in multiples of 32, or 4 for a 3x3 layer
+ * of stride 1 with kp = 64 and N at most 256; taps 9: 3x3 with padding 1 and
  * stride 1 or 2; taps 1: 1x1): out[pixel, n] = epilogue(sum over (tap, c) x[pixel + tap, c] w[n, (tap, c)]),
  * w BF16 [N][kp] with columns in (ky, kx, c) order, N, kp and ldc in multiples of 8, out 32-byte aligned; flags, bias and err as
  * vl_nn_gemm_bf16, and the same results bit for bit as im2col and that GEMM. */
 int vl_nn_conv_bf16(const void* x, int B, int H, int W, int C, int stride, int taps, const void* w, int kp, int N,
                     void* out, int ldc, const float* bias, int flags, int* err, void* stream);
 /* Weight gradient of a 3x3 layer without the im2col matrix: gwt [kp][N] FP32 = sum over pixels of
- * x[pixel + tap, c] dz[pixel, n] (the rows past 9 C are zero). Output rows of a multiple of 64 pixels, or whose
+ * x[pixel + tap, c] dz[pixel, n] (the rows past 9 C are zero; gwt 32-byte aligned). C as above; unless C = 4, output rows of a multiple of 64 pixels, or whose
  * length divides 64 with whole 64-pixel blocks in an image. */
 int vl_nn_wgrad_bf16(const void* x, int B, int H, int W, int C, int stride, const void* dz, int N, float* gwt, int kp,
                      int* err, void* stream);

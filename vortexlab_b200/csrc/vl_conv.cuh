@@ -833,5 +833,261 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_rows(const __grid_constant__ C
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols));
 }
 
+// ------------------------------------------------------------------ the 4-channel input layer
+// A pixel has 8 bytes: less than a TMA box row. Four warps gather the 9 x 4 patch of a pixel a thread and write it as
+// the row (taps in order, zeros to 64) of a 128-byte swizzled tile, which serves the forward product as the K-major
+// operand (128 pixels) and the weight gradient as the MN-major one (64 pixels of K). Products as over the
+// im2col matrix, bit for bit (steps of 16 that are zero throughout are left out of the forward pass). B200, 16 x 128 x
+// 256 pixels, 4 -> 32 channels: im2col 93 + GEMM 39 us -> 23, weight gradient over the matrix 37 -> 31.
+struct FirstParams {
+  int B, H, W;
+  const __nv_bfloat16* x;        // [B][H][W][4]
+  long long pixels;              // B H W
+  int tiles;                     // forward: 128-pixel tiles
+  int kblocks, kb_per;           // weight gradient: 64-pixel K blocks
+  int bn, kp;
+  EpiParams ep;
+};
+constexpr int kFirstStages = 4;
+
+// Row `row` of a swizzled tile: the patch of pixel r (zero past the last pixel). Chunks of 16 bytes [0, CHUNKS).
+template <int CHUNKS>
+__device__ __forceinline__ void patch_row(const FirstParams& p, long long r, uint8_t* tile, int row) {
+  uint2 t[9];
+  const bool in = r < p.pixels;
+  const unsigned q = (unsigned)(in ? r : 0);
+  const int x = (int)(q % (unsigned)p.W), yb = (int)(q / (unsigned)p.W), y = yb % p.H;
+  const uint2* src = reinterpret_cast<const uint2*>(p.x) + q;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    const int dy = k / 3 - 1, dx = k % 3 - 1;
+    const bool ok = in && y + dy >= 0 && y + dy < p.H && x + dx >= 0 && x + dx < p.W;
+    t[k] = ok ? __ldg(src + dy * p.W + dx) : make_uint2(0u, 0u);
+  }
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c) {
+    const uint2 a = 2 * c < 9 ? t[2 * c < 9 ? 2 * c : 0] : make_uint2(0u, 0u);
+    const uint2 b = 2 * c + 1 < 9 ? t[2 * c + 1 < 9 ? 2 * c + 1 : 0] : make_uint2(0u, 0u);
+    *reinterpret_cast<uint4*>(tile + row * 128 + ((c ^ (row & 7)) << 4)) = make_uint4(a.x, a.y, b.x, b.y);
+  }
+}
+
+// Warps 0-3 gather, warp 4 issues, warps 5-8 store.
+__global__ void __launch_bounds__(288, 1) k_conv_first(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ FirstParams p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t full[kFirstStages], empty[kFirstStages], wfull, tfull[2], tempty[2];
+  __shared__ uint32_t tmem_base;
+  __shared__ int failed;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  uint8_t* weights = smem + kFirstStages * 16384;
+  const EpiParams& ep = p.ep;
+  const uint32_t cols = p.bn <= 32 ? 32u : (p.bn <= 64 ? 64u : (p.bn <= 128 ? 128u : 256u));
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kFirstStages; ++s) {
+      mbar_init(&full[s], 128);
+      mbar_init(&empty[s], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&tfull[i], 1);
+      mbar_init(&tempty[i], 4);
+    }
+    mbar_init(&wfull, 1);
+    failed = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 4) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "r"(2 * cols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = tmem_base;
+  bool ok = true;
+  if (warp < 4) {
+    int s = 0;
+    uint32_t phase = 1;
+    for (int t = (int)blockIdx.x; t < p.tiles; t += (int)gridDim.x) {
+      if (!mbar_wait(&empty[s], phase, ep.spin_limit)) {
+        atomicExch(&failed, 1);
+        break;
+      }
+      patch_row<6>(p, (long long)t * BM + threadIdx.x, smem + s * 16384, (int)threadIdx.x);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tensor cores read it
+      mbar_arrive(&full[s]);
+      if (++s == kFirstStages) {
+        s = 0;
+        phase ^= 1;
+      }
+    }
+  } else if (warp == 4) {
+    const uint32_t idesc = instr_desc_bf16(p.bn);
+    if (elect_one()) {
+      mbar_expect_tx(&wfull, (uint32_t)(p.bn * 128));
+      tma_load_2d(&tmB, &wfull, weights, 0, 0);
+    }
+    __syncwarp();
+    if (!mbar_wait(&wfull, 0, ep.spin_limit)) {
+      atomicExch(&failed, 1);
+      ok = false;
+    }
+    const uint64_t db = smem_desc_sw128(smem_u32(weights));
+    int s = 0, n = 0;
+    uint32_t phase = 0;
+    for (int t = (int)blockIdx.x; t < p.tiles && ok; t += (int)gridDim.x, ++n) {
+      const int buf = n & 1;
+      if (!mbar_wait(&tempty[buf], ((uint32_t)(n >> 1) & 1u) ^ 1u, ep.spin_limit) || !mbar_wait(&full[s], phase, ep.spin_limit)) {
+        atomicExch(&failed, 1);
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const uint64_t da = smem_desc_sw128(smem_u32(smem + s * 16384));
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) mma_bf16(tmem + (uint32_t)buf * cols, da + 2u * k, db + 2u * k, idesc, k > 0 ? 1u : 0u);
+        mma_commit(&empty[s]);
+        mma_commit(&tfull[buf]);
+      }
+      __syncwarp();
+      if (++s == kFirstStages) {
+        s = 0;
+        phase ^= 1;
+      }
+    }
+  } else {
+    const int prow = (warp & 3) * 32;
+    int n = 0;
+    for (int t = (int)blockIdx.x; t < p.tiles; t += (int)gridDim.x, ++n) {
+      const int buf = n & 1;
+      if (!mbar_wait(&tfull[buf], (uint32_t)(n >> 1) & 1u, ep.spin_limit)) {
+        atomicExch(&failed, 1);
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const long long r = (long long)t * BM + prow + lane;
+      store_tile(ep, tmem + (uint32_t)buf * cols + ((uint32_t)prow << 16), p.bn, 0, r < p.pixels, (size_t)r, false, ep.out);
+      asm volatile("tcgen05.fence::before_thread_sync;");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty[buf]);
+    }
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (failed && threadIdx.x == 0) {
+    mbar_wait(&wfull, 0, ep.spin_limit);        // the weights' copy may still be landing
+    if (ep.err) atomicExch(ep.err, 1);
+  }
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  if (warp == 4) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * cols));
+}
+
+// gwt[k, n] over the K blocks of this split: warps 0-3 gather (two threads a pixel), warp 4 loads dz and issues.
+__global__ void __launch_bounds__(160, 1) k_wgrad_first(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ FirstParams p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t full[kFirstStages], empty[kFirstStages], done;
+  __shared__ uint32_t tmem_base;
+  __shared__ int failed, issued_loads;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int kb_first = (int)blockIdx.x * p.kb_per, kblocks = min(p.kblocks - kb_first, p.kb_per);
+  const int stage_bytes = 8192 + p.bn * 128;
+  const uint32_t cols = p.bn <= 64 ? 64u : (p.bn <= 128 ? 128u : 256u);
+  const EpiParams& ep = p.ep;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kFirstStages; ++s) {
+      mbar_init(&full[s], 65);                  // 64 gathering threads and the expected bytes of dz
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(&done, 1);
+    failed = 0;
+    issued_loads = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 4) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "r"(cols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = tmem_base;
+  if (warp < 4) {
+    // warps 0-1 take the even K blocks, warps 2-3 the odd ones
+    for (int kb = warp >> 1; kb < kblocks; kb += 2) {
+      const int s = kb % kFirstStages;
+      if (!mbar_wait(&empty[s], ((uint32_t)(kb / kFirstStages) & 1u) ^ 1u, ep.spin_limit)) {
+        atomicExch(&failed, 1);
+        break;
+      }
+      const int row = (int)threadIdx.x & 63;
+      patch_row<8>(p, (long long)(kb_first + kb) * 64 + row, smem + s * stage_bytes, row);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      mbar_arrive(&full[s]);
+    }
+  } else {
+    const uint32_t idesc = instr_desc_bf16(p.bn, OP_A_MN | OP_B_MN);
+    const int boxes = p.bn / 64;
+    int issued = 0;
+    bool ok = true;
+    auto load = [&](int kb) {                   // dz of K block kb
+      const int s = kb % kFirstStages;
+      if (!mbar_wait(&empty[s], ((uint32_t)(kb / kFirstStages) & 1u) ^ 1u, ep.spin_limit)) return false;
+      if (elect_one()) {
+        mbar_expect_tx(&full[s], (uint32_t)(p.bn * 128));
+        for (int c = 0; c < boxes; ++c)
+          tma_load_2d(&tmB, &full[s], smem + s * stage_bytes + 8192 + 8192 * c, 64 * c, (kb_first + kb) * 64);
+      }
+      __syncwarp();
+      ++issued;
+      return true;
+    };
+    for (int kb = 0; kb < min(kFirstStages - 1, kblocks) && ok; ++kb) ok = load(kb);
+    for (int kb = 0; kb < kblocks && ok; ++kb) {
+      const int s = kb % kFirstStages;
+      if (!mbar_wait(&full[s], (uint32_t)(kb / kFirstStages) & 1u, ep.spin_limit)) {
+        ok = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const uint32_t a_addr = smem_u32(smem + s * stage_bytes);
+      // 64 rows of M: the second column block is the first one again, and its rows are dropped
+      const uint64_t da = smem_desc_sw128_mn(a_addr) & ~((uint64_t)0x3FFFu << 16), db = smem_desc_sw128_mn(a_addr + 8192u);
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) mma_bf16(tmem, da + 128u * k, db + 128u * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+        mma_commit(&empty[s]);
+      }
+      __syncwarp();
+      if (kb + kFirstStages - 1 < kblocks) ok = load(kb + kFirstStages - 1);
+    }
+    if (!ok) atomicExch(&failed, 1);
+    if (elect_one()) mma_commit(&done);
+    if (lane == 0) issued_loads = issued;
+  }
+  __syncwarp();
+  const bool have = mbar_wait(&done, 0, ep.spin_limit);
+  if (!have) atomicExch(&failed, 1);
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  __syncthreads();
+  const bool good = !failed;
+  if (!good && threadIdx.x == 0) {
+    const int issued = issued_loads;
+    for (int kb = issued > kFirstStages ? issued - kFirstStages : 0; kb < issued; ++kb)
+      mbar_wait(&full[kb % kFirstStages], (uint32_t)(kb / kFirstStages) & 1u, ep.spin_limit);
+    if (ep.err) atomicExch(ep.err, 1);
+  }
+  if (good && warp < 2) {
+    const int row = warp * 32 + lane;
+    store_tile(ep, tmem + ((uint32_t)(warp * 32) << 16), p.bn, 0, row < p.kp, (size_t)row, false,
+               (float*)ep.out + (size_t)blockIdx.x * ep.split_stride);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (warp == 4) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols));
+}
+
 }  // namespace gemm
 }  // namespace vl

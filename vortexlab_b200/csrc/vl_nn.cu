@@ -418,6 +418,64 @@ int launch_wgrad(const CUtensorMap& ta, const CUtensorMap& tb, vl::gemm::WgradPa
   return splits > 1 ? split_reduce((const float*)p.ep.out, splits, kp, N, out, N, 0, s) : VL_OK;
 }
 
+// The 4-channel layer (x: [B, H, W, 4], 3x3, stride 1).
+int launch_conv_first(const void* x, int B, int H, int W, const void* w, int kp, int N, const vl::gemm::EpiParams& ep,
+                      cudaStream_t s) {
+  using namespace vl::gemm;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  FirstParams p{};
+  p.B = B;
+  p.H = H;
+  p.W = W;
+  p.x = (const __nv_bfloat16*)x;
+  p.pixels = (long long)B * H * W;
+  p.tiles = (int)((p.pixels + BM - 1) / BM);
+  p.bn = N <= 32 ? 32 : (N + 63) / 64 * 64;
+  p.kp = kp;
+  p.ep = ep;
+  CUtensorMap tb;
+  int rc = make_map(&tb, w, (uint64_t)N, (uint64_t)kp, (uint64_t)kp, (uint32_t)p.bn);
+  if (rc) return rc;
+  const int smem = kFirstStages * 16384 + p.bn * 128 + 1024, most = kFirstStages * 16384 + 256 * 128 + 1024;
+  cudaError_t e = cudaFuncSetAttribute(k_conv_first, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  if (e != cudaSuccess) return fail(VL_ECUDA, std::string("convolution smem attribute: ") + cudaGetErrorString(e));
+  const int per_sm = p.bn <= 128 ? 2 : 1;
+  k_conv_first<<<(unsigned)std::min(p.tiles, per_sm * sm_count(dev)), 288, smem, s>>>(tb, p);
+  e = cudaGetLastError();
+  return e == cudaSuccess ? VL_OK : fail(VL_ECUDA, std::string("convolution launch: ") + cudaGetErrorString(e));
+}
+
+int launch_wgrad_first(const void* x, int B, int H, int W, const void* dz, int N, int kp, float* out,
+                       const vl::gemm::EpiParams& ep, cudaStream_t s) {
+  using namespace vl::gemm;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  FirstParams p{};
+  p.B = B;
+  p.H = H;
+  p.W = W;
+  p.x = (const __nv_bfloat16*)x;
+  p.pixels = (long long)B * H * W;
+  p.kblocks = (int)((p.pixels + 63) / 64);
+  p.bn = N <= 64 ? 64 : (N <= 128 ? 128 : 256);
+  p.kp = kp;
+  p.ep = ep;
+  int splits = 1;
+  int rc = wgrad_split(dev, kp, N, p.bn, p.kblocks, &p.kb_per, &splits, &p.ep, out);
+  if (rc) return rc;
+  CUtensorMap tb;
+  rc = make_map(&tb, dz, (uint64_t)p.pixels, (uint64_t)N, (uint64_t)N, 64u);
+  if (rc) return rc;
+  const int smem = kFirstStages * (8192 + p.bn * 128) + 1024, most = kFirstStages * (8192 + 256 * 128) + 1024;
+  cudaError_t e = cudaFuncSetAttribute(k_wgrad_first, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  if (e != cudaSuccess) return fail(VL_ECUDA, std::string("weight gradient smem attribute: ") + cudaGetErrorString(e));
+  k_wgrad_first<<<(unsigned)splits, 160, smem, s>>>(tb, p);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return fail(VL_ECUDA, std::string("weight gradient launch: ") + cudaGetErrorString(e));
+  return splits > 1 ? split_reduce((const float*)p.ep.out, splits, kp, N, out, N, 0, s) : VL_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -427,9 +485,22 @@ int vl_nn_conv_bf16(const void* x, int B, int H, int W, int C, int stride, int t
   using namespace vl::gemm;
   if (!x || !w || !out || B < 1 || H < 1 || W < 1 || N < 1 || (stride != 1 && stride != 2) || (taps != 1 && taps != 9))
     return fail(VL_EINVAL, "convolution: bad arguments");
-  if (C < 32 || C % 32 || kp % 8 || kp < taps * C || N % 8 || ldc % 8 || ((uintptr_t)out & 31) || ((uintptr_t)bias & 15))
-    return fail(VL_EINVAL, "convolution: channels in 32s, output channels in 8s, 32-byte aligned rows");
+  const bool first = C == 4 && taps == 9 && stride == 1 && kp == 64 && N <= 256 && !(flags & EPI_ACCUM) &&
+                     (long long)B * H * W < 0x7fffff80LL && !((uintptr_t)x & 7);
+  if ((!first && (C < 32 || C % 32)) || kp % 8 || kp < taps * C || N % 8 || ldc % 8 || ((uintptr_t)out & 31) || ((uintptr_t)bias & 15))
+    return fail(VL_EINVAL, "convolution: channels in 32s (or the 4-channel 3x3 layer), output channels in 8s, 32-byte aligned rows");
   if ((flags & EPI_BIAS) && !bias) return fail(VL_EINVAL, "convolution: bias requested without a bias");
+  if (first) {
+    EpiParams ep{};
+    ep.out = out;
+    ep.ldc = ldc;
+    ep.bias = bias;
+    ep.n_valid = N;
+    ep.flags = flags & (EPI_BIAS | EPI_RELU | EPI_BF16);
+    ep.err = err;
+    ep.spin_limit = kSpinLimit;
+    return launch_conv_first(x, B, H, W, w, kp, N, ep, (cudaStream_t)stream);
+  }
   const int kc = C % 64 == 0 ? 64 : 32;
   ConvParams p;
   p.Ho = (H + stride - 1) / stride;
@@ -502,7 +573,15 @@ int vl_nn_wgrad_bf16(const void* x, int B, int H, int W, int C, int stride, cons
     return fail(VL_EINVAL, "weight gradient: bad arguments");
   const int Ho = (H + stride - 1) / stride, Wo = (W + stride - 1) / stride;
   const int bw = Wo % 64 == 0 ? 64 : Wo;
-  if (C < 32 || C % 32 || kp < 9 * C || N % 8 || ((uintptr_t)gwt & 15) || bw > 64 || 64 % bw || Ho % (64 / bw))
+  if (C == 4 && stride == 1 && kp == 64 && N <= 256 && N % 8 == 0 && (long long)B * H * W < 0x7fffff80LL &&
+      !((uintptr_t)x & 7) && !((uintptr_t)gwt & 31)) {
+    EpiParams ep{};
+    ep.n_valid = N;
+    ep.err = err;
+    ep.spin_limit = kSpinLimit;
+    return launch_wgrad_first(x, B, H, W, dz, N, kp, gwt, ep, (cudaStream_t)stream);
+  }
+  if (C < 32 || C % 32 || kp < 9 * C || N % 8 || ((uintptr_t)gwt & 31) || bw > 64 || 64 % bw || Ho % (64 / bw))
     return fail(VL_EINVAL, "weight gradient: channels in 32s, output rows that 64-pixel blocks divide");
   const int kc = C % 64 == 0 ? 64 : 32;
   WgradParams p;

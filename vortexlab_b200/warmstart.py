@@ -13,8 +13,8 @@ Every convolution is a BF16 product on the tcgen05 tensor cores with FP32 accumu
 operand tiles are loaded tap by tap from the activations (vl_nn_conv_bf16; no im2col matrix); its
 backward pass is two more (weights: x^T dz, both operands read MN-major where they lie,
 vl_nn_wgrad_bf16; data: dz with the mirrored weights for stride-1 layers, dz W^T then col2im for
-stride 2). The 4-channel input layer, and weight gradients on grids that 64-pixel blocks do not
-divide, go through the materialised im2col matrix and vl_nn_gemm_bf16.
+stride 2). Weight gradients on grids that 64-pixel blocks do not divide go through the materialised
+im2col matrix and vl_nn_gemm_bf16.
 Master weights and Adam moments are FP32. torch provides device memory only: every arithmetic
 operation on the device runs in this library's kernels.
 
@@ -137,9 +137,10 @@ class Conv:
         self.ho, self.wo = (h + self.stride - 1) // self.stride, (w + self.stride - 1) // self.stride
         self.rows = B * self.ho * self.wo
         bf = dict(dtype=torch.bfloat16, device="cuda")
-        self.direct = self.cin % 32 == 0 and self.cout % 8 == 0
+        first = self.cin == 4 and self.k == 3 and self.stride == 1 and self.cout <= 256
+        self.direct = (first or self.cin % 32 == 0) and self.cout % 8 == 0
         w64 = 64 if self.wo % 64 == 0 else self.wo
-        self.direct_w = self.direct and self.k == 3 and 64 % w64 == 0 and self.ho % (64 // w64) == 0
+        self.direct_w = self.direct and self.k == 3 and (first or (64 % w64 == 0 and self.ho % (64 // w64) == 0))
         # the im2col matrix, where a product still goes through it
         self.cols = torch.zeros(self.rows, self.kp, **bf) if self.k == 3 and not (self.direct and self.direct_w) else None
         self.flip = self.k == 3 and self.stride == 1
