@@ -419,6 +419,11 @@ int vl_nn_conv_bf16(const void* x, int B, int H, int W, int C, int stride, int t
  * length divides 64 with whole 64-pixel blocks in an image. */
 int vl_nn_wgrad_bf16(const void* x, int B, int H, int W, int C, int stride, const void* dz, int N, float* gwt, int kp,
                      int* err, void* stream);
+/* Input gradient of a 3x3 layer of stride 2 and padding 1: dx [B][H][W][C] FP32 (= or, with accumulate, +=) the
+ * col2im of dz W^T, without that matrix and with its sums: dz BF16 [B][(H+1)/2][(W+1)/2][N], wt BF16 [9 C][N] (rows in
+ * (ky, kx, c) order), C in multiples of 8, N of 32, dx 32-byte aligned. */
+int vl_nn_dgrad2_bf16(const void* dz, int B, int H, int W, int C, int N, const void* wt, float* dx, int accumulate, int* err,
+                      void* stream);
 int vl_nn_im2col(const void* x, int B, int H, int W, int C, int stride, int kp, void* cols, void* stream);
 int vl_nn_col2im(const float* dcols, int B, int H, int W, int C, int stride, int kp, float* dx, int accumulate,
                  void* stream);

@@ -95,6 +95,28 @@ def test_weight_gradient(gpu, B, H, W, C, stride, N):
     assert torch.equal(got[:kp], want) and bool((got[kp] == 7.0).all())
 
 
+@pytest.mark.parametrize("B,H,W,C,N", [(1, 16, 32, 32, 64), (2, 15, 33, 32, 32), (1, 1, 1, 8, 32), (1, 2, 3, 40, 96),
+                                       (2, 32, 64, 128, 256), (3, 22, 70, 64, 128), (1, 9, 17, 192, 64), (4, 64, 256, 32, 64)])
+@pytest.mark.parametrize("accumulate", [0, 1])
+def test_stride2_input_gradient(gpu, B, H, W, C, N, accumulate):
+    """Against dz W^T written out and gathered by col2im."""
+    import torch
+    from vortexlab_b200 import warmstart as WS
+    from vortexlab_b200._lib import check, lib
+    g, _, w, _, kp, ho, wo = _setup(B, H, W, C, 2, N)
+    R = B * ho * wo
+    dz = torch.randn(R, N, generator=g, device="cuda").to(torch.bfloat16)
+    wt = w.t().contiguous()
+    err = WS._Err()
+    dcols = torch.zeros(R, kp, device="cuda")
+    WS.gemm(dz, N, wt, N, R, kp, N, dcols, kp, 0, None, err)
+    want = torch.randn(B * H * W + 1, C, generator=g, device="cuda")
+    got = want.clone()
+    check(lib.vl_nn_col2im(WS._p(dcols), B, H, W, C, 2, kp, WS._p(want), accumulate, None))
+    check(lib.vl_nn_dgrad2_bf16(WS._p(dz), B, H, W, C, N, WS._p(wt), WS._p(got), accumulate, err.ptr(), None))
+    assert int(err.t.item()) == 0 and torch.equal(got, want)
+
+
 def test_bad_arguments_are_refused(gpu):
     import torch
     from vortexlab_b200 import warmstart as WS

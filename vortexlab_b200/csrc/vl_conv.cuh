@@ -1089,5 +1089,205 @@ __global__ void __launch_bounds__(160, 1) k_wgrad_first(const __grid_constant__ 
   if (warp == 4) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols));
 }
 
+// ------------------------------------------------------------------ input gradient of a stride-2 layer
+// dx[iy, ix, c] = the sum, over the taps (ky, kx) that read the pixel, of sum_n dz[oy, ox, n] w[n, (ky, kx, c)]. Pixels of
+// one parity class (iy & 1, ix & 1) are read by the same 1, 2, 2 or 4 taps, each at one offset into dz: a tile is 128
+// pixels of a class, each tap a product of its own over n (two accumulators in turn), and the storing warps add the
+// taps in order in registers. The sums are those of dz W^T written out in FP32 and gathered by col2im, bit for
+// bit; that matrix (9 values for each of dz's pixels and channels) was written and read through HBM: batch 16,
+// 128 x 256 pixels 32 <- 64 channels 98 + 121 us -> 41, 64 x 128 64 <- 128 49 + 60 -> 23, 32 x 64 128 <- 256 29 + 23
+// -> 20. What is left reads and writes dx once (67 MB each at the first size, 21 us) in 128-byte pieces two pixels apart.
+struct Dgrad2Params {
+  int units, tiles, tiles_x, tiles_y;   // 4 classes x B x tiles of a class and image
+  int bw, bh, log2_bw;
+  int H, W, C, chunks;                  // dx; chunks of KC channels n
+  int stages, n_valid;
+  int accumulate;
+  float* dx;
+  int* err;
+  unsigned spin_limit;
+};
+
+template <int KC, int BN>
+__global__ void __launch_bounds__(kConvThreads, 1) k_dgrad2(const __grid_constant__ CUtensorMap tmA,
+                                                            const __grid_constant__ CUtensorMap tmB,
+                                                            const __grid_constant__ Dgrad2Params p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t full[kConvMaxStages], empty[kConvMaxStages], tfull[2], tempty[2];
+  __shared__ uint32_t tmem_base;
+  __shared__ int failed, issued_loads;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int n0 = (int)blockIdx.y * BN;
+  constexpr int STAGE = conv_stage_bytes<KC>(BN);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&tfull[i], 1);
+      mbar_init(&tempty[i], 4);
+    }
+    failed = 0;
+    issued_loads = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "r"(2u * BN));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = tmem_base;
+  const int per_class = p.units / 4;            // (the class of four taps first)
+
+  if (threadIdx.x == 0) {
+    int s = 0, issued = 0;
+    uint32_t phase = 1;
+    bool ok = true;
+    for (int u = (int)blockIdx.x; u < p.units && ok; u += (int)gridDim.x) {
+      const int cls = 3 - u / per_class, v = u % per_class, b = v / p.tiles, q = v - b * p.tiles;
+      const int ty = q / p.tiles_x, j0 = (q - ty * p.tiles_x) * p.bw, i0 = ty * p.bh;
+      const int py = cls >> 1, px = cls & 1;
+      for (int a = 0; a <= py && ok; ++a) {
+        for (int e = 0; e <= px && ok; ++e) {
+          const int ky = py ? 2 * a : 1, kx = px ? 2 * e : 1, dy = py && a == 0, dx = px && e == 0;
+          for (int c = 0; c < p.chunks; ++c) {
+            if (!mbar_wait(&empty[s], phase, p.spin_limit)) {
+              atomicExch(&failed, 1);
+              ok = false;
+              break;
+            }
+            uint8_t* sa = smem + s * STAGE;
+            mbar_expect_tx(&full[s], (uint32_t)STAGE);
+            tma_load_4d(&tmA, &full[s], sa, c * KC, j0 + dx, i0 + dy, b);
+            tma_load_2d(&tmB, &full[s], sa + BM * KC * 2, c * KC, (ky * 3 + kx) * p.C + n0);
+            ++issued;
+            if (++s == p.stages) {
+              s = 0;
+              phase ^= 1;
+            }
+          }
+        }
+      }
+    }
+    issued_loads = issued;
+  } else if (warp == 1) {
+    const uint32_t idesc = instr_desc_bf16(BN);
+    int s = 0, n = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int u = (int)blockIdx.x; u < p.units && ok; u += (int)gridDim.x) {
+      const int cls = 3 - u / per_class, taps = (1 + (cls >> 1)) * (1 + (cls & 1));
+      for (int t = 0; t < taps && ok; ++t, ++n) {
+        const int buf = n & 1;
+        if (!mbar_wait(&tempty[buf], ((uint32_t)(n >> 1) & 1u) ^ 1u, p.spin_limit)) {
+          atomicExch(&failed, 1);
+          ok = false;
+          break;
+        }
+        for (int c = 0; c < p.chunks; ++c) {
+          if (!mbar_wait(&full[s], phase, p.spin_limit)) {
+            atomicExch(&failed, 1);
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;");
+          const uint32_t a_addr = smem_u32(smem + s * STAGE), b_addr = a_addr + BM * KC * 2;
+          const uint64_t da = KC == 64 ? smem_desc_sw128(a_addr) : smem_desc_sw64(a_addr);
+          const uint64_t db = KC == 64 ? smem_desc_sw128(b_addr) : smem_desc_sw64(b_addr);
+          if (elect_one()) {
+#pragma unroll
+            for (int k = 0; k < KC / 16; ++k)
+              mma_bf16(tmem + (uint32_t)(buf * BN), da + 2u * k, db + 2u * k, idesc, (c > 0 || k > 0) ? 1u : 0u);
+            mma_commit(&empty[s]);
+            if (c == p.chunks - 1) mma_commit(&tfull[buf]);
+          }
+          __syncwarp();
+          if (++s == p.stages) {
+            s = 0;
+            phase ^= 1;
+          }
+        }
+      }
+    }
+  } else if (warp >= 2) {
+    const int prow = (warp & 3) * 32, m = prow + lane;
+    int n = 0;
+    bool ok = true;
+    for (int u = (int)blockIdx.x; u < p.units && ok; u += (int)gridDim.x) {
+      const int cls = 3 - u / per_class, v = u % per_class, b = v / p.tiles, q = v - b * p.tiles;
+      const int ty = q / p.tiles_x, tx = q - ty * p.tiles_x, taps = (1 + (cls >> 1)) * (1 + (cls & 1));
+      float acc[BN];
+#pragma unroll
+      for (int j = 0; j < BN; ++j) acc[j] = 0.0f;
+      for (int t = 0; t < taps; ++t, ++n) {
+        const int buf = n & 1;
+        if (!mbar_wait(&tfull[buf], (uint32_t)(n >> 1) & 1u, p.spin_limit)) {
+          atomicExch(&failed, 1);
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;");
+#pragma unroll
+        for (int c0 = 0; c0 < BN; c0 += 32) {
+          uint32_t r[32];
+          tmem_ld32(tmem + (uint32_t)(buf * BN + c0) + ((uint32_t)prow << 16), r);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) acc[c0 + j] += __uint_as_float(r[j]);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tempty[buf]);
+      }
+      const int x = 2 * (tx * p.bw + (m & (p.bw - 1))) + (cls & 1), y = 2 * (ty * p.bh + (m >> p.log2_bw)) + (cls >> 1);
+      if (ok && x < p.W && y < p.H) {
+        float* o = p.dx + (((size_t)b * p.H + y) * p.W + x) * p.C + n0;
+#pragma unroll
+        for (int c0 = 0; c0 < BN; c0 += 32) {   // (n_valid: a multiple of 8)
+          if (p.accumulate) {
+            uint32_t e[32];
+#pragma unroll
+            for (int j = 0; j < 32; j += 8)
+              if (n0 + c0 + j < p.n_valid)
+                asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                             : "=r"(e[j]), "=r"(e[j + 1]), "=r"(e[j + 2]), "=r"(e[j + 3]), "=r"(e[j + 4]), "=r"(e[j + 5]),
+                               "=r"(e[j + 6]), "=r"(e[j + 7])
+                             : "l"(o + c0 + j));
+              else
+#pragma unroll
+                for (int i = 0; i < 8; ++i) e[j + i] = 0;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc[c0 + j] = __uint_as_float(e[j]) + acc[c0 + j];
+          }
+#pragma unroll
+          for (int j = c0; j < c0 + 32; j += 8)
+            if (n0 + j < p.n_valid)
+              asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o + j), "r"(__float_as_uint(acc[j])),
+                           "r"(__float_as_uint(acc[j + 1])), "r"(__float_as_uint(acc[j + 2])), "r"(__float_as_uint(acc[j + 3])),
+                           "r"(__float_as_uint(acc[j + 4])), "r"(__float_as_uint(acc[j + 5])), "r"(__float_as_uint(acc[j + 6])),
+                           "r"(__float_as_uint(acc[j + 7]))
+                           : "memory");
+        }
+      }
+      __syncwarp();
+    }
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (failed && threadIdx.x == 0) {
+    const int issued = issued_loads;
+    for (int it = issued > p.stages ? issued - p.stages : 0; it < issued; ++it)
+      mbar_wait(&full[it % p.stages], (uint32_t)(it / p.stages) & 1u, p.spin_limit);
+    if (p.err) atomicExch(p.err, 1);
+  }
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2u * BN));
+}
+
 }  // namespace gemm
 }  // namespace vl

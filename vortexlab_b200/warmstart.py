@@ -12,8 +12,8 @@ c0 = 32 it has 1.95 M parameters.
 Every convolution is a BF16 product on the tcgen05 tensor cores with FP32 accumulation, whose
 operand tiles are loaded tap by tap from the activations (vl_nn_conv_bf16; no im2col matrix); its
 backward pass is two more (weights: x^T dz, both operands read MN-major where they lie,
-vl_nn_wgrad_bf16; data: dz with the mirrored weights for stride-1 layers, dz W^T then col2im for
-stride 2). Weight gradients on grids that 64-pixel blocks do not divide go through the materialised
+vl_nn_wgrad_bf16; data: dz with the mirrored weights for stride-1 layers, dz W^T summed by
+parity of the pixel for stride 2, vl_nn_dgrad2_bf16). Weight gradients on grids that 64-pixel blocks do not divide go through the materialised
 im2col matrix and vl_nn_gemm_bf16.
 Master weights and Adam moments are FP32. torch provides device memory only: every arithmetic
 operation on the device runs in this library's kernels.
@@ -149,8 +149,9 @@ class Conv:
             self.direct_x = self.cout % 32 == 0 and self.cin % 8 == 0
             self.dcols = None if self.direct_x else torch.zeros(self.rows, self.kpf, **bf)
             self.wf = torch.zeros(self.cin, self.kpf, **bf)
-        elif self.k == 3:   # stride 2: dz W^T, then col2im
-            self.dcols = torch.zeros(self.rows, self.kp, dtype=torch.float32, device="cuda")
+        elif self.k == 3:   # stride 2: dz W^T gathered by parity of the pixel (or written out, then col2im)
+            self.direct_x = self.cout % 32 == 0 and self.cin % 8 == 0
+            self.dcols = None if self.direct_x else torch.zeros(self.rows, self.kp, dtype=torch.float32, device="cuda")
         self.y = torch.zeros(self.rows, self.cout, **bf) if self.relu else \
             torch.zeros(self.rows, self.cout, dtype=torch.float32, device="cuda")
         self.dz = torch.zeros(self.rows, self.cout, **bf)
@@ -204,6 +205,9 @@ class Conv:
             check(lib.vl_nn_im2col(_p(self.dz), self.B, self.ho, self.wo, self.cout, 1, self.kpf, _p(self.dcols), None))
             gemm(self.dcols, self.kpf, self.wf, self.kpf, self.rows, self.cin, self.kpf, dx, self.cin,
                  EPI_ACCUM if accumulate else 0, None, err)
+        elif self.k == 3 and self.direct_x:
+            check(lib.vl_nn_dgrad2_bf16(_p(self.dz), self.B, self.h, self.wd, self.cin, self.cout, _p(self.wbt), _p(dx),
+                                        int(accumulate), err.ptr() if err is not None else None, None))
         elif self.k == 3:
             gemm(self.dz, self.cout, self.wbt, self.cout, self.rows, self.kp, self.cout, self.dcols, self.kp, 0, None,
                  err)
