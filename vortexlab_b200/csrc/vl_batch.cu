@@ -4,8 +4,8 @@
 // Global step s advances every tunnel that still has steps to run. Between the steps at which some
 // tunnel finishes, the set of active tunnels is fixed: that stretch ("segment") uses one tile list
 // and one link-chunk list and is replayed from a captured CUDA graph of 32 steps. Each step is the
-// batched link kernel and the batched bulk kernel, scheduled as for a single sim (concurrent on a
-// forked stream, either order on one stream, or the staged pair).
+// batched link rules and the batched bulk update (both in one launch, one kernel after the other in
+// either order, or the staged pair), after the outlet offsets of the tunnels that have them.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -88,8 +88,8 @@ struct vl_batch {
   void* d_lb = nullptr;                  // staged step: returning population per link
   void* d_ownc = nullptr;                // staged step: boundary nodes' own populations
   bool own_ok = false;                   // d_ownc holds the active tunnels' current boundary nodes
-  cudaStream_t stream = nullptr, aux = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev0 = nullptr, ev1 = nullptr;
+  cudaStream_t stream = nullptr;
+  cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   vl::BatchParams P{};
   int ntiles = 0, nchunks = 0;
   int schedule = 0;
@@ -117,10 +117,9 @@ struct vl_batch {
                     d_tun, d_st, d_tiles, d_chunks, d_outl, d_partials, d_hist, d_bdesc, d_segb, d_lb, d_ownc};
     for (void* p : ptrs)
       if (p) cudaFree(p);
-    cudaEvent_t evs[] = {ev_fork, ev_join, ev0, ev1};
+    cudaEvent_t evs[] = {ev0, ev1};
     for (cudaEvent_t e : evs)
       if (e) cudaEventDestroy(e);
-    if (aux) cudaStreamDestroy(aux);
     if (stream) cudaStreamDestroy(stream);
     if (copy) cudaStreamDestroy(copy);
     if (h_stage) cudaFreeHost(h_stage);
@@ -204,7 +203,10 @@ struct vl_batch {
   }
 
   // Kernels a step launches: bulk and links, and the outlet offsets where a tunnel has an outlet.
-  int per_step() const { return (ntiles > 0) + (nchunks > 0) + (nchunks > 0 && P.noutl > 0); }
+  int per_step() const {
+    const bool one = schedule == 0 && ntiles > 0 && nchunks > 0;
+    return (one ? 1 : (ntiles > 0) + (nchunks > 0)) + (nchunks > 0 && P.noutl > 0);
+  }
 
   // Whether the work lists already hold exactly the tunnels active at step s.
   bool lists_current() const {
@@ -231,20 +233,10 @@ struct vl_batch {
       if ((e = L->batch_step(P, ntiles, nchunks, 1 | 4, a(), b(), stream)) != cudaSuccess) return e;
       return L->batch_step(P, ntiles, nchunks, 2 | 4, a(), b(), stream);
     }
-    cudaStream_t ls = schedule == 0 ? aux : stream;
-    if (schedule == 0) {
-      if ((e = cudaEventRecord(ev_fork, stream)) != cudaSuccess) return e;
-      if ((e = cudaStreamWaitEvent(aux, ev_fork, 0)) != cudaSuccess) return e;
-    }
-    if (schedule == 2) {
-      if ((e = L->batch_step(P, ntiles, nchunks, 2, a(), b(), stream)) != cudaSuccess) return e;
-      return L->batch_step(P, ntiles, nchunks, 1, a(), b(), stream);
-    }
-    if ((e = L->batch_step(P, ntiles, nchunks, 1, a(), b(), ls)) != cudaSuccess) return e;
-    if (schedule == 0 && (e = cudaEventRecord(ev_join, aux)) != cudaSuccess) return e;
-    if ((e = L->batch_step(P, ntiles, nchunks, 2, a(), b(), stream)) != cudaSuccess) return e;
-    if (schedule == 0) return cudaStreamWaitEvent(stream, ev_join, 0);
-    return cudaSuccess;
+    if (schedule == 0) return L->batch_step(P, ntiles, nchunks, 3, a(), b(), stream);
+    const int first = schedule == 1 ? 1 : 2;
+    if ((e = L->batch_step(P, ntiles, nchunks, first, a(), b(), stream)) != cudaSuccess) return e;
+    return L->batch_step(P, ntiles, nchunks, 3 - first, a(), b(), stream);
   }
 
   int ensure_graph() {
@@ -514,18 +506,7 @@ int vl_batch_build(vl_batch* b) {
   VB_CUDA(cudaMalloc(&b->d_partials, std::max(nchunk, 1) * 2 * sizeof(double)));
   VB_CUDA(cudaMalloc(&b->d_hist, std::max<unsigned long long>(hist, 1) * 2 * sizeof(double)));
   VB_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
-#ifdef VL_BATCH_AUX_PRIORITY
-  {
-    int lo = 0, hi = 0;
-    VB_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-    VB_CUDA(cudaStreamCreateWithPriority(&b->aux, cudaStreamNonBlocking, hi));
-  }
-#else
-  VB_CUDA(cudaStreamCreateWithFlags(&b->aux, cudaStreamNonBlocking));
-#endif
   VB_CUDA(cudaStreamCreateWithFlags(&b->copy, cudaStreamNonBlocking));
-  VB_CUDA(cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming));
-  VB_CUDA(cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming));
   VB_CUDA(cudaEventCreate(&b->ev0));
   VB_CUDA(cudaEventCreate(&b->ev1));
   // Start states: uniform rest, or the inflow profile when the tunnel has no ramp

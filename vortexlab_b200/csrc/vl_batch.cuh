@@ -146,15 +146,15 @@ __device__ __forceinline__ void tunnel_controls(const BatchParams& p, const Batc
   target = T.u_ref * v1;
 }
 
+// Tile `tile` of the list, by a block.
 template <class S, int STAGED>
-__global__ void __launch_bounds__(kBlock) k_batch_bulk(const __grid_constant__ BatchParams p, const S* __restrict__ A,
-                                                       S* __restrict__ B) {
+__device__ __forceinline__ void batch_tile(const BatchParams& p, const S* __restrict__ A, S* __restrict__ B, int tile) {
   using R = typename Store<S>::R;
   // Only tunnels that are active for the whole launch are in the tile list (the host rebuilds it
   // when a tunnel finishes), so the tile never checks the tunnel's t, which the link kernel's
   // epilogue may advance concurrently.
-  if (p.prefetch_tiles) batch_prefetch(p, A, (int)blockIdx.x + p.prefetch_tiles, p.packed ? 32 : 1 << p.log2_tx);
-  const int4 td = __ldg(p.tiles + blockIdx.x);
+  if (p.prefetch_tiles) batch_prefetch(p, A, tile + p.prefetch_tiles, p.packed ? 32 : 1 << p.log2_tx);
+  const int4 td = __ldg(p.tiles + tile);
   const BatchTunnel& T = p.tun[td.x];
   const int nx = T.nx, ny = T.ny;
   int x, y;
@@ -203,6 +203,12 @@ __global__ void __launch_bounds__(kBlock) k_batch_bulk(const __grid_constant__ B
   }
 }
 
+template <class S, int STAGED>
+__global__ void __launch_bounds__(kBlock) k_batch_bulk(const __grid_constant__ BatchParams p, const S* __restrict__ A,
+                                                       S* __restrict__ B) {
+  batch_tile<S, STAGED>(p, A, B, (int)blockIdx.x);
+}
+
 // The two-cell form of k_batch_bulk for narrow storage (every tunnel's row length even): a tile is
 // 2 * 2^log2_tx cells x ty rows, thread t of the tile updates the pair at 2 (t mod 2^log2_tx) of
 // row t / 2^log2_tx; a warp covers 64 cells of one row (2^log2_tx >= 32).
@@ -217,10 +223,9 @@ constexpr int batch_pair_min_blocks() {
   return sizeof(S) == 4 ? VL_BATCH_PAIR_MIN_BLOCKS : 4;
 }
 template <class S, int STAGED>
-__global__ void __launch_bounds__(kBlock, batch_pair_min_blocks<S>()) k_batch_bulk2(const __grid_constant__ BatchParams p, const S* __restrict__ A,
-                                                        S* __restrict__ B) {
-  if (p.prefetch_tiles) batch_prefetch(p, A, (int)blockIdx.x + p.prefetch_tiles, p.packed ? 64 : 2 << p.log2_tx);
-  const int4 td = __ldg(p.tiles + blockIdx.x);
+__device__ __forceinline__ void batch_tile2(const BatchParams& p, const S* __restrict__ A, S* __restrict__ B, int tile) {
+  if (p.prefetch_tiles) batch_prefetch(p, A, tile + p.prefetch_tiles, p.packed ? 64 : 2 << p.log2_tx);
+  const int4 td = __ldg(p.tiles + tile);
   const BatchTunnel& T = p.tun[td.x];
   PairTask t;
   t.nx = T.nx;
@@ -249,6 +254,12 @@ __global__ void __launch_bounds__(kBlock, batch_pair_min_blocks<S>()) k_batch_bu
   group_update<S, 2, STAGED>(t, A + T.pop_off, B + T.pop_off);
 }
 
+template <class S, int STAGED>
+__global__ void __launch_bounds__(kBlock, batch_pair_min_blocks<S>()) k_batch_bulk2(const __grid_constant__ BatchParams p, const S* __restrict__ A,
+                                                        S* __restrict__ B) {
+  batch_tile2<S, STAGED>(p, A, B, (int)blockIdx.x);
+}
+
 // STAGED = 1: the link rules only (k_links_stage for a chunk): own populations from the compact
 // copy, the returning populations to the per-link array, no pull, collision or store.
 // The outlet density offset of each active absorbing tunnel at its current step, once per tunnel
@@ -257,6 +268,7 @@ __global__ void __launch_bounds__(kBlock, batch_pair_min_blocks<S>()) k_batch_bu
 template <class S>
 __global__ void __launch_bounds__(kBlock) k_batch_outlet(const __grid_constant__ BatchParams p, const S* __restrict__ A) {
   __shared__ double s_un[kBlock];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // k_batch_step may start beside this
   const int k = __ldg(p.outl + blockIdx.x);
   const BatchTunnel& T = p.tun[k];
   BatchState* st = &p.st[k];
@@ -269,15 +281,15 @@ __global__ void __launch_bounds__(kBlock) k_batch_outlet(const __grid_constant__
   if (threadIdx.x == 0) st->drho_now = drho;
 }
 
-template <class S, int STAGED>
-__global__ void __launch_bounds__(kBlock) k_batch_links(const __grid_constant__ BatchParams p, const S* __restrict__ A,
-                                                        S* __restrict__ B) {
+// Link chunk `chunk` of the list, by a block (WAIT: beside k_batch_outlet, whose offsets it waits for).
+template <class S, int STAGED, int WAIT = 0>
+__device__ __forceinline__ void batch_chunk(const BatchParams& p, const S* __restrict__ A, S* __restrict__ B, int chunk) {
   using R = typename Store<S>::R;
   __shared__ double s_acc[2][kBlock];
   __shared__ double red[kBlock];
   __shared__ int last;
   const int tid = threadIdx.x;
-  const int4 cd = __ldg(p.chunks + blockIdx.x);
+  const int4 cd = __ldg(p.chunks + chunk);
   const BatchTunnel& T = p.tun[cd.x];
   BatchState* st = &p.st[cd.x];
   const unsigned long long t = st->t;
@@ -286,6 +298,7 @@ __global__ void __launch_bounds__(kBlock) k_batch_links(const __grid_constant__ 
   S* b = B + T.pop_off;
   double vs[4], target;
   tunnel_controls(p, T, t, vs, target);
+  if (WAIT) asm volatile("griddepcontrol.wait;" ::: "memory");   // drho_now below
   const double drho = (T.absorbing && T.np > 0) ? st->drho_now : 0.0;   // k_batch_outlet, just before
   if (cd.w == T.chunk_off && tid == 0 && !p.dry) st->drho = drho;
   s_acc[0][tid] = 0.0;
@@ -336,6 +349,40 @@ __global__ void __launch_bounds__(kBlock) k_batch_links(const __grid_constant__ 
     }
     st->arrive = 0;
     __threadfence();
+  }
+}
+
+template <class S, int STAGED>
+__global__ void __launch_bounds__(kBlock) k_batch_links(const __grid_constant__ BatchParams p, const S* __restrict__ A,
+                                                        S* __restrict__ B) {
+  batch_chunk<S, STAGED>(p, A, B, (int)blockIdx.x);
+}
+
+// Tiles of a k_batch_step block: two of the one-cell form (a tile takes a few microseconds, and a slot is empty while the
+// next block starts: 24 tunnels in FP64 109 us a step with one, 103 with two), one of the two-cell form (whose registers
+// the loop would spill: FP32 60 us, and 72 with the loop).
+template <int PAIRS>
+constexpr int batch_step_tiles() {
+  return PAIRS ? 1 : 2;
+}
+
+// A step's link chunks and tiles in one launch, instead of two kernels on forked streams: the link chunks are a long
+// chain of dependent loads (28 us beside the tiles) and have the first nchunks blocks, so it ends under the tiles. Only
+// they wait for k_batch_outlet, which lets this kernel start beside it (the tiles read nothing that it writes; their
+// populations were complete before it began). 24 tunnels of 300 x 150 to 800 x 400 cells, microseconds a step: FP32 68.5
+// -> 59.5, FP64 115 -> 103, 16-bit 65 -> 58; two of 240 x 120 15.6 -> 14.9. Taking warp segments by a counter in memory
+// instead of by block was slower (71 to 92: one address takes an addition every few clocks).
+template <class S, int PAIRS>
+__global__ void __launch_bounds__(kBlock, PAIRS ? batch_pair_min_blocks<S>() : 4) k_batch_step(
+    const __grid_constant__ BatchParams p, const S* __restrict__ A, S* __restrict__ B, int nchunks) {
+  const int k = (int)blockIdx.x - nchunks;
+  if (k < 0) {
+    batch_chunk<S, 0, 1>(p, A, B, (int)blockIdx.x);
+  } else if constexpr (PAIRS) {
+    batch_tile2<S, 0>(p, A, B, k);
+  } else {
+    constexpr int n = batch_step_tiles<PAIRS>();
+    for (int t = n * k; t < n * k + n && t < p.ntiles; ++t) batch_tile<S, 0>(p, A, B, t);
   }
 }
 

@@ -635,6 +635,32 @@ __device__ __forceinline__ LinkView load_link(const LinkRecDev* links, int l) {
   return L;
 }
 
+// s plus n values in shared memory, one after another (the order of the reference); the next eight
+// are loaded during the chain of additions (9 cycles each).
+__device__ __forceinline__ double serial_sum(const double* v, int n, double s = 0.0) {
+  int k = 0;
+  if (n >= 8) {
+    double x[8], y[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = v[i];
+    for (; k + 24 <= n; k += 16) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) y[i] = v[k + 8 + i];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s += x[i];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = v[k + 16 + i];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s += y[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += x[i];
+    k += 8;
+  }
+  for (; k < n; ++k) s += v[k];
+  return s;
+}
+
 // Outlet density offset (src/sim.rs:444-455): the velocity of every non-radiating pressure node
 // from its own populations in `a`, summed sequentially in pnode order. Block-wide; every thread
 // calls it and receives the result.
@@ -658,10 +684,7 @@ __device__ double outlet_offset(const S* __restrict__ a, unsigned ns, const int3
       s_un[tid] = (double)pnode_n[2 * k] * ux + (double)pnode_n[2 * k + 1] * uy;
     }
     __syncthreads();
-    if (tid == 0) {
-      const int m = min(kBlock, np - base);
-      for (int q = 0; q < m; ++q) sum += s_un[q];
-    }
+    if (tid == 0) sum = serial_sum(s_un, min(kBlock, np - base), sum);
     __syncthreads();
   }
   if (tid == 0) s_drho = (sum / (double)np - target) / sqrt_cs2;

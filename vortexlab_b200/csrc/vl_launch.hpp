@@ -38,7 +38,7 @@ struct Launchers {
   int (*resident_blocks)(const StepParams& p, const ResidentParams& r, int ck, int sms);
   // Records the pressure probe of the last step of a batch (one block).
   cudaError_t (*probe)(const StepParams& p, const void* a, cudaStream_t s);
-  // One step of a batch of tunnels: which = 1 link kernel, 2 bulk kernel, 3 both; + 4 the staged
+  // One step of a batch of tunnels: which = 1 link kernel, 2 bulk kernel, 3 both in one launch; + 4 the staged
   // pair (link rules only, then the bulk kernel that also updates boundary cells).
   cudaError_t (*batch_step)(const BatchParams& p, int ntiles, int nchunks, int which, const void* a, void* b,
                             cudaStream_t s);

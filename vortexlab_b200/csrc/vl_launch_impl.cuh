@@ -187,11 +187,28 @@ struct LaunchImpl {
     k_probe<S><<<1, kBlock, 0, s>>>(p, (const S*)a);
     return cudaGetLastError();
   }
-  // which: 1 link kernel, 2 bulk kernel, 3 both; + 4 the staged pair.
+  // which: 1 link kernel, 2 bulk kernel, 3 both in one launch; + 4 the staged pair.
   static cudaError_t batch_step(const BatchParams& p, int ntiles, int nchunks, int which, const void* a, void* b,
                                 cudaStream_t s) {
     bool pairs = false;
     if constexpr (!std::is_same<S, double>::value) pairs = p.pairs != 0;
+    if (which == 3 && nchunks > 0 && ntiles > 0) {
+      if (p.noutl > 0) k_batch_outlet<S><<<p.noutl, kBlock, 0, s>>>(p, (const S*)a);
+      cudaLaunchConfig_t c{};
+      const int per = pairs ? batch_step_tiles<1>() : batch_step_tiles<0>();
+      c.gridDim = dim3((unsigned)(nchunks + (ntiles + per - 1) / per));
+      c.blockDim = dim3(kBlock);
+      c.stream = s;
+      cudaLaunchAttribute at;
+      at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at.val.programmaticStreamSerializationAllowed = 1;
+      c.attrs = &at;
+      c.numAttrs = p.noutl > 0 ? 1 : 0;
+      if constexpr (!std::is_same<S, double>::value) {
+        if (pairs) return cudaLaunchKernelEx(&c, k_batch_step<S, 1>, p, (const S*)a, (S*)b, nchunks);
+      }
+      return cudaLaunchKernelEx(&c, k_batch_step<S, 0>, p, (const S*)a, (S*)b, nchunks);
+    }
     if ((which & 1) && nchunks > 0 && p.noutl > 0) k_batch_outlet<S><<<p.noutl, kBlock, 0, s>>>(p, (const S*)a);
     if (which & 4) {
       if ((which & 1) && nchunks > 0) k_batch_links<S, 1><<<nchunks, kBlock, 0, s>>>(p, (const S*)a, (S*)b);

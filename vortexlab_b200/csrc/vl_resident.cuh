@@ -112,33 +112,6 @@ __device__ __forceinline__ bool poll_arrived(const unsigned* counter, unsigned t
   return false;
 }
 
-// The sequential sum of n values in shared memory (the order of the reference); the next eight
-// are loaded during the chain of additions (9 cycles each).
-__device__ __forceinline__ double serial_sum(const double* v, int n) {
-  double s = 0.0;
-  int k = 0;
-  if (n >= 8) {
-    double x[8], y[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] = v[i];
-    for (; k + 24 <= n; k += 16) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) y[i] = v[k + 8 + i];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) s += x[i];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = v[k + 16 + i];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) s += y[i];
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) s += x[i];
-    k += 8;
-  }
-  for (; k < n; ++k) s += v[k];
-  return s;
-}
-
 // The named barrier between a block's summing warp and its outlet tasks' warps.
 __device__ __forceinline__ void outlet_sum_ready(int tasks) {
   asm volatile("bar.arrive 8, %0;" ::"r"(32 * (1 + tasks)) : "memory");
