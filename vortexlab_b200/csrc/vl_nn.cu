@@ -109,22 +109,43 @@ int workspace(int dev, size_t bytes, void** out) {
 }
 
 // out[m, n] (leading dimension ldc) = (accumulate ? out : 0) + sum over z of ws[z][m][n], z in order.
-// Sixteen splits' values are loaded ahead of the additions: with few outputs (a thin layer: 2,048 values
-// of 296 splits) one thread's chain of loads was the time (53 us -> 9 us).
+// A thread's chain of loads is the time where the outputs are few, as they are where the splits are many: the values of
+// AHEAD splits are in flight, the next ones requested before these are added (2,048 outputs of 296 splits 23 us with a
+// wait for each 16, 17 with AHEAD 32, 10 with 64; 9,216 of about 150 10.6, 8.9, 5.9). Where the splits are few, 16 and
+// fewer registers (303,104 outputs and more: 10 us, 13 with 32).
+template <int AHEAD>
 __global__ void k_split_reduce(const float* __restrict__ ws, int splits, int M, int N, float* __restrict__ out,
                                int ldc, int accumulate) {
+  constexpr int H = AHEAD / 2;
   const long long total = (long long)M * N;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    float s = 0.0f;
+    const float* q = ws + i;
+    float s = 0.0f, v[H], u[H];
     int z = 0;
-    for (; z + 16 <= splits; z += 16) {
-      float v[16];
+    if (splits >= AHEAD) {
 #pragma unroll
-      for (int k = 0; k < 16; ++k) v[k] = __ldcs(ws + (long long)(z + k) * total + i);
+      for (int k = 0; k < H; ++k) v[k] = __ldcs(q + (long long)k * total);
+      for (; z + AHEAD + H <= splits; z += AHEAD) {
 #pragma unroll
-      for (int k = 0; k < 16; ++k) s += v[k];
+        for (int k = 0; k < H; ++k) u[k] = __ldcs(q + (long long)(z + H + k) * total);
+#pragma unroll
+        for (int k = 0; k < H; ++k) s += v[k];
+#pragma unroll
+        for (int k = 0; k < H; ++k) v[k] = __ldcs(q + (long long)(z + AHEAD + k) * total);
+#pragma unroll
+        for (int k = 0; k < H; ++k) s += u[k];
+      }
+#pragma unroll
+      for (int k = 0; k < H; ++k) s += v[k];
+      z += H;
     }
-    for (; z < splits; ++z) s += ws[(long long)z * total + i];
+    for (; z < splits; z += H) {   // (at most AHEAD values)
+#pragma unroll
+      for (int k = 0; k < H; ++k) u[k] = z + k < splits ? __ldcs(q + (long long)(z + k) * total) : 0.0f;
+#pragma unroll
+      for (int k = 0; k < H; ++k)
+        if (z + k < splits) s += u[k];
+    }
     float* o = out + (i / N) * ldc + (i % N);
     *o = accumulate ? *o + s : s;
   }
@@ -133,7 +154,10 @@ __global__ void k_split_reduce(const float* __restrict__ ws, int splits, int M, 
 int split_reduce(const float* ws, int splits, int M, int N, float* out, int ldc, int accumulate, cudaStream_t s) {
   const long long total = (long long)M * N;
   const int blocks = (int)std::min<long long>((total + 63) / 64, 148 * 32);
-  k_split_reduce<<<blocks, 64, 0, s>>>(ws, splits, M, N, out, ldc, accumulate);
+  if (splits >= 64)
+    k_split_reduce<64><<<blocks, 64, 0, s>>>(ws, splits, M, N, out, ldc, accumulate);
+  else
+    k_split_reduce<16><<<blocks, 64, 0, s>>>(ws, splits, M, N, out, ldc, accumulate);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? VL_OK : fail(VL_ECUDA, std::string("gemm split reduce: ") + cudaGetErrorString(e));
 }
