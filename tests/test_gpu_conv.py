@@ -117,6 +117,39 @@ def test_stride2_input_gradient(gpu, B, H, W, C, N, accumulate):
     assert int(err.t.item()) == 0 and torch.equal(got, want)
 
 
+@pytest.mark.parametrize("stride,offset", [(1, 1), (1, 4), (2, 4), (2, 8)])
+def test_layer_takes_input_gradients_at_any_alignment(gpu, stride, offset):
+    """An input gradient that does not start on 32 bytes goes through the matrix, with the same values."""
+    import torch
+    from vortexlab_b200 import warmstart as WS
+    g = torch.Generator(device="cuda").manual_seed(offset)
+    B, H, W, C, N = 2, 16, 32, 32, 64
+    c = WS.Conv(C, N, stride=stride, seed=3)
+    c.alloc(B, H, W)
+    err = WS._Err()
+    x = torch.relu(torch.randn(B, H, W, C, generator=g, device="cuda")).bfloat16()
+    dy = torch.randn(c.rows, N, generator=g, device="cuda")
+    want = torch.zeros(B * H * W * C, device="cuda")
+    got = torch.zeros(want.numel() + 32, device="cuda")[offset:offset + want.numel()]
+    for dx in (want, got):
+        c.forward(x, err)
+        c.backward(dy, dx, False, err)
+    assert int(err.t.item()) == 0 and torch.equal(got, want)
+
+
+def test_input_changed_before_backward_is_refused(gpu):
+    """The weight gradient reads the layer's input again."""
+    import torch
+    from vortexlab_b200 import warmstart as WS
+    c = WS.Conv(32, 32, seed=3)
+    c.alloc(1, 8, 64)
+    x = torch.zeros(1, 8, 64, 32, dtype=torch.bfloat16, device="cuda")
+    c.forward(x, None)
+    x += 1
+    with pytest.raises(RuntimeError, match="changed in place"):
+        c.backward(torch.zeros(c.rows, 32, device="cuda"), None, False, None, need_dx=False)
+
+
 def test_bad_arguments_are_refused(gpu):
     import torch
     from vortexlab_b200 import warmstart as WS

@@ -147,19 +147,21 @@ class Conv:
         if self.flip:       # input gradient as a convolution of dz with mirrored weights
             self.kpf = _kp(9 * self.cout)
             self.direct_x = self.cout % 32 == 0 and self.cin % 8 == 0
-            self.dcols = None if self.direct_x else torch.zeros(self.rows, self.kpf, **bf)
+            self.dcols = None
             self.wf = torch.zeros(self.cin, self.kpf, **bf)
         elif self.k == 3:   # stride 2: dz W^T gathered by parity of the pixel (or written out, then col2im)
             self.direct_x = self.cout % 32 == 0 and self.cin % 8 == 0
-            self.dcols = None if self.direct_x else torch.zeros(self.rows, self.kp, dtype=torch.float32, device="cuda")
+            self.dcols = None
         self.y = torch.zeros(self.rows, self.cout, **bf) if self.relu else \
             torch.zeros(self.rows, self.cout, dtype=torch.float32, device="cuda")
         self.dz = torch.zeros(self.rows, self.cout, **bf)
         self.colsum = torch.zeros(self.cout, (self.rows + 31) // 32, dtype=torch.float32, device="cuda")
 
     def forward(self, x, err):
-        """x: BF16 [B, h, w, cin] (contiguous). Returns y: BF16 (ReLU layers) or FP32 [rows, cout]."""
+        """x: BF16 [B, h, w, cin] (contiguous), which `backward` reads again: it must be left as it is
+        until then. Returns y: BF16 (ReLU layers) or FP32 [rows, cout]."""
         self.x = x
+        self.x_version = 0 if x.is_inference() else x._version   # (inference tensors have none)
         self.has_cols = False
         flags = EPI_BIAS | ((EPI_RELU | EPI_BF16) if self.relu else 0)
         if self.direct:
@@ -183,6 +185,8 @@ class Conv:
     def backward(self, dy, dx, accumulate, err, need_dx=True):
         """dy: FP32 [rows, cout], the gradient of the layer output. Writes (or, with `accumulate`,
         adds) the input gradient into dx (FP32 [B, h, w, cin]); sets gw and gb."""
+        if self.direct_w and not self.x.is_inference() and self.x._version != self.x_version:
+            raise RuntimeError("the layer's input was changed in place between forward and backward")
         check(lib.vl_nn_act_bwd(_p(dy), _p(self.y) if self.relu else None, self.rows, self.cout, int(self.relu),
                                 _p(self.dz), None, _p(self.colsum), None))
         check(lib.vl_nn_bias_grad(_p(self.colsum), self.rows, self.cout, _p(self.gb), None))
@@ -195,9 +199,14 @@ class Conv:
                  None, err)
         if not need_dx:
             return
+        direct_x = self.k == 3 and self.direct_x and dx.data_ptr() % 32 == 0    # (the direct kernels store 32 bytes)
+        if self.k == 3 and not direct_x and self.dcols is None:
+            torch = _t()
+            self.dcols = torch.zeros(self.rows, self.kpf, dtype=torch.bfloat16, device="cuda") if self.flip else \
+                torch.zeros(self.rows, self.kp, dtype=torch.float32, device="cuda")
         if self.flip:
             check(lib.vl_nn_flip_weights(_p(self.wb), self.cout, self.cin, self.kp, self.kpf, _p(self.wf), None))
-            if self.direct_x:
+            if direct_x:
                 check(lib.vl_nn_conv_bf16(_p(self.dz), self.B, self.ho, self.wo, self.cout, 1, 9, _p(self.wf), self.kpf,
                                           self.cin, _p(dx), self.cin, None, EPI_ACCUM if accumulate else 0,
                                           err.ptr() if err is not None else None, None))
@@ -205,7 +214,7 @@ class Conv:
             check(lib.vl_nn_im2col(_p(self.dz), self.B, self.ho, self.wo, self.cout, 1, self.kpf, _p(self.dcols), None))
             gemm(self.dcols, self.kpf, self.wf, self.kpf, self.rows, self.cin, self.kpf, dx, self.cin,
                  EPI_ACCUM if accumulate else 0, None, err)
-        elif self.k == 3 and self.direct_x:
+        elif direct_x:
             check(lib.vl_nn_dgrad2_bf16(_p(self.dz), self.B, self.h, self.wd, self.cin, self.cout, _p(self.wbt), _p(dx),
                                         int(accumulate), err.ptr() if err is not None else None, None))
         elif self.k == 3:
