@@ -211,7 +211,8 @@ int vl_sim_step_profiled(vl_sim* s, uint64_t steps, double* link_ms, double* bul
  * VL_SCHEDULE_STAGED: a kernel that applies the link rules only (the population each link returns
  * into the fluid), then a bulk kernel that updates every fluid cell, boundary cells included, in
  * coalesced row tiles. All four give bit-identical results; only the speed differs. The batch
- * engine (vl_batch_set_schedule) takes the first three.
+ * engine (vl_batch_set_schedule) takes all four; its VL_SCHEDULE_CONCURRENT is one launch of the link rules and the
+ * bulk update, beside the outlet offsets.
  * Until a schedule is chosen here, calls of a few steps and more on a small domain (its populations stay
  * in the L2) run in one kernel that takes all the steps of the call, with the same results; so they do
  * after vl_sim_autotune, which then decides for the other calls. */

@@ -260,11 +260,9 @@ __global__ void __launch_bounds__(kBlock, batch_pair_min_blocks<S>()) k_batch_bu
   batch_tile2<S, STAGED>(p, A, B, (int)blockIdx.x);
 }
 
-// STAGED = 1: the link rules only (k_links_stage for a chunk): own populations from the compact
-// copy, the returning populations to the per-link array, no pull, collision or store.
 // The outlet density offset of each active absorbing tunnel at its current step, once per tunnel
 // (src/sim.rs:425-440; the sequential sum in outlet-node order of the reference), for every link
-// chunk of that tunnel to read; launched on the link kernel's stream just before it.
+// chunk of that tunnel to read; launched just before the kernel that takes the chunks.
 template <class S>
 __global__ void __launch_bounds__(kBlock) k_batch_outlet(const __grid_constant__ BatchParams p, const S* __restrict__ A) {
   __shared__ double s_un[kBlock];
@@ -281,7 +279,9 @@ __global__ void __launch_bounds__(kBlock) k_batch_outlet(const __grid_constant__
   if (threadIdx.x == 0) st->drho_now = drho;
 }
 
-// Link chunk `chunk` of the list, by a block (WAIT: beside k_batch_outlet, whose offsets it waits for).
+// Link chunk `chunk` of the list, by a block (WAIT: beside k_batch_outlet, whose offsets it waits for). STAGED = 1: the
+// link rules only (k_links_stage for a chunk): own populations from the compact copy, the returning populations to the
+// per-link array, no pull, collision or store.
 template <class S, int STAGED, int WAIT = 0>
 __device__ __forceinline__ void batch_chunk(const BatchParams& p, const S* __restrict__ A, S* __restrict__ B, int chunk) {
   using R = typename Store<S>::R;

@@ -204,10 +204,12 @@ struct LaunchImpl {
       at.val.programmaticStreamSerializationAllowed = 1;
       c.attrs = &at;
       c.numAttrs = p.noutl > 0 ? 1 : 0;
+      auto fn = k_batch_step<S, 0>;
       if constexpr (!std::is_same<S, double>::value) {
-        if (pairs) return cudaLaunchKernelEx(&c, k_batch_step<S, 1>, p, (const S*)a, (S*)b, nchunks);
+        if (pairs) fn = k_batch_step<S, 1>;
       }
-      return cudaLaunchKernelEx(&c, k_batch_step<S, 0>, p, (const S*)a, (S*)b, nchunks);
+      const cudaError_t e = cudaLaunchKernelEx(&c, fn, p, (const S*)a, (S*)b, nchunks);
+      return e != cudaSuccess ? e : cudaGetLastError();
     }
     if ((which & 1) && nchunks > 0 && p.noutl > 0) k_batch_outlet<S><<<p.noutl, kBlock, 0, s>>>(p, (const S*)a);
     if (which & 4) {
