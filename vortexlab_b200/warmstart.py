@@ -157,12 +157,16 @@ class Conv:
         self.dz = torch.zeros(self.rows, self.cout, **bf)
         self.colsum = torch.zeros(self.cout, (self.rows + 31) // 32, dtype=torch.float32, device="cuda")
 
-    def forward(self, x, err):
-        """x: BF16 [B, h, w, cin] (contiguous), which `backward` reads again: it must be left as it is
-        until then. Returns y: BF16 (ReLU layers) or FP32 [rows, cout]."""
+    def forward(self, x, err, held=False):
+        """x: BF16 [B, h, w, cin] (contiguous). Where `backward` reads it again (a direct weight gradient,
+        a 1x1 layer) it must be left as it is until then; otherwise its im2col matrix is gathered here.
+        `held`: the caller leaves x as it is in any case, and the matrix is gathered only if `backward` is
+        called. Returns y: BF16 (ReLU layers) or FP32 [rows, cout]."""
         self.x = x
         self.x_version = 0 if x.is_inference() else x._version   # (inference tensors have none)
         self.has_cols = False
+        if self.k == 3 and not self.direct_w and not held:
+            self._im2col()
         flags = EPI_BIAS | ((EPI_RELU | EPI_BF16) if self.relu else 0)
         if self.direct:
             check(lib.vl_nn_conv_bf16(_p(x), self.B, self.h, self.wd, self.cin, self.stride, self.k * self.k, _p(self.wb),
@@ -185,7 +189,7 @@ class Conv:
     def backward(self, dy, dx, accumulate, err, need_dx=True):
         """dy: FP32 [rows, cout], the gradient of the layer output. Writes (or, with `accumulate`,
         adds) the input gradient into dx (FP32 [B, h, w, cin]); sets gw and gb."""
-        if self.direct_w and not self.x.is_inference() and self.x._version != self.x_version:
+        if self.k == 3 and not self.has_cols and not self.x.is_inference() and self.x._version != self.x_version:
             raise RuntimeError("the layer's input was changed in place between forward and backward")
         check(lib.vl_nn_act_bwd(_p(dy), _p(self.y) if self.relu else None, self.rows, self.cout, int(self.relu),
                                 _p(self.dz), None, _p(self.colsum), None))
@@ -301,7 +305,8 @@ class UNet:
         e = []
         cur = x
         for a, b in self.enc:
-            cur = b.forward(a.forward(cur, err), err)
+            # (the layers' outputs are the network's own: it leaves them as they are until `backward`)
+            cur = b.forward(a.forward(cur, err, held=cur is not x), err, held=True)
             e.append(cur)
         d = e[-1]
         for l in range(self.levels - 2, -1, -1):
@@ -311,7 +316,7 @@ class UNet:
             check(lib.vl_nn_copy_channels(_p(e[l]), self.B * self.hs[l] * self.ws[l], self.ch[l], _p(self.cat[l]), ctot,
                                           self.ch[l + 1], None))
             a, b = self.dec[l]
-            d = b.forward(a.forward(self.cat[l], err), err)
+            d = b.forward(a.forward(self.cat[l], err, held=True), err, held=True)
         return self.head.forward(d, err)
 
     def backward(self, dout):
