@@ -59,3 +59,21 @@ def test_network_on_an_odd_grid(gpu):
         grads.append([out] + [t.clone() for c in net.layers() for t in (c.gw, c.gb)])
     for a, b in zip(*grads):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("cin,cout,h,w,stride", [(32, 32, 8, 64, 1), (4, 32, 9, 33, 1), (64, 64, 16, 64, 2)])
+def test_inference_input_changed_before_backward(gpu, cin, cout, h, w, stride):
+    """An inference tensor carries no version: the layer keeps its own copy."""
+    import torch
+    WS, c, x, dy = _layer(cin, cout, 2, h, w, stride)
+    assert c.direct_w
+    err = WS._Err()
+    if cin == 4:
+        c.backward = lambda dy, dx, acc, err, f=c.backward: f(dy, None, acc, err, need_dx=False)
+    want = _gradients(c, x, dy, err)
+    with torch.inference_mode():
+        xi = x * 1
+        got = _gradients(c, xi, dy, err, lambda: xi.mul_(-2))
+    assert int(err.t.item()) == 0
+    for a, b in zip(want, got):
+        assert torch.equal(a, b)

@@ -143,6 +143,7 @@ class Conv:
         self.direct_w = self.direct and self.k == 3 and (first or (64 % w64 == 0 and self.ho % (64 // w64) == 0))
         # the im2col matrix, where a product still goes through it
         self.cols = torch.zeros(self.rows, self.kp, **bf) if self.k == 3 and not (self.direct and self.direct_w) else None
+        self.xcopy = None
         self.flip = self.k == 3 and self.stride == 1
         if self.flip:       # input gradient as a convolution of dz with mirrored weights
             self.kpf = _kp(9 * self.cout)
@@ -159,14 +160,21 @@ class Conv:
 
     def forward(self, x, err, held=False):
         """x: BF16 [B, h, w, cin] (contiguous). Where `backward` reads it again (a direct weight gradient,
-        a 1x1 layer) it must be left as it is until then; otherwise its im2col matrix is gathered here.
+        a 1x1 layer) it must be left as it is until then (a change in place is refused; an inference tensor,
+        whose changes do not show, is copied); otherwise its im2col matrix is gathered here.
         `held`: the caller leaves x as it is in any case, and the matrix is gathered only if `backward` is
         called. Returns y: BF16 (ReLU layers) or FP32 [rows, cout]."""
         self.x = x
         self.x_version = 0 if x.is_inference() else x._version   # (inference tensors have none)
         self.has_cols = False
-        if self.k == 3 and not self.direct_w and not held:
-            self._im2col()
+        if self.k == 3 and not held:
+            if not self.direct_w:
+                self._im2col()
+            elif x.is_inference():
+                if self.xcopy is None:
+                    self.xcopy = _t().zeros(self.B * self.h * self.wd, self.cin, dtype=_t().bfloat16, device="cuda")
+                check(lib.vl_nn_copy_channels(_p(x), self.B * self.h * self.wd, self.cin, _p(self.xcopy), self.cin, 0, None))
+                self.x = self.xcopy
         flags = EPI_BIAS | ((EPI_RELU | EPI_BF16) if self.relu else 0)
         if self.direct:
             check(lib.vl_nn_conv_bf16(_p(x), self.B, self.h, self.wd, self.cin, self.stride, self.k * self.k, _p(self.wb),
