@@ -398,7 +398,10 @@ struct vl_sim {
     const int per_row = (P.nx + 32 * v - 1) / (32 * v);
     const long long nseg = (long long)per_row * P.ny;
     const int G = RP.grid;
+    RP.tables = 0;
     if (L->resident_blocks(P, RP, ck, sms) < G || nseg > 0x7fffffff) { resident_ok = false; return VL_OK; }
+    RP.tables = 1;
+    if (L->resident_blocks(P, RP, ck, sms) < G) RP.tables = 0;   // too many for the shared memory
     // Segments that a task, an outlet node's place in the serial sum, the force sums and a chunk of them
     // stand for (a segment is about 150 cycles of a block). Half and twice these move a step by 3 % at
     // most on tunnels of D = 24, 37 and 60 and the rig at 20 and 80 cells per diameter.
@@ -677,6 +680,13 @@ void staged_split(const vl::CompiledDomain& d, const std::vector<int32_t>& lnode
   }
 }
 
+vl::LinkRecDev device_link(const vl::LinkRec& h) {
+  vl::LinkRecDev g;
+  g.q = h.q; g.cu6 = h.cu6; g.uw0 = h.uw[0]; g.uw1 = h.uw[1]; g.rho = h.rho;
+  g.behind = h.behind; g.dir = h.dir; g.flags = h.flags; g.vgroup = h.vgroup; g.fgroup = h.fgroup;
+  return g;
+}
+
 // Whether the resident step kernel takes this domain, and its tables. The rule on size, us per step of
 // the resident kernel / of the fastest schedule of two kernels (B200):
 //   towing tanks and rigs (an absorbing outlet: the two-kernel step waits for its serial outlet sum)
@@ -741,9 +751,11 @@ int resident_setup(vl_sim& s) {
   std::vector<vl::WallRec> walls;
   std::vector<int4> trec;
   std::vector<uint8_t> chunk_force((size_t)s.P.nlink, 0);
-  size_t most = 0;
+  std::vector<vl::LinkRecDev> tlinks;
+  size_t most = 0, most_walls = 0, most_links = 0;
   for (int g = 0; g < G; ++g) {
     size_t count = 0;
+    const size_t walls0 = walls.size(), links0 = tlinks.size();
     for (size_t t = (size_t)g; g < G - 1 && t < tasks.size(); t += (size_t)(G - 1), ++count) {
       const int w0 = (int)walls.size();
       for (size_t at = 0; at < 32; ++at) {
@@ -789,13 +801,22 @@ int resident_setup(vl_sim& s) {
           w.cu6 = h.cu6;
           walls.push_back(w);
         }
-        nodes.push_back(make_int4((int)cell, mask, d.bnode_first[b], kind[t] == vl::TASK_OUTLET ? outlet_of[b] : (int)b));
+        unsigned w = (unsigned)b;
+        if (kind[t] == vl::TASK_OUTLET) {
+          const size_t k = (size_t)outlet_of[b];
+          w = (unsigned)k | (unsigned)(d.pnode_nx[k] + 1) << 28 | (unsigned)(d.pnode_ny[k] + 1) << 30;
+        }
+        nodes.push_back(make_int4((int)cell, mask, (int)tlinks.size(), (int)w));
+        if ((unsigned)mask & (0x3ffffu << 9))                   // open links or force
+          for (int l = d.bnode_first[b]; l < d.bnode_first[b + 1]; ++l) tlinks.push_back(device_link(d.links[(size_t)l]));
       }
       const int w1 = (int)walls.size();
-      trec.push_back(make_int4(w0, w1, kind[t], 0));
+      trec.push_back(make_int4(w0, w1, kind[t], (int)tlinks.size()));
     }
     s.res_task_first[(size_t)g + 1] = s.res_task_first[(size_t)g] + (int)count;
     most = std::max(most, count);
+    most_walls = std::max(most_walls, walls.size() - walls0);
+    most_links = std::max(most_links, tlinks.size() - links0);
   }
   std::vector<int32_t> force_chunks;
   for (size_t c = 0; c < chunk_force.size(); ++c)
@@ -803,6 +824,8 @@ int resident_setup(vl_sim& s) {
   vl::ResidentParams& RP = s.RP;
   RP.grid = G;
   RP.max_tasks = (int)most;
+  RP.max_walls = (int)most_walls;
+  RP.max_links = (int)most_links;
   RP.nforce = (int)force_chunks.size();
   bool ok = true;
   auto put = [&](auto** dst, const void* src, size_t bytes, bool zero) {
@@ -817,6 +840,7 @@ int resident_setup(vl_sim& s) {
   put(&RP.task_first, s.res_task_first.data(), s.res_task_first.size() * 4, false);
   put(&RP.nodes, nodes.data(), nodes.size() * sizeof(int4), false);
   put(&RP.walls, walls.data(), walls.size() * sizeof(vl::WallRec), false);
+  put(&RP.links, tlinks.data(), tlinks.size() * sizeof(vl::LinkRecDev), false);
   put(&RP.tasks, trec.data(), trec.size() * sizeof(int4), false);
   s.res_outlets = block_outlets;
   put(&RP.block_outlets, block_outlets.data(), block_outlets.size() * 4, false);
@@ -868,12 +892,7 @@ vl_sim* make_sim(vl::CompiledDomain&& dom, int precision) {
     return nullptr;
   }
   std::vector<vl::LinkRecDev> links(d.links.size());
-  for (size_t k = 0; k < d.links.size(); ++k) {
-    const vl::LinkRec& h = d.links[k];
-    vl::LinkRecDev& g = links[k];
-    g.q = h.q; g.cu6 = h.cu6; g.uw0 = h.uw[0]; g.uw1 = h.uw[1]; g.rho = h.rho;
-    g.behind = h.behind; g.dir = h.dir; g.flags = h.flags; g.vgroup = h.vgroup; g.fgroup = h.fgroup;
-  }
+  for (size_t k = 0; k < d.links.size(); ++k) links[k] = device_link(d.links[k]);
   std::vector<int8_t> pn(2 * d.pnode_idx.size());
   for (size_t k = 0; k < d.pnode_idx.size(); ++k) { pn[2 * k] = d.pnode_nx[k]; pn[2 * k + 1] = d.pnode_ny[k]; }
   if (!chk(alloc_copy((void**)&s->d_flag, d.flag.data(), d.n)) ||

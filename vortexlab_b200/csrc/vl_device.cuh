@@ -395,11 +395,11 @@ struct WholeBlock {
 
 // Pressure-drop probe (src/cases/cylinder.rs:54-59) of the state `a` recorded as step `tstep`
 // of the history: probe_density (src/sim.rs:624-644) at distances 1, 2, 3 from each wall point,
-// extrapolated to the wall (src/sim.rs:648-651). Block-wide; every thread must call it.
+// extrapolated to the wall (src/sim.rs:648-651). Block-wide; every thread must call it. c: the control block, or a
+// copy of it.
 template <class S, class Part = WholeBlock>
-__device__ void record_probe(const StepParams& p, const S* a, long long tstep, Part part = Part()) {
+__device__ void record_probe(const StepParams& p, const S* a, long long tstep, const Ctl* c, Part part = Part()) {
   __shared__ double rho_c[kProbeCorners];
-  Ctl* c = p.ctl;
   const long long rs = (long long)c->rec_start;
   if (!c->dp_on || !c->rec_cap || tstep < rs || tstep - rs >= (long long)c->rec_cap) return;
   const int tid = part.tid();
@@ -472,7 +472,7 @@ __device__ void step_epilogue(const StepParams& p, const S* __restrict__ a, int 
   __syncthreads();
   const unsigned long long t = c->t;
   const bool commit = !c->dry;
-  if (commit) record_probe<S>(p, a, (long long)t - 1);
+  if (commit) record_probe<S>(p, a, (long long)t - 1, c);
   if (tid == 0) {
     if (commit) {
       bool finite = true;
@@ -526,7 +526,7 @@ __device__ __forceinline__ void arrive(const StepParams& p, const S* __restrict_
 // Records the pressure probe of the last step of a batch (its result is the current `a`).
 template <class S>
 __global__ void __launch_bounds__(kBlock) k_probe(const __grid_constant__ StepParams p, const S* __restrict__ a) {
-  record_probe<S>(p, a, (long long)p.ctl->t - 1);
+  record_probe<S>(p, a, (long long)p.ctl->t - 1, p.ctl);
 }
 
 // ------------------------------------------------------------------ bulk kernel
@@ -617,9 +617,7 @@ struct LinkView {
   int behind, dir, flags, vgroup, fgroup;
 };
 
-__device__ __forceinline__ LinkView load_link(const LinkRecDev* links, int l) {
-  const int4* v = reinterpret_cast<const int4*>(links + l);
-  const int4 w0 = __ldg(v), w1 = __ldg(v + 1), w2 = __ldg(v + 2);
+__device__ __forceinline__ LinkView link_view(const int4& w0, const int4& w1, const int4& w2) {
   LinkView L;
   L.q = __hiloint2double(w0.y, w0.x);
   L.cu6 = __hiloint2double(w0.w, w0.z);
@@ -633,6 +631,10 @@ __device__ __forceinline__ LinkView load_link(const LinkRecDev* links, int l) {
   L.vgroup = (int)((packed >> 16) & 0xffu);
   L.fgroup = (int)(int8_t)(packed >> 24);
   return L;
+}
+__device__ __forceinline__ LinkView load_link(const LinkRecDev* links, int l) {
+  const int4* v = reinterpret_cast<const int4*>(links + l);
+  return link_view(__ldg(v), __ldg(v + 1), __ldg(v + 2));
 }
 
 // s plus n values in shared memory, one after another (the order of the reference); the next eight

@@ -127,14 +127,16 @@ struct LaunchImpl {
     return v < 2 ? v : 2;
   }
   static size_t resident_bytes(const StepParams& p, const ResidentParams& r) {
-    return (size_t)((p.np + 1) / 2 * 2) * sizeof(double) + (size_t)r.max_tasks * sizeof(TaskScratch<typename Store<S>::R>);
+    const size_t base =
+        (size_t)((p.np + 1) / 2 * 2) * sizeof(double) + (size_t)r.max_tasks * sizeof(TaskScratch<typename Store<S>::R>);
+    return r.tables ? base + resident_table_bytes(r) : base;
   }
   // Blocks of the kernel that fit the device at once (0: it cannot run).
   static int resident_blocks(const StepParams& p, const ResidentParams& r, int ck, int sms) {
     const void* fn = (const void*)resident_fn(p, ck);
     int per = 0;
-    if (resident_bytes(p, r) > (size_t)kResidentSmem ||
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidentSmem) != cudaSuccess ||
+    if (resident_bytes(p, r) > (size_t)(r.tables ? kResidentSmemTables : kResidentSmem) ||
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidentSmemTables) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kResidentThreads, resident_bytes(p, r)) != cudaSuccess) {
       cudaGetLastError();
       return 0;

@@ -20,10 +20,14 @@
 // The force terms of a task are formed after the block has arrived, per node in link order; that
 // part sums them by the tree of k_links over the same chunks of kBlock nodes.
 //
-// Populations are read from the L2 (ld.global.cg: another block wrote them a step before). The
-// counter is polled with relaxed loads, which leave the L1 alone, so the tables (read-only path) stay
-// in it from step to step; a block's stores are ordered before its arrival by the release, and no
-// population load is issued before the poll has returned. Every value is computed by the functions of
+// Populations are read from the L2 (ld.global.cg: another block wrote them a step before). A block's
+// stores are ordered before its arrival by the release; the counter is polled with relaxed loads, and a
+// fence of GPU scope after the last of them, before the barrier that lets the block go on, makes the wait
+// an acquire. The fence drops the L1, so what a block reads in every step (its tasks' tables, the control
+// block, the chunks with force) is kept in its shared memory. us per step without the fence and with the
+// tables in the L1 / with the fence / with the tables in shared memory: rig of 442 x 84 FP64 5.31 / 6.04 /
+// 5.36, 1762 x 330 15.8 / 15.7 / 13.9, tank of 482 x 242 FP32 6.5 / 7.1 / 6.5, 1802 x 902 28.4 / 28.5 /
+// 26.0, disk box of 700 x 450 FP64 9.4 / 10.1 / 8.5. Every value is computed by the functions of
 // the two-kernel step in their order, so states, forces and records are bit-identical to it.
 //
 // Every wait is bounded (kWaitPolls polls); a block that gives up sets Ctl::stalled and leaves, and
@@ -40,7 +44,8 @@ constexpr int kResidentThreads = 1024;      // 32 warps of 64 registers: enough 
 constexpr int kResidentWarps = kResidentThreads / 32;
 constexpr int kResidentTaskWarps = 16;      // the warps that take boundary tasks
 constexpr int kResidentSumPart = 2;         // the part of the last block that sums the forces
-constexpr int kResidentSmem = 160 * 1024;   // most dynamic shared memory of a block
+constexpr int kResidentSmem = 160 * 1024;   // most dynamic shared memory of a block, and of one with its tables
+constexpr int kResidentSmemTables = 200 * 1024;
 
 // A wall link of a task: c1, c2 are the coefficients of its rule (link_back: 0.5 / q and 1 - 0.5 / q, or
 // 2 q and 1 - 2 q), worked out in the arithmetic type; `behind` the population a[j][behind] of the near
@@ -57,6 +62,8 @@ struct alignas(16) WallRec {
 
 enum : int { TASK_WALL = 0, TASK_OPEN = 1, TASK_OUTLET = 2 };   // nodes with wall links only; with open links
 
+constexpr unsigned kOutletIndex = (1u << 28) - 1u;
+
 struct ResidentParams {
   int steps;
   int grid;
@@ -64,13 +71,17 @@ struct ResidentParams {
   const int32_t* task_first;    // [grid + 1] first task of each block
   int segs_per_row;             // segments of 32 V cells
   // Per task and lane {cell or -1; link directions j: wall 1 << j, open 1 << (j + 9), and with force or (an
-  // outlet node) pressure 1 << (j + 18); first link; rank in the boundary-node list, or index in the outlet list}.
+  // outlet node) pressure 1 << (j + 18); first link in `links`; rank in the boundary-node list, or index in the outlet
+  // list and the normal's components + 1 << 28 and << 30}.
   const int4* nodes;
   // with a cell at the grid's edge: x = 0 1 << 27, x = nx - 1 1 << 28, y = 0 1 << 29, y = ny - 1 1 << 30
   const WallRec* walls;
-  const int4* tasks;            // {first wall record, end, kind, -}
+  const int4* tasks;            // {first wall record, end, kind, end of its nodes' records in `links`}
+  const void* links;            // LinkRecDev[]: the links of the nodes with open links or force, by task and node
   const int32_t* block_outlets; // outlet tasks of each block
   int max_tasks;                // most tasks of a block
+  int max_walls, max_links;     // most wall records and records of `links` of a block
+  int tables;                   // the block's tasks, nodes, wall and link records are copied to its shared memory
   const int32_t* force_chunks;  // chunks that hold a node with force
   int nforce;
   unsigned* arrived;            // arrivals since the sim was built
@@ -90,6 +101,23 @@ struct TaskScratch {
   R own[2][9][32];
 };
 
+// The tables' part of it: nodes, tasks, wall and link records of a block.
+inline size_t resident_table_bytes(const ResidentParams& r) {
+  return (size_t)r.max_tasks * 33 * sizeof(int4) + (size_t)r.max_walls * sizeof(WallRec) +
+         (size_t)r.max_links * sizeof(LinkRecDev);
+}
+// n records of a global table to shared memory, by the block.
+template <class T>
+__device__ __forceinline__ const T* copy_table(uint4*& at, const T* src, int n) {
+  constexpr int kWords = sizeof(T) / sizeof(uint4);
+  static_assert(sizeof(T) % sizeof(uint4) == 0, "copied in 16-byte words");
+  const uint4* q = reinterpret_cast<const uint4*>(src);
+  for (int k = (int)threadIdx.x; k < n * kWords; k += kResidentThreads) at[k] = __ldg(q + k);
+  const T* out = reinterpret_cast<const T*>(at);
+  at += n * kWords;
+  return out;
+}
+
 // One part of a block.
 struct PartOf {
   int part;
@@ -102,12 +130,17 @@ __device__ __forceinline__ void grid_arrive(unsigned* counter) {
   if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
 }
 
-// Waits (thread 0 of the block) until `target` arrivals have been counted.
+// Waits (one thread of the block) until `target` arrivals have been counted. The polls are relaxed; the fence
+// behind the last one makes it an acquire of the other blocks' releases, and the barrier after it (in the
+// caller) orders the block's loads behind it.
 __device__ __forceinline__ bool poll_arrived(const unsigned* counter, unsigned target) {
   for (unsigned k = 0; k < kWaitPolls; ++k) {
     unsigned v;
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-    if ((int)(v - target) >= 0) return true;
+    if ((int)(v - target) >= 0) {
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      return true;
+    }
   }
   return false;
 }
@@ -140,18 +173,18 @@ __device__ __forceinline__ void pull_node(const S* a, unsigned ns, int nx, int n
 }
 
 // Normal velocity of an outlet node from its populations as stored (outlet_offset).
-__device__ __forceinline__ double outlet_velocity(const double* f, const StepParams& p, int k) {
+__device__ __forceinline__ double outlet_velocity(const double* f, const StepParams& p, int nx, int ny) {
   double rho, jx, jy;
   moments(f, rho, jx, jy);
   const double ux = jx / rho - 0.5 * p.gx, uy = jy / rho - 0.5 * p.gy;
-  return (double)p.pnode_n[2 * k] * ux + (double)p.pnode_n[2 * k + 1] * uy;
+  return (double)nx * ux + (double)ny * uy;
 }
 
 // What a task's open links return, as far as it follows from the nodes' own populations (link_back): of
 // a radiating link everything, of a pressure link the factor 1 + cu^2 / 2 - 1.5 u^2 and the link's density.
 template <class S>
-__device__ __forceinline__ void open_prepare(const StepParams& p, const int4& nd, int kind, int parity,
-                                             TaskScratch<typename Store<S>::R>& t) {
+__device__ __forceinline__ void open_prepare(const StepParams& p, const LinkRecDev* links, const int4& nd, int kind,
+                                             int parity, TaskScratch<typename Store<S>::R>& t) {
   using R = typename Store<S>::R;
   const int lane = (int)(threadIdx.x & 31u);
   if (nd.x < 0 || !((nd.y >> 9) & 0x1ff)) return;
@@ -167,7 +200,7 @@ __device__ __forceinline__ void open_prepare(const StepParams& p, const int4& nd
     if (!((nd.y >> (j + 9)) & 1)) continue;
     const R cu = R(3.0) * ((R)cx_of(j) * ux + (R)cy_of(j) * uy);
     R g = R(1.0) + R(0.5) * cu * cu - R(1.5) * (ux * ux + uy * uy);
-    const int4 w = __ldg(reinterpret_cast<const int4*>((const LinkRecDev*)p.links + nd.z + __popc(all & ((1u << j) - 1u))) + 2);
+    const int4 w = *(reinterpret_cast<const int4*>(links + nd.z + __popc(all & ((1u << j) - 1u))) + 2);
     const R lrho = (R)__hiloint2double(w.y, w.x);
     if (kind == TASK_OUTLET && ((nd.y >> (j + 18)) & 1)) {
       t.back[j - 1][lane] = lrho;
@@ -181,13 +214,14 @@ __device__ __forceinline__ void open_prepare(const StepParams& p, const int4& nd
   }
 }
 
-// One task of a warp: its boundary nodes updated. vs: the step's wall speeds; parity: the step's; outlets:
-// the outlet tasks of the block that wait for *s_drho (an outlet task; 0: no target); un_new: the
-// outlet velocities after the step.
+// One task of a warp: its boundary nodes updated. walls: the records, by td's indices; vs: the step's wall
+// speeds; parity: the step's; outlets: the outlet tasks of the block that wait for *s_drho (an outlet task;
+// 0: no target); un_new: the outlet velocities after the step.
 template <class S, int CK>
-__device__ __forceinline__ void boundary_task(const StepParams& p, const ResidentParams& r, const int4& nd, const int4& td,
-                                              const S* a, S* b, const double* vs, int parity, int outlets,
-                                              const double* s_drho, double* un_new, TaskScratch<typename Store<S>::R>& t) {
+__device__ __forceinline__ void boundary_task(const StepParams& p, const int4& nd, const int4& td,
+                                              const WallRec* walls, const S* a, S* b, const double* vs, int parity,
+                                              int outlets, const double* s_drho, double* un_new,
+                                              TaskScratch<typename Store<S>::R>& t) {
   using R = typename Store<S>::R;
   const int lane = (int)(threadIdx.x & 31u);
   const unsigned cell = (unsigned)nd.x;
@@ -202,7 +236,7 @@ __device__ __forceinline__ void boundary_task(const StepParams& p, const Residen
     for (int m = 0; m < U; ++m) {
       const int l = base + m * 32;
       if (l < td.y) {
-        const uint4 w = __ldg(reinterpret_cast<const uint4*>(r.walls + l));
+        const uint4 w = *reinterpret_cast<const uint4*>(walls + l);
         slot[m] = w.y;
         meta[m] = w.z;
         if ((w.z & 3u) == WALL_NEAR) bval[m] = Store<S>::ld_cg(a + w.x, (int)(w.y / 32) + 1);
@@ -212,8 +246,8 @@ __device__ __forceinline__ void boundary_task(const StepParams& p, const Residen
     for (int m = 0; m < U; ++m) {
       const int l = base + m * 32;
       if (l < td.y) {
-        const double2 cc = __ldg(reinterpret_cast<const double2*>(r.walls + l) + 1);
-        const R corr = (R)__ldg(&r.walls[l].cu6) * (R)vs[(meta[m] >> 2) & 3u];
+        const double2 cc = *(reinterpret_cast<const double2*>(walls + l) + 1);
+        const R corr = (R)walls[l].cu6 * (R)vs[(meta[m] >> 2) & 3u];
         const unsigned type = meta[m] & 3u;
         const int j = (int)(slot[m] / 32) + 1, node = (int)(slot[m] & 31u);
         const R out = own[j * 32 + node];
@@ -257,7 +291,8 @@ __device__ __forceinline__ void boundary_task(const StepParams& p, const Residen
     double fd[9];
 #pragma unroll
     for (int i = 0; i < 9; ++i) fd[i] = (double)f[i];
-    __stcg(un_new + nd.w, outlet_velocity(fd, p, nd.w));
+    const unsigned w = (unsigned)nd.w;
+    __stcg(un_new + (w & kOutletIndex), outlet_velocity(fd, p, (int)((w >> 28) & 3u) - 1, (int)(w >> 30) - 1));
   }
 #pragma unroll
   for (int i = 0; i < 9; ++i) t.own[parity ^ 1][i][lane] = f[i];
@@ -265,8 +300,8 @@ __device__ __forceinline__ void boundary_task(const StepParams& p, const Residen
 
 // The force terms of a task's nodes, per node in link order (after boundary_task).
 template <class S>
-__device__ __forceinline__ void task_force(const StepParams& p, const int4& nd, const double* vs, int parity,
-                                           double* node_force, const TaskScratch<typename Store<S>::R>& t) {
+__device__ __forceinline__ void task_force(const StepParams& p, const LinkRecDev* links, const int4& nd,
+                                           const double* vs, int parity, double* node_force, const TaskScratch<typename Store<S>::R>& t) {
   using R = typename Store<S>::R;
   const int lane = (int)(threadIdx.x & 31u);
   const unsigned fm = ((unsigned)nd.y >> 18) & 0x1ffu;
@@ -277,7 +312,8 @@ __device__ __forceinline__ void task_force(const StepParams& p, const int4& nd, 
   for (int k = 0; k < 2 * kMaxGroups; ++k) acc[k] = 0.0;
   for (int j = 1; j < 9; ++j) {
     if (!((fm >> j) & 1u)) continue;
-    const LinkView L = load_link((const LinkRecDev*)p.links, nd.z + __popc(all & ((1u << j) - 1u)));
+    const int4* rec = reinterpret_cast<const int4*>(links + nd.z + __popc(all & ((1u << j) - 1u)));
+    const LinkView L = link_view(rec[0], rec[1], rec[2]);
     double tx, ty;
     force_terms(L, (double)t.own[parity][j][lane], (double)t.back[j - 1][lane], (double)(R)vs[L.vgroup], tx, ty);
 #pragma unroll
@@ -300,13 +336,13 @@ __device__ __forceinline__ void task_force(const StepParams& p, const int4& nd, 
 template <class S>
 __device__ __forceinline__ void resident_epilogue(const StepParams& p, const ResidentParams& r, unsigned long long t,
                                                   int slot, bool final_step, double (*s_part)[kBlock], double* s_force,
-                                                  const PartOf& me) {
-  Ctl* c = p.ctl;
+                                                  const int* s_chunks, const Ctl* k0, const PartOf& me) {
+  Ctl* c = p.ctl;                                               // (read in the copy k0, but for `nonfinite`)
   const int tid = me.tid(), lane = tid & 31, warp = tid >> 5;
   const int ncomp = 2 * p.ngroups;
   const double* nf = r.node_force + (size_t)slot * ncomp * p.nbs;
   for (int q = warp; q < r.nforce * ncomp; q += kBlock / 32) {
-    const int ch = __ldg(r.force_chunks + q / ncomp), k = q % ncomp;
+    const int ch = s_chunks[q / ncomp], k = q % ncomp;
     double v[kBlock / 32];
 #pragma unroll
     for (int w = 0; w < kBlock / 32; ++w) {
@@ -339,7 +375,7 @@ __device__ __forceinline__ void resident_epilogue(const StepParams& p, const Res
   }
   me.sync();
   if (tid == 0) {
-    const int has_target = c->sched_on ? c->absorbing : c->has_target;
+    const int has_target = k0->sched_on ? k0->absorbing : k0->has_target;
     const double drho = p.np > 0 && has_target ? __ldcg(r.drho + slot) : 0.0;
     bool finite = true;
     for (int k = 0; k < ncomp; ++k) finite = finite && isfinite(s_force[k]);
@@ -347,17 +383,17 @@ __device__ __forceinline__ void resident_epilogue(const StepParams& p, const Res
       c->nonfinite = 1;
       c->nonfinite_t = t;
     }
-    if (c->rec_cap && t >= c->rec_start && t - c->rec_start < c->rec_cap) {
-      double* h = c->hist + (size_t)(t - c->rec_start) * kRec;
+    if (k0->rec_cap && t >= k0->rec_start && t - k0->rec_start < k0->rec_cap) {
+      double* h = k0->hist + (size_t)(t - k0->rec_start) * kRec;
       for (int k = 0; k < 2 * kMaxGroups; ++k) h[k] = k < ncomp ? s_force[k] : 0.0;
       h[8] = drho;
-      if (!c->dp_on) h[9] = 0.0;                                // else the probe, one step before this
+      if (!k0->dp_on) h[9] = 0.0;                               // else the probe, one step before this
     }
     if (final_step) {
       for (int k = 0; k < 2 * kMaxGroups; ++k) c->force[k] = k < ncomp ? s_force[k] : 0.0;
       c->drho = drho;
-      if (c->sched_on) {
-        const Controls k = read_controls(c, t);
+      if (k0->sched_on) {
+        const Controls k = read_controls(k0, t);
         c->vscale[1] = k.vs[1];
         c->vscale[2] = k.vs[2];
         c->target = k.target;
@@ -382,6 +418,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
   __shared__ int s_next[2];                                     // next segment of the block, by parity
   __shared__ int s_go;
   __shared__ double s_drho;
+  __shared__ int s_chunks[kBlock];                              // the last part's chunks with force
+  __shared__ Ctl s_ctl;                                         // the control block at the start
   extern __shared__ double s_dyn[];
   const int bid = (int)blockIdx.x, lane = (int)(threadIdx.x & 31u), warp = (int)threadIdx.x >> 5;
   Ctl* c = p.ctl;
@@ -394,10 +432,30 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
   double* s_un = s_dyn;                                         // the summing warp's outlet velocities
   TaskScratch<R>* scratch = (TaskScratch<R>*)(s_dyn + (p.np + 1) / 2 * 2);
   const int outlets = has_target ? __ldg(r.block_outlets + bid) : 0;
+  // The block's tasks, their nodes, wall and link records: copied to shared memory where they fit (the acquire
+  // of every step drops the L1, and a task would begin with a chain of L2 loads).
+  const int4 *nodes = r.nodes + (size_t)task0 * 32, *tds = r.tasks + task0;
+  const WallRec* walls = r.walls;
+  const LinkRecDev* links = (const LinkRecDev*)r.links;
+  if (r.tables && task1 > task0) {
+    const int w0 = __ldg(&tds[0].x), w1 = __ldg(&r.tasks[task1 - 1].y);
+    const int l0 = task0 > 0 ? __ldg(&tds[-1].w) : 0, l1 = __ldg(&r.tasks[task1 - 1].w);
+    uint4* at = (uint4*)(scratch + r.max_tasks);
+    nodes = copy_table(at, nodes, (task1 - task0) * 32);
+    tds = copy_table(at, tds, task1 - task0);
+    walls = copy_table(at, walls + w0, w1 - w0) - w0;           // (indexed as the whole tables are)
+    links = copy_table(at, links + l0, l1 - l0) - l0;
+  }
   const size_t force_set = (size_t)2 * p.ngroups * p.nbs;
 
+  static_assert(sizeof(Ctl) % 8 == 0, "copied in 8-byte words");
+  for (int k = (int)threadIdx.x; k < (int)(sizeof(Ctl) / 8); k += kResidentThreads)
+    ((unsigned long long*)&s_ctl)[k] = ((const unsigned long long*)c)[k];
+  if (last)
+    for (int k = me.tid(); k < r.nforce; k += kBlock) s_chunks[k] = __ldg(r.force_chunks + k);
+
   // controls of step s into shared memory (one thread)
-  auto controls = [&](int s) {
+  auto controls = [&](int s, const Ctl* c) {
     const Controls k = read_controls(c, t0 + (unsigned long long)s);
 #pragma unroll
     for (int g = 0; g < 4; ++g) s_vs[s & 1][g] = k.vs[g];
@@ -406,7 +464,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
     s_next[s & 1] = seg0;
   };
 
-  if (threadIdx.x == 0) controls(0);
+  if (threadIdx.x == 0) controls(0, c);
   for (int k = (int)threadIdx.x; k < 2 * kMaxGroups * kBlock; k += kResidentThreads) (&s_part[0][0])[k] = 0.0;
   // Outlet velocities of the start state; every block computes all of them into the same values, so
   // no grid-wide wait is needed before the first step.
@@ -415,7 +473,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
     double f[9];
 #pragma unroll
     for (int i = 0; i < 9; ++i) f[i] = (double)Store<S>::ld_cg(buf0 + (size_t)i * p.ns + idx, i);
-    __stcg(r.un + k, outlet_velocity(f, p, k));
+    __stcg(r.un + k, outlet_velocity(f, p, p.pnode_n[2 * k], p.pnode_n[2 * k + 1]));
   }
   __threadfence();
   // The nodes' own populations in the start state.
@@ -427,7 +485,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
 #pragma unroll
         for (int d = 0; d < 9; ++d) t.own[0][d][lane] = Store<S>::ld_cg(buf0 + (unsigned)d * p.ns + (unsigned)nd.x, d);
       }
-      open_prepare<S>(p, nd, __ldg(r.tasks + task).z, 0, t);
+      open_prepare<S>(p, (const LinkRecDev*)r.links, nd, __ldg(r.tasks + task).z, 0, t);
     }
   }
   __syncthreads();
@@ -440,12 +498,12 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
     const int slot2 = slot == 2 ? 0 : slot + 1;                 // (s - 2) % 3
 
     if (last) {
-      if (s > 0) record_probe<S>(p, a, (long long)(t0 + s) - 1, me);
-      if (s > 1) resident_epilogue<S>(p, r, t0 + s - 2, slot2, false, s_part, s_force, me);
+      if (s > 0) record_probe<S>(p, a, (long long)(t0 + s) - 1, &s_ctl, me);
+      if (s > 1) resident_epilogue<S>(p, r, t0 + s - 2, slot2, false, s_part, s_force, s_chunks, &s_ctl, me);
     } else if (warp < kResidentTaskWarps) {
       for (int task = task0 + warp; task < task1; task += kResidentTaskWarps) {
-        const int4 nd = __ldg(r.nodes + (size_t)task * 32 + lane), td = __ldg(r.tasks + task);
-        boundary_task<S, CK>(p, r, nd, td, a, b, s_vs[s & 1], s & 1, td.z == TASK_OUTLET ? outlets : 0, &s_drho,
+        const int4 nd = nodes[(task - task0) * 32 + lane], td = tds[task - task0];
+        boundary_task<S, CK>(p, nd, td, walls, a, b, s_vs[s & 1], s & 1, td.z == TASK_OUTLET ? outlets : 0, &s_drho,
                              r.un + ((s & 1) ^ 1) * p.np, scratch[task - task0]);
         __syncwarp();
       }
@@ -514,14 +572,14 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
     // After the arrival (the block has synchronised: the step's controls and counter are free).
     if (warp < kResidentTaskWarps) {
       for (int task = task0 + warp; task < task1; task += kResidentTaskWarps) {
-        const int4 nd = __ldg(r.nodes + (size_t)task * 32 + lane);
-        const int kind = __ldg(r.tasks + task).z;
+        const int4 nd = nodes[(task - task0) * 32 + lane];
+        const int kind = tds[task - task0].z;
         TaskScratch<R>& t = scratch[task - task0];
-        if (kind == TASK_OUTLET || kind == TASK_OPEN) open_prepare<S>(p, nd, kind, (s & 1) ^ 1, t);
-        if (kind != TASK_OUTLET) task_force<S>(p, nd, s_vs[s & 1], s & 1, r.node_force + slot * force_set, t);
+        if (kind == TASK_OUTLET || kind == TASK_OPEN) open_prepare<S>(p, links, nd, kind, (s & 1) ^ 1, t);
+        if (kind != TASK_OUTLET) task_force<S>(p, links, nd, s_vs[s & 1], s & 1, r.node_force + slot * force_set, t);
       }
     }
-    if (threadIdx.x == kResidentThreads - 32) controls(s + 1);
+    if (threadIdx.x == kResidentThreads - 32) controls(s + 1, &s_ctl);
     if (threadIdx.x == kResidentThreads - 64) {
       s_go = poll_arrived(r.arrived, target);
       if (!s_go) c->stalled = 1;
@@ -540,9 +598,10 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
   }
   __syncthreads();
   if (!s_go || !last) return;
-  record_probe<S>(p, (r.steps & 1) ? buf1 : buf0, (long long)(t0 + r.steps) - 1, me);
-  if (r.steps > 1) resident_epilogue<S>(p, r, t0 + r.steps - 2, slot == 2 ? 0 : slot + 1, false, s_part, s_force, me);
-  resident_epilogue<S>(p, r, t0 + r.steps - 1, slot == 0 ? 2 : slot - 1, true, s_part, s_force, me);
+  record_probe<S>(p, (r.steps & 1) ? buf1 : buf0, (long long)(t0 + r.steps) - 1, &s_ctl, me);
+  if (r.steps > 1)
+    resident_epilogue<S>(p, r, t0 + r.steps - 2, slot == 2 ? 0 : slot + 1, false, s_part, s_force, s_chunks, &s_ctl, me);
+  resident_epilogue<S>(p, r, t0 + r.steps - 1, slot == 0 ? 2 : slot - 1, true, s_part, s_force, s_chunks, &s_ctl, me);
 }
 
 }  // namespace vl
