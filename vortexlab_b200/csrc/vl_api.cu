@@ -690,15 +690,21 @@ vl::LinkRecDev device_link(const vl::LinkRec& h) {
 // Whether the resident step kernel takes this domain, and its tables. The rule on size, us per step of
 // the resident kernel / of the fastest schedule of two kernels (B200):
 //   towing tanks and rigs (an absorbing outlet: the two-kernel step waits for its serial outlet sum)
-//     FP64  442 x 84 5.3 / 12.7, 742 x 372 9.2 / 17.2, 1202 x 602 21.6 / 29.0, 1762 x 330 15.0 / 21.3
-//     FP32  302 x 152 5.6 / 13.7, 1042 x 522 10.9 / 21.0, 1802 x 902 27.8 / 35.4
-//     16-bit fixed point 1202 x 602 12.6 / 23.5
+//     FP64  442 x 84 5.4 / 12.3, 742 x 372 8.7 / 19.0, 1282 x 642 26.4 / 31.6, 1762 x 330 13.9 / 21.3
+//     FP32  302 x 152 5.6 / 13.2, 1002 x 502 9.8 / 19.9, 1282 x 642 14.1 / 22.7, 1822 x 912 29.2 / 35.4
+//     16-bit 1282 x 642 13.1 / 22.5 (half), 15.4 / 23.8 (custom), 13.4 / 23.3 (fixed point),
+//            1822 x 912 20.5 / 29.0, 26.8 / 31.2, 22.1 / 29.4
 //   boxes without an outlet
-//     FP64  300 x 200 4.9 / 9.9, 700 x 450 9.4 / 13.2, 1000 x 600 16.5 / 17.6, 1200 x 700 26.9 / 25.4
-//     FP32  700 x 450 7.9 / 12.1, 1001 x 600 11.9 / 14.4, 1600 x 900 29.3 / 21.0
-//     16-bit 1000 x 600 11.3 / 13.7 (fixed point), 13.0 / 13.4 (custom), 2002 x 1200 41.0 / 25.7
+//     FP64  300 x 200 5.1 / 12.1, 700 x 450 8.5 / 13.0, 1000 x 640 18.7 / 18.9; 1200 x 700 26.9 / 25.4
+//     FP32  700 x 450 8.0 / 12.0, 1000 x 640 11.6 / 13.3; 1600 x 900 29.3 / 21.0
+//     16-bit 1000 x 640 11.6 / 13.1, 13.9 / 13.8, 12.0 / 13.2; 2002 x 1200 41.0 / 25.7 (fixed point)
 // so: the two population buffers within the L2 (128 MB) and at most 1.7 M cells with an outlet, 0.64 M
-// without. Besides, no outlet node may have a link with a force group (its task forms no force terms), at
+// without. The force sums are one block's work, 0.24 us for a chunk of 256 boundary nodes and a group;
+// without them the step takes any number of boundary nodes (640 x 400, 104,000 links: 9.5 / 14.2). Boxes
+// of disks, FP64, with force on 29 chunks 640 x 400 10.6 / 12.8, 300 x 200 9.9 / 11.2; on 34 1000 x 600
+// 18.1 / 17.2; on 46 640 x 400 14.7 / 13.2; on 151 45 / 15.6. With an outlet on 39 300 x 200 13.2 / 14.9, on
+// 62 1000 x 600 25.9 / 27.4, on 72 640 x 400 21.9 / 20.1. So: at most 30 chunks with force times groups, 45 with
+// an outlet. Besides, no outlet node may have a link with a force group (its task forms no force terms), at
 // most kBlock chunks of boundary nodes (the force sums' shared memory).
 int resident_setup(vl_sim& s) {
   const vl::CompiledDomain& d = s.dom;
@@ -721,6 +727,14 @@ int resident_setup(vl_sim& s) {
     for (int l = d.bnode_first[g]; l < d.bnode_first[g + 1]; ++l) any = any || (d.links[(size_t)l].flags & 1);
     (any ? open : order).push_back(g);
   }
+  std::vector<uint8_t> chunk_force((size_t)s.P.nlink, 0);
+  for (size_t g = 0; g < nb; ++g)
+    for (int l = d.bnode_first[g]; l < d.bnode_first[g + 1]; ++l)
+      if (d.links[(size_t)l].fgroup >= 0) chunk_force[g / (size_t)vl::kBlock] = 1;
+  std::vector<int32_t> force_chunks;
+  for (size_t c = 0; c < chunk_force.size(); ++c)
+    if (chunk_force[c]) force_chunks.push_back((int32_t)c);
+  if (force_chunks.size() * (size_t)d.ngroups > (np > 0 ? 45u : 30u)) return VL_OK;
   int sms = 0;
   VL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s.device));
   if (sms < 2) return VL_OK;
@@ -750,7 +764,6 @@ int resident_setup(vl_sim& s) {
   std::vector<int4> nodes;
   std::vector<vl::WallRec> walls;
   std::vector<int4> trec;
-  std::vector<uint8_t> chunk_force((size_t)s.P.nlink, 0);
   std::vector<vl::LinkRecDev> tlinks;
   size_t most = 0, most_walls = 0, most_links = 0;
   for (int g = 0; g < G; ++g) {
@@ -776,10 +789,7 @@ int resident_setup(vl_sim& s) {
             continue;
           }
           mask |= 1 << j;
-          if (h.fgroup >= 0) {
-            mask |= 1 << (j + 18);
-            chunk_force[b / (size_t)vl::kBlock] = 1;
-          }
+          if (h.fgroup >= 0) mask |= 1 << (j + 18);
           vl::WallRec w;
           std::memset(&w, 0, sizeof w);
           w.slot = (unsigned)((size_t)(j - 1) * 32 + at);
@@ -818,9 +828,6 @@ int resident_setup(vl_sim& s) {
     most_walls = std::max(most_walls, walls.size() - walls0);
     most_links = std::max(most_links, tlinks.size() - links0);
   }
-  std::vector<int32_t> force_chunks;
-  for (size_t c = 0; c < chunk_force.size(); ++c)
-    if (chunk_force[c]) force_chunks.push_back((int32_t)c);
   vl::ResidentParams& RP = s.RP;
   RP.grid = G;
   RP.max_tasks = (int)most;
