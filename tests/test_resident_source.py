@@ -31,3 +31,12 @@ def test_every_wait_is_followed_by_a_block_barrier():
     for at in waits:
         rest = t[at:]
         assert rest.index("__syncthreads();") < re.search(r"if \(!s_go[^)]*\) return", rest).start()
+
+
+def test_no_two_blocks_write_one_word_of_the_outlet_sum():
+    """The outlet velocities of the start state go to each block's own shared memory, and one block records the
+    offset (all blocks used to store the same values to the same global words)."""
+    t = _text()
+    start = t[t.index("__global__ void"):t.index("for (int s = 0; s < r.steps; ++s)")]
+    assert "s_un[k] = outlet_velocity" in start and "r.un" not in start
+    assert re.search(r"if \(bid == 0\) __stcg\(r\.drho \+ slot, drho\);", t)

@@ -466,16 +466,15 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
 
   if (threadIdx.x == 0) controls(0, c);
   for (int k = (int)threadIdx.x; k < 2 * kMaxGroups * kBlock; k += kResidentThreads) (&s_part[0][0])[k] = 0.0;
-  // Outlet velocities of the start state; every block computes all of them into the same values, so
-  // no grid-wide wait is needed before the first step.
-  for (int k = (int)threadIdx.x; k < p.np; k += kResidentThreads) {
+  // Outlet velocities of the start state, in the shared memory of every block that sums them: no grid-wide
+  // wait is needed before the first step, and no two blocks write a word.
+  for (int k = (int)threadIdx.x; outlets > 0 && k < p.np; k += kResidentThreads) {
     const int idx = __ldg(p.pnode_idx + k);
     double f[9];
 #pragma unroll
     for (int i = 0; i < 9; ++i) f[i] = (double)Store<S>::ld_cg(buf0 + (size_t)i * p.ns + idx, i);
-    __stcg(r.un + k, outlet_velocity(f, p, p.pnode_n[2 * k], p.pnode_n[2 * k + 1]));
+    s_un[k] = outlet_velocity(f, p, p.pnode_n[2 * k], p.pnode_n[2 * k + 1]);
   }
-  __threadfence();
   // The nodes' own populations in the start state.
   if (warp < kResidentTaskWarps) {
     for (int task = task0 + warp; task < task1; task += kResidentTaskWarps) {
@@ -509,7 +508,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
       }
     } else if (outlets > 0 && warp == kResidentWarps - 1) {
       const double* un = r.un + (s & 1) * p.np;
-      for (int base = 0; base < p.np; base += 16 * 32) {        // 16 loads of a lane in flight
+      for (int base = 0; s > 0 && base < p.np; base += 16 * 32) {   // 16 loads of a lane in flight
         double v[16];
 #pragma unroll
         for (int m = 0; m < 16; ++m)
@@ -522,7 +521,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
       const double drho = (serial_sum(s_un, p.np) / (double)p.np - s_target[s & 1]) / p.sqrt_cs2;
       if (lane == 0) {
         s_drho = drho;
-        __stcg(r.drho + slot, drho);                            // (every block with outlet tasks writes this value)
+        if (bid == 0) __stcg(r.drho + slot, drho);              // (block 0 has outlet tasks if any block has)
       }
       __syncwarp();
       outlet_sum_ready(outlets);
