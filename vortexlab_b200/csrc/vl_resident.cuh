@@ -118,6 +118,16 @@ __device__ __forceinline__ const T* copy_table(uint4*& at, const T* src, int n) 
   return out;
 }
 
+// Where a block finds its tables (kept in shared memory: pointers held over the steps would be spilled, and
+// the acquire drops the spilled lines too).
+struct BlockTables {
+  const int4* nodes;            // of its first task
+  const int4* tasks;
+  const WallRec* walls;
+  const LinkRecDev* links;
+  int ntasks;
+};
+
 // One part of a block.
 struct PartOf {
   int part;
@@ -420,6 +430,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
   __shared__ double s_drho;
   __shared__ int s_chunks[kBlock];                              // the last part's chunks with force
   __shared__ Ctl s_ctl;                                         // the control block at the start
+  __shared__ BlockTables s_tab;
   extern __shared__ double s_dyn[];
   const int bid = (int)blockIdx.x, lane = (int)(threadIdx.x & 31u), warp = (int)threadIdx.x >> 5;
   Ctl* c = p.ctl;
@@ -434,17 +445,20 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
   const int outlets = has_target ? __ldg(r.block_outlets + bid) : 0;
   // The block's tasks, their nodes, wall and link records: copied to shared memory where they fit (the acquire
   // of every step drops the L1, and a task would begin with a chain of L2 loads).
-  const int4 *nodes = r.nodes + (size_t)task0 * 32, *tds = r.tasks + task0;
-  const WallRec* walls = r.walls;
-  const LinkRecDev* links = (const LinkRecDev*)r.links;
-  if (r.tables && task1 > task0) {
-    const int w0 = __ldg(&tds[0].x), w1 = __ldg(&r.tasks[task1 - 1].y);
-    const int l0 = task0 > 0 ? __ldg(&tds[-1].w) : 0, l1 = __ldg(&r.tasks[task1 - 1].w);
-    uint4* at = (uint4*)(scratch + r.max_tasks);
-    nodes = copy_table(at, nodes, (task1 - task0) * 32);
-    tds = copy_table(at, tds, task1 - task0);
-    walls = copy_table(at, walls + w0, w1 - w0) - w0;           // (indexed as the whole tables are)
-    links = copy_table(at, links + l0, l1 - l0) - l0;
+  {
+    const int4 *nodes = r.nodes + (size_t)task0 * 32, *tds = r.tasks + task0;
+    const WallRec* walls = r.walls;
+    const LinkRecDev* links = (const LinkRecDev*)r.links;
+    if (r.tables && task1 > task0) {
+      const int w0 = __ldg(&tds[0].x), w1 = __ldg(&r.tasks[task1 - 1].y);
+      const int l0 = task0 > 0 ? __ldg(&tds[-1].w) : 0, l1 = __ldg(&r.tasks[task1 - 1].w);
+      uint4* at = (uint4*)(scratch + r.max_tasks);
+      nodes = copy_table(at, nodes, (task1 - task0) * 32);
+      tds = copy_table(at, tds, task1 - task0);
+      walls = copy_table(at, walls + w0, w1 - w0) - w0;         // (indexed as the whole tables are)
+      links = copy_table(at, links + l0, l1 - l0) - l0;
+    }
+    if (threadIdx.x == 0) s_tab = {nodes, tds, walls, links, task1 - task0};
   }
   const size_t force_set = (size_t)2 * p.ngroups * p.nbs;
 
@@ -500,10 +514,10 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
       if (s > 0) record_probe<S>(p, a, (long long)(t0 + s) - 1, &s_ctl, me);
       if (s > 1) resident_epilogue<S>(p, r, t0 + s - 2, slot2, false, s_part, s_force, s_chunks, &s_ctl, me);
     } else if (warp < kResidentTaskWarps) {
-      for (int task = task0 + warp; task < task1; task += kResidentTaskWarps) {
-        const int4 nd = nodes[(task - task0) * 32 + lane], td = tds[task - task0];
-        boundary_task<S, CK>(p, nd, td, walls, a, b, s_vs[s & 1], s & 1, td.z == TASK_OUTLET ? outlets : 0, &s_drho,
-                             r.un + ((s & 1) ^ 1) * p.np, scratch[task - task0]);
+      for (int task = warp; task < s_tab.ntasks; task += kResidentTaskWarps) {
+        const int4 nd = s_tab.nodes[task * 32 + lane], td = s_tab.tasks[task];
+        boundary_task<S, CK>(p, nd, td, s_tab.walls, a, b, s_vs[s & 1], s & 1, td.z == TASK_OUTLET ? outlets : 0, &s_drho,
+                             r.un + ((s & 1) ^ 1) * p.np, scratch[task]);
         __syncwarp();
       }
     } else if (outlets > 0 && warp == kResidentWarps - 1) {
@@ -570,12 +584,12 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
     target += (unsigned)r.grid;
     // After the arrival (the block has synchronised: the step's controls and counter are free).
     if (warp < kResidentTaskWarps) {
-      for (int task = task0 + warp; task < task1; task += kResidentTaskWarps) {
-        const int4 nd = nodes[(task - task0) * 32 + lane];
-        const int kind = tds[task - task0].z;
-        TaskScratch<R>& t = scratch[task - task0];
-        if (kind == TASK_OUTLET || kind == TASK_OPEN) open_prepare<S>(p, links, nd, kind, (s & 1) ^ 1, t);
-        if (kind != TASK_OUTLET) task_force<S>(p, links, nd, s_vs[s & 1], s & 1, r.node_force + slot * force_set, t);
+      for (int task = warp; task < s_tab.ntasks; task += kResidentTaskWarps) {
+        const int4 nd = s_tab.nodes[task * 32 + lane];
+        const int kind = s_tab.tasks[task].z;
+        TaskScratch<R>& t = scratch[task];
+        if (kind == TASK_OUTLET || kind == TASK_OPEN) open_prepare<S>(p, s_tab.links, nd, kind, (s & 1) ^ 1, t);
+        if (kind != TASK_OUTLET) task_force<S>(p, s_tab.links, nd, s_vs[s & 1], s & 1, r.node_force + slot * force_set, t);
       }
     }
     if (threadIdx.x == kResidentThreads - 32) controls(s + 1, &s_ctl);
