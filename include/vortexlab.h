@@ -159,6 +159,11 @@ int vl_sim_init(vl_sim* s, const double* rho, const double* ux, const double* uy
                 double rho0, double ux0, double uy0);
 /* Sim::step :391-420, `steps` times, queued on the sim's stream (returns before completion). */
 int vl_sim_step(vl_sim* s, uint64_t steps);
+/* Exercises the error path of the kernel that takes many steps of a small domain in one launch: its blocks wait for
+ * one arrival more than they make, and the waits run out (after seconds). From then on every call
+ * that steps the sim or reads its state fails with VL_ECUDA, until vl_sim_init starts it again. VL_EINVAL for a
+ * sim that this kernel does not take. */
+int vl_sim_test_stall(vl_sim* s, uint64_t steps);
 int vl_sim_synchronize(vl_sim* s);
 int vl_sim_set_vscale(vl_sim* s, int group, double value);                 /* pub vscale :196 */
 int vl_sim_get_vscale(const vl_sim* s, double* out4);

@@ -152,6 +152,7 @@ struct vl_sim {
     void* ptrs[] = {buf[0], buf[1], d_flag, d_bidx, d_bfirst, d_links, d_pidx, d_pn, d_ctl,
                     d_partials, d_hist, d_sched, d_red, d_cells, d_gather, d_bdesc, d_wbfirst, d_lb, d_ownc, d_lnode};
     for (void* p : d_res) cudaFree(p);
+    if (RP.host_stalled) cudaFreeHost((void*)RP.host_stalled);
     if (d_scratch) cudaFree(d_scratch);
     for (void* p : ptrs)
       if (p) cudaFree(p);
@@ -174,8 +175,28 @@ struct vl_sim {
   // Reads the device control block into the host mirror (synchronises the stream).
   int pull_ctl() {
     VL_CUDA(cudaMemcpyAsync(&hctl, d_ctl, sizeof(vl::Ctl), cudaMemcpyDeviceToHost, stream));
+    return sync();
+  }
+  // Whether a wait of the resident step kernel ran out (after the stream has been waited for: in any step so
+  // far). The state is then half a step's; every call that steps or reads it fails until vl_sim_init.
+  bool stalled() const { return RP.host_stalled && *RP.host_stalled; }
+  int check_stall() const {
+    if (stalled())
+      return fail(VL_ECUDA, "resident step kernel: a block gave up waiting for the others (vl_sim_init starts again)");
+    return VL_OK;
+  }
+  int sync() {
     VL_CUDA(cudaStreamSynchronize(stream));
-    if (hctl.stalled) return fail(VL_ECUDA, "resident step kernel: a block gave up waiting for the others");
+    return check_stall();
+  }
+  // For a new start state: the kernel's counter and flags as they were when the sim was built, if it stalled.
+  int clear_stall() {
+    VL_CUDA(cudaStreamSynchronize(stream));
+    if (!stalled()) return VL_OK;
+    VL_CUDA(cudaMemsetAsync(RP.arrived, 0, sizeof(unsigned), stream));
+    VL_CUDA(cudaMemsetAsync(&d_ctl->stalled, 0, sizeof(int), stream));
+    res_arrived = 0;
+    *RP.host_stalled = 0;
     return VL_OK;
   }
 
@@ -435,7 +456,7 @@ struct vl_sim {
   }
 
   // Steps in the resident kernel, a bounded number per launch. `done`: false when it cannot run here.
-  int step_resident(uint64_t steps, bool& done) {
+  int step_resident(uint64_t steps, bool& done, bool test_stall = false) {
     done = false;
     if (int rc = resident_tables()) return rc;
     if (!resident_ok) return VL_OK;
@@ -443,7 +464,7 @@ struct vl_sim {
     uint64_t left = steps;
     while (left > 0) {
       RP.steps = (int)std::min<uint64_t>(left, kResidentMaxSteps);
-      RP.arrived0 = res_arrived;
+      RP.arrived0 = res_arrived + (test_stall ? 1u : 0u);      // (one arrival more than there are blocks to make it)
       cudaError_t e = L->resident(P, RP, ck, buf[cur], buf[cur ^ 1], stream);
       if (e != cudaSuccess) return cuda_fail(e, "resident step kernel");
       res_arrived += (unsigned)(RP.steps + 1) * (unsigned)RP.grid;
@@ -461,6 +482,7 @@ struct vl_sim {
 
   int step(uint64_t steps) {
     VL_CUDA(cudaSetDevice(device));
+    if (int rc = check_stall()) return rc;
     if (resident && resident_ok && !P.stream && steps >= (uint64_t)kResidentMinSteps) {
       bool done = false;
       if (int rc = step_resident(steps, done)) return rc;
@@ -494,6 +516,7 @@ struct vl_sim {
   std::vector<cudaEvent_t> pev;
   int step_profiled(uint64_t steps, double* link_ms, double* bulk_ms, double* total_ms) {
     VL_CUDA(cudaSetDevice(device));
+    if (int rc = check_stall()) return rc;
     const size_t need = 4 * (size_t)steps + 2;
     while (pev.size() < need) {
       cudaEvent_t e;
@@ -563,8 +586,7 @@ struct vl_sim {
     cudaError_t e = L->gather((int)cells.size(), ns, d_cells, a(), d_gather, stream);
     if (e != cudaSuccess) return cuda_fail(e, "gather");
     VL_CUDA(cudaMemcpyAsync(out.data(), d_gather, out.size() * sizeof(double), cudaMemcpyDeviceToHost, stream));
-    VL_CUDA(cudaStreamSynchronize(stream));
-    return VL_OK;
+    return sync();
   }
 };
 
@@ -856,7 +878,11 @@ int resident_setup(vl_sim& s) {
   put(&RP.node_force, nullptr, 3 * (size_t)2 * d.ngroups * s.P.nbs * f8, true);
   put(&RP.un, nullptr, 2 * np * f8, true);
   put(&RP.drho, nullptr, 3 * f8, true);
+  int* flag = nullptr;
+  if (ok && cudaHostAlloc(&flag, sizeof(int), cudaHostAllocMapped) != cudaSuccess) ok = false;
   if (!ok) return VL_ENOMEM;
+  *flag = 0;
+  RP.host_stalled = flag;                                       // (one address for the host and the device)
   RP.seg_first = s.d_res_seg;
   s.resident_ok = true;
   return VL_OK;
@@ -1308,8 +1334,8 @@ int vl_sim_init(vl_sim* s, const double* rho, const double* ux, const double* uy
   if (e != cudaSuccess) return cuda_fail(e, "init");
   s->own_ok = false;
   // t = 0 (src/sim.rs:370); the force and the outlet offset restart from zero.
-  int rc = s->pull_ctl();
-  if (rc) return rc;
+  int rc = s->clear_stall();
+  if (rc || (rc = s->pull_ctl())) return rc;
   s->hctl.t = 0;
   s->hctl.arrive = 0;
   s->hctl.nonfinite = 0;
@@ -1327,10 +1353,17 @@ int vl_sim_step(vl_sim* s, uint64_t steps) {
   return s->step(steps);
 }
 
+int vl_sim_test_stall(vl_sim* s, uint64_t steps) {
+  if (!s || !s->resident_ok) return fail(VL_EINVAL, "test_stall: not a sim that the resident step kernel takes");
+  VL_CUDA(cudaSetDevice(s->device));
+  if (int rc = s->check_stall()) return rc;
+  bool done = false;
+  return s->step_resident(steps, done, true);
+}
+
 int vl_sim_synchronize(vl_sim* s) {
   if (!s) return fail(VL_EINVAL, "null sim");
-  VL_CUDA(cudaStreamSynchronize(s->stream));
-  return VL_OK;
+  return s->sync();
 }
 
 int vl_sim_set_vscale(vl_sim* s, int g, double v) {
@@ -1408,8 +1441,7 @@ int vl_sim_download(vl_sim* s, double* out) {
     s->scratch_done();
     if (e != cudaSuccess) return cuda_fail(e, "download");
   }
-  VL_CUDA(cudaStreamSynchronize(s->stream));
-  return VL_OK;
+  return s->sync();
 }
 
 int vl_sim_upload(vl_sim* s, const double* in) {
@@ -1428,8 +1460,7 @@ int vl_sim_upload(vl_sim* s, const double* in) {
     cudaFree(tmp);
     if (e != cudaSuccess) return cuda_fail(e, "upload");
   }
-  VL_CUDA(cudaStreamSynchronize(s->stream));
-  return VL_OK;
+  return s->sync();
 }
 
 int vl_sim_flags(vl_sim* s, uint8_t* out) {
@@ -1453,7 +1484,7 @@ int vl_sim_macros_field(vl_sim* s, double* rho, double* ux, double* uy) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
   s->scratch_done();
   if (e != cudaSuccess) return cuda_fail(e, "macros_field");
-  return VL_OK;
+  return s->check_stall();
 }
 
 int vl_sim_macros(vl_sim* s, size_t x, size_t y, double* out3) {
@@ -1478,7 +1509,7 @@ static int sim_reduce(vl_sim* s, double* mass, double* mom, double* vmax) {
   if (e != cudaSuccess) return cuda_fail(e, "reduce");
   std::vector<double> r(kReduceBlocks * 7);
   VL_CUDA(cudaMemcpyAsync(r.data(), s->d_red, r.size() * 8, cudaMemcpyDeviceToHost, s->stream));
-  VL_CUDA(cudaStreamSynchronize(s->stream));
+  if (int rc = s->sync()) return rc;
   // Fixed-order combination of the per-block compensated sums.
   double acc[6] = {0, 0, 0, 0, 0, 0};
   double vm = 0.0;
@@ -1536,7 +1567,7 @@ int vl_sim_vorticity(vl_sim* s, float* out) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
   s->scratch_done();
   if (e != cudaSuccess) return cuda_fail(e, "vorticity");
-  return VL_OK;
+  return s->check_stall();
 }
 
 int vl_sim_probe_density(vl_sim* s, double x, double y, double* out) {
@@ -1632,7 +1663,7 @@ int vl_sim_last_step_ms(vl_sim* s, float* ms) {
   if (!s->timed) return fail(VL_EINVAL, "no step batch timed yet");
   VL_CUDA(cudaEventSynchronize(s->ev1));
   VL_CUDA(cudaEventElapsedTime(ms, s->ev0, s->ev1));
-  return VL_OK;
+  return s->check_stall();
 }
 
 int vl_sim_set_schedule(vl_sim* s, int schedule) {

@@ -30,8 +30,9 @@
 // 26.0, disk box of 700 x 450 FP64 9.4 / 10.1 / 8.5. Every value is computed by the functions of
 // the two-kernel step in their order, so states, forces and records are bit-identical to it.
 //
-// Every wait is bounded (kWaitPolls polls); a block that gives up sets Ctl::stalled and leaves, and
-// so do the blocks that wait for it. The launch is cooperative: all blocks are on the chip at once.
+// Every wait is bounded (kWaitPolls polls); a block that gives up sets Ctl::stalled and the host's flag
+// and leaves, and so do the blocks that wait for it and all blocks of later launches. The launch is
+// cooperative: all blocks are on the chip at once.
 #pragma once
 
 #include "vl_device.cuh"
@@ -84,6 +85,7 @@ struct ResidentParams {
   int tables;                   // the block's tasks, nodes, wall and link records are copied to its shared memory
   const int32_t* force_chunks;  // chunks that hold a node with force
   int nforce;
+  volatile int* host_stalled;   // in host memory: set with Ctl::stalled
   unsigned* arrived;            // arrivals since the sim was built
   unsigned arrived0;            // arrivals before this launch
   double* node_force;           // three sets of [2 * ngroups][nbs], zero for nodes without force
@@ -153,6 +155,13 @@ __device__ __forceinline__ bool poll_arrived(const unsigned* counter, unsigned t
     }
   }
   return false;
+}
+
+// A wait ran out (one thread of each block that gives up).
+__device__ __forceinline__ void mark_stalled(const StepParams& p, const ResidentParams& r) {
+  *(volatile int*)&p.ctl->stalled = 1;
+  *r.host_stalled = 1;
+  __threadfence_system();
 }
 
 // The named barrier between a block's summing warp and its outlet tasks' warps.
@@ -434,6 +443,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
   extern __shared__ double s_dyn[];
   const int bid = (int)blockIdx.x, lane = (int)(threadIdx.x & 31u), warp = (int)threadIdx.x >> 5;
   Ctl* c = p.ctl;
+  // An earlier launch gave up (one thread reads the flag: the block leaves as one).
+  if (__syncthreads_or(threadIdx.x == 0 && *(volatile int*)&c->stalled)) return;
   const unsigned long long t0 = c->t;
   const int seg0 = __ldg(r.seg_first + bid), seg1 = __ldg(r.seg_first + bid + 1);
   const int task0 = __ldg(r.task_first + bid), task1 = __ldg(r.task_first + bid + 1);
@@ -593,23 +604,21 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
       }
     }
     if (threadIdx.x == kResidentThreads - 32) controls(s + 1, &s_ctl);
-    if (threadIdx.x == kResidentThreads - 64) {
-      s_go = poll_arrived(r.arrived, target);
-      if (!s_go) c->stalled = 1;
-    }
+    if (threadIdx.x == kResidentThreads - 64) s_go = poll_arrived(r.arrived, target);
     __syncthreads();
-    if (!s_go) return;
+    if (!s_go) {
+      if (threadIdx.x == 0) mark_stalled(p, r);
+      return;
+    }
     slot = slot2;
   }
   // The force terms of the last step are complete after one more arrival.
   grid_arrive(r.arrived);
   target += (unsigned)r.grid;
   if (bid != r.grid - 1) return;
-  if (threadIdx.x == 0) {
-    s_go = poll_arrived(r.arrived, target);
-    if (!s_go) c->stalled = 1;
-  }
+  if (threadIdx.x == 0) s_go = poll_arrived(r.arrived, target);
   __syncthreads();
+  if (!s_go && threadIdx.x == 0) mark_stalled(p, r);
   if (!s_go || !last) return;
   record_probe<S>(p, (r.steps & 1) ? buf1 : buf0, (long long)(t0 + r.steps) - 1, &s_ctl, me);
   if (r.steps > 1)
