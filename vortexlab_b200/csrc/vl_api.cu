@@ -85,6 +85,44 @@ __global__ void k_vorticity(int nx, int ny, const uint8_t* __restrict__ flag, co
 
 int vl::set_error(int code, const char* msg) { return fail(code, msg); }
 
+namespace {
+
+// Flags in host memory that a kernel can set (one address for the host and every device). Handed out from pages of
+// 1,024, kept for the next sim: a page takes 2.3 ms to allocate and a third of that to release.
+class HostFlags {
+ public:
+  volatile int* take() {
+    std::lock_guard<std::mutex> guard(m_);
+    if (free_.empty()) {
+      int* page = nullptr;
+      if (cudaHostAlloc(&page, kPage * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+      }
+      for (int k = 0; k < kPage; ++k) free_.push_back(page + k);
+    }
+    volatile int* f = free_.back();
+    free_.pop_back();
+    *f = 0;
+    return f;
+  }
+  void give(volatile int* f) {
+    std::lock_guard<std::mutex> guard(m_);
+    free_.push_back(f);
+  }
+
+ private:
+  static constexpr int kPage = 1024;
+  std::mutex m_;
+  std::vector<volatile int*> free_;
+};
+HostFlags& host_flags() {
+  static HostFlags* f = new HostFlags;                          // (outlives every sim)
+  return *f;
+}
+
+}  // namespace
+
 // ==================================================================== device-resident sim
 struct vl_sim {
   int device = 0;
@@ -135,10 +173,9 @@ struct vl_sim {
   bool resident = true;            // no schedule was chosen by name
   int res_v = 0;                   // cells per thread that the segment table was made for
   vl::ResidentParams RP{};
-  int32_t* d_res_seg = nullptr;    // one of them: the segment table
+  int32_t* d_res_seg = nullptr;    // the segment table (in d_res)
   std::vector<int32_t> res_task_first, res_outlets;   // first task / outlet tasks of each block
-  // device tables and buffers of the kernel (ResidentParams), one allocation each
-  std::vector<void*> d_res;
+  void* d_res = nullptr;           // device tables and buffers of the kernel (ResidentParams)
   unsigned res_arrived = 0;        // arrivals of every launch so far
   uint64_t t_host = 0;
   uint64_t rec_start = 0, rec_cap = 0;
@@ -151,8 +188,8 @@ struct vl_sim {
     if (gexec) cudaGraphExecDestroy(gexec);
     void* ptrs[] = {buf[0], buf[1], d_flag, d_bidx, d_bfirst, d_links, d_pidx, d_pn, d_ctl,
                     d_partials, d_hist, d_sched, d_red, d_cells, d_gather, d_bdesc, d_wbfirst, d_lb, d_ownc, d_lnode};
-    for (void* p : d_res) cudaFree(p);
-    if (RP.host_stalled) cudaFreeHost((void*)RP.host_stalled);
+    if (d_res) cudaFree(d_res);
+    if (RP.host_stalled) host_flags().give(RP.host_stalled);    // (after cudaFree, which waited for the kernels)
     if (d_scratch) cudaFree(d_scratch);
     for (void* p : ptrs)
       if (p) cudaFree(p);
@@ -856,33 +893,43 @@ int resident_setup(vl_sim& s) {
   RP.max_walls = (int)most_walls;
   RP.max_links = (int)most_links;
   RP.nforce = (int)force_chunks.size();
-  bool ok = true;
-  auto put = [&](auto** dst, const void* src, size_t bytes, bool zero) {
-    void* q = nullptr;
-    if (!ok || alloc_copy(&q, src, bytes) != VL_OK) { ok = false; return; }
-    s.d_res.push_back(q);
-    if (zero && cudaMemset(q, 0, bytes ? bytes : 16) != cudaSuccess) { fail(VL_ECUDA, "resident tables"); ok = false; }
-    *dst = (std::remove_pointer_t<decltype(dst)>)q;
+  // One allocation: the tables, copied in one piece, then what starts from zero. Without it (or the host's flag)
+  // the sim takes the two-kernel step.
+  std::vector<char> host;
+  size_t total = 0;
+  std::vector<std::pair<void**, size_t>> at;
+  auto put = [&](auto** dst, const void* src, size_t bytes) {
+    at.emplace_back((void**)dst, total);
+    if (src) {
+      host.resize(total + bytes);
+      if (bytes) std::memcpy(host.data() + total, src, bytes);
+    }
+    total = (total + bytes + 255) / 256 * 256;
   };
   const size_t f8 = sizeof(double);
-  put(&s.d_res_seg, nullptr, ((size_t)G + 1) * 4, true);
-  put(&RP.task_first, s.res_task_first.data(), s.res_task_first.size() * 4, false);
-  put(&RP.nodes, nodes.data(), nodes.size() * sizeof(int4), false);
-  put(&RP.walls, walls.data(), walls.size() * sizeof(vl::WallRec), false);
-  put(&RP.links, tlinks.data(), tlinks.size() * sizeof(vl::LinkRecDev), false);
-  put(&RP.tasks, trec.data(), trec.size() * sizeof(int4), false);
+  put(&RP.task_first, s.res_task_first.data(), s.res_task_first.size() * 4);
+  put(&RP.nodes, nodes.data(), nodes.size() * sizeof(int4));
+  put(&RP.walls, walls.data(), walls.size() * sizeof(vl::WallRec));
+  put(&RP.links, tlinks.data(), tlinks.size() * sizeof(vl::LinkRecDev));
+  put(&RP.tasks, trec.data(), trec.size() * sizeof(int4));
+  put(&RP.block_outlets, block_outlets.data(), block_outlets.size() * 4);
+  put(&RP.force_chunks, force_chunks.data(), force_chunks.size() * 4);
+  const size_t copied = total;
+  put(&s.d_res_seg, nullptr, ((size_t)G + 1) * 4);
+  put(&RP.arrived, nullptr, sizeof(unsigned));
+  put(&RP.node_force, nullptr, 3 * (size_t)2 * d.ngroups * s.P.nbs * f8);
+  put(&RP.un, nullptr, 2 * np * f8);
+  put(&RP.drho, nullptr, 3 * f8);
+  if (cudaMalloc(&s.d_res, total) != cudaSuccess || !(RP.host_stalled = host_flags().take())) {
+    cudaGetLastError();
+    if (s.d_res) cudaFree(s.d_res);
+    s.d_res = nullptr;
+    return VL_OK;
+  }
+  for (const auto& a : at) *a.first = (char*)s.d_res + a.second;
+  if (!host.empty()) VL_CUDA(cudaMemcpy(s.d_res, host.data(), host.size(), cudaMemcpyHostToDevice));
+  VL_CUDA(cudaMemset((char*)s.d_res + copied, 0, total - copied));
   s.res_outlets = block_outlets;
-  put(&RP.block_outlets, block_outlets.data(), block_outlets.size() * 4, false);
-  put(&RP.force_chunks, force_chunks.data(), force_chunks.size() * 4, false);
-  put(&RP.arrived, nullptr, sizeof(unsigned), true);
-  put(&RP.node_force, nullptr, 3 * (size_t)2 * d.ngroups * s.P.nbs * f8, true);
-  put(&RP.un, nullptr, 2 * np * f8, true);
-  put(&RP.drho, nullptr, 3 * f8, true);
-  int* flag = nullptr;
-  if (ok && cudaHostAlloc(&flag, sizeof(int), cudaHostAllocMapped) != cudaSuccess) ok = false;
-  if (!ok) return VL_ENOMEM;
-  *flag = 0;
-  RP.host_stalled = flag;                                       // (one address for the host and the device)
   RP.seg_first = s.d_res_seg;
   s.resident_ok = true;
   return VL_OK;
