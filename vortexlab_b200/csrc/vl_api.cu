@@ -824,6 +824,9 @@ int resident_setup(vl_sim& s) {
   std::vector<vl::WallRec> walls;
   std::vector<int4> trec;
   std::vector<vl::LinkRecDev> tlinks;
+  nodes.reserve(tasks.size() * 32);
+  walls.reserve(d.links.size());
+  trec.reserve(tasks.size());
   size_t most = 0, most_walls = 0, most_links = 0;
   for (int g = 0; g < G; ++g) {
     size_t count = 0;
@@ -893,17 +896,17 @@ int resident_setup(vl_sim& s) {
   RP.max_walls = (int)most_walls;
   RP.max_links = (int)most_links;
   RP.nforce = (int)force_chunks.size();
-  // One allocation: the tables, copied in one piece, then what starts from zero. Without it (or the host's flag)
-  // the sim takes the two-kernel step.
-  std::vector<char> host;
+  // One allocation: the tables, then what starts from zero. Without it (or the host's flag) the sim takes the
+  // two-kernel step.
+  struct Part {
+    void** dst;
+    const void* src;
+    size_t bytes, at;
+  };
+  std::vector<Part> parts;
   size_t total = 0;
-  std::vector<std::pair<void**, size_t>> at;
   auto put = [&](auto** dst, const void* src, size_t bytes) {
-    at.emplace_back((void**)dst, total);
-    if (src) {
-      host.resize(total + bytes);
-      if (bytes) std::memcpy(host.data() + total, src, bytes);
-    }
+    parts.push_back({(void**)dst, src, bytes, total});
     total = (total + bytes + 255) / 256 * 256;
   };
   const size_t f8 = sizeof(double);
@@ -926,8 +929,10 @@ int resident_setup(vl_sim& s) {
     s.d_res = nullptr;
     return VL_OK;
   }
-  for (const auto& a : at) *a.first = (char*)s.d_res + a.second;
-  if (!host.empty()) VL_CUDA(cudaMemcpy(s.d_res, host.data(), host.size(), cudaMemcpyHostToDevice));
+  for (const Part& q : parts) {
+    *q.dst = (char*)s.d_res + q.at;
+    if (q.src && q.bytes) VL_CUDA(cudaMemcpy(*q.dst, q.src, q.bytes, cudaMemcpyHostToDevice));
+  }
   VL_CUDA(cudaMemset((char*)s.d_res + copied, 0, total - copied));
   s.res_outlets = block_outlets;
   RP.seg_first = s.d_res_seg;
