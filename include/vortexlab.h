@@ -164,6 +164,9 @@ int vl_sim_step(vl_sim* s, uint64_t steps);
  * that steps the sim or reads its state fails with VL_ECUDA, until vl_sim_init starts it again. VL_EINVAL for a
  * sim that this kernel does not take. */
 int vl_sim_test_stall(vl_sim* s, uint64_t steps);
+/* vl_sim_step with a launch of that kernel that asks for more blocks than the device holds: it is refused, and the sim
+ * takes these and all later steps by the two-kernel step. */
+int vl_sim_test_refused(vl_sim* s, uint64_t steps);
 int vl_sim_synchronize(vl_sim* s);
 int vl_sim_set_vscale(vl_sim* s, int group, double value);                 /* pub vscale :196 */
 int vl_sim_get_vscale(const vl_sim* s, double* out4);

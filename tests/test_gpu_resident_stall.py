@@ -43,3 +43,29 @@ def test_other_sims_do_not_stall(gpu):
     assert V.lib.vl_sim_test_stall(sim._h, 8) < 0
     sim.step(8)
     sim.synchronize()
+
+
+@pytest.mark.parametrize("before", [0, 5])
+def test_refused_launch_takes_the_two_kernel_step(gpu, before):
+    """A cooperative launch that the device refuses (here for its number of blocks): the same steps by two kernels."""
+    V = gpu
+    got = []
+    for refuse in (False, True):
+        sim = S.product_sim(S.tunnel_like(radiating=True))
+        sim.init((1.0, 0.02, 0.0))
+        sim.record(120)
+        sim.vscale[1], sim.vscale[2] = 0.5, 0.002
+        if before:
+            sim.step(before)
+        if refuse:
+            V._lib.check(V.lib.vl_sim_test_refused(sim._h, 70))
+        else:
+            sim.step(70)
+        n0 = sim.launch_count()
+        sim.step(40)
+        assert (sim.launch_count() - n0 > 40) == refuse
+        assert sim.last_step_ms() > 0
+        got.append((sim.populations(), sim.history(), sim.t))
+    assert got[0][2] == got[1][2] == 110 + before
+    assert np.isfinite(got[0][0]).all()
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])

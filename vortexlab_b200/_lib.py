@@ -87,6 +87,7 @@ def _declare(L):
         "vl_sim_init": (i, [vp, P(d), P(d), P(d), d, d, d]),
         "vl_sim_step": (i, [vp, u64]),
         "vl_sim_test_stall": (i, [vp, u64]),
+        "vl_sim_test_refused": (i, [vp, u64]),
         "vl_sim_synchronize": (i, [vp]),
         "vl_sim_set_vscale": (i, [vp, i, d]),
         "vl_sim_get_vscale": (i, [vp, P(d)]),

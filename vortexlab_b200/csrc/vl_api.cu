@@ -492,42 +492,50 @@ struct vl_sim {
     return VL_OK;
   }
 
-  // Steps in the resident kernel, a bounded number per launch. `done`: false when it cannot run here.
-  int step_resident(uint64_t steps, bool& done, bool test_stall = false) {
-    done = false;
+  // Steps in the resident kernel, a bounded number per launch. `left`: the steps still to take, some or all of
+  // them if its launch was refused (fewer blocks than it needs may be had at once, in a partition of the device
+  // say): the sim then takes the two-kernel step.
+  enum class Test { none, stall, refuse };
+  int step_resident(uint64_t& left, Test test = Test::none) {
     if (int rc = resident_tables()) return rc;
     if (!resident_ok) return VL_OK;
     VL_CUDA(cudaEventRecord(ev0, stream));
-    uint64_t left = steps;
     while (left > 0) {
       RP.steps = (int)std::min<uint64_t>(left, kResidentMaxSteps);
-      RP.arrived0 = res_arrived + (test_stall ? 1u : 0u);      // (one arrival more than there are blocks to make it)
-      cudaError_t e = L->resident(P, RP, ck, buf[cur], buf[cur ^ 1], stream);
-      if (e != cudaSuccess) return cuda_fail(e, "resident step kernel");
+      RP.arrived0 = res_arrived + (test == Test::stall ? 1u : 0u);   // (one arrival more than there are blocks to make it)
+      const int grid = RP.grid;
+      if (test == Test::refuse) RP.grid = 1 << 24;
+      const cudaError_t e = L->resident(P, RP, ck, buf[cur], buf[cur ^ 1], stream);
+      RP.grid = grid;
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        resident_ok = false;
+        return VL_OK;
+      }
       res_arrived += (unsigned)(RP.steps + 1) * (unsigned)RP.grid;
       launches += 1;
       cur ^= RP.steps & 1;
       left -= (uint64_t)RP.steps;
+      own_ok = false;
     }
-    VL_CUDA(cudaEventRecord(ev1, stream));
-    timed = true;
-    t_host += steps;
-    own_ok = false;
-    done = true;
     return VL_OK;
   }
 
-  int step(uint64_t steps) {
+  int step(uint64_t steps, Test test = Test::none) {
     VL_CUDA(cudaSetDevice(device));
     if (int rc = check_stall()) return rc;
+    uint64_t left = steps;
     if (resident && resident_ok && !P.stream && steps >= (uint64_t)kResidentMinSteps) {
-      bool done = false;
-      if (int rc = step_resident(steps, done)) return rc;
-      if (done) return VL_OK;
+      if (int rc = step_resident(left, test)) return rc;
+      if (left == 0) {
+        VL_CUDA(cudaEventRecord(ev1, stream));
+        timed = true;
+        t_host += steps;
+        return VL_OK;
+      }
     }
     if (int rc = prepare_steps()) return rc;
-    VL_CUDA(cudaEventRecord(ev0, stream));
-    uint64_t left = steps;
+    if (left == steps) VL_CUDA(cudaEventRecord(ev0, stream));
     while (left > 0) {
       if (left >= (uint64_t)kGraphSteps && cur == 0) {
         int rc = ensure_graph();
@@ -1407,10 +1415,15 @@ int vl_sim_step(vl_sim* s, uint64_t steps) {
 
 int vl_sim_test_stall(vl_sim* s, uint64_t steps) {
   if (!s || !s->resident_ok) return fail(VL_EINVAL, "test_stall: not a sim that the resident step kernel takes");
-  VL_CUDA(cudaSetDevice(s->device));
-  if (int rc = s->check_stall()) return rc;
-  bool done = false;
-  return s->step_resident(steps, done, true);
+  if (s->P.stream || steps < kResidentMinSteps) return fail(VL_EINVAL, "test_stall: too few steps, or bulk copies");
+  s->resident = true;
+  return s->step(steps, vl_sim::Test::stall);
+}
+
+int vl_sim_test_refused(vl_sim* s, uint64_t steps) {
+  if (!s || !s->resident_ok) return fail(VL_EINVAL, "test_refused: not a sim that the resident step kernel takes");
+  s->resident = true;
+  return s->step(steps, vl_sim::Test::refuse);
 }
 
 int vl_sim_synchronize(vl_sim* s) {
