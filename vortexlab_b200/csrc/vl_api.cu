@@ -340,8 +340,8 @@ struct vl_sim {
   }
 
   int set_schedule(int sc) {
-    resident = false;
     if (sc < 0 || sc >= VL_SCHEDULE_COUNT) return fail(VL_EINVAL, "schedule must be 0, 1, 2 or 3");
+    resident = false;
     if (sc != schedule && gexec) {
       VL_CUDA(cudaStreamSynchronize(stream));
       cudaGraphExecDestroy(gexec);
