@@ -1,0 +1,85 @@
+"""The resident step kernel takes most of the device for a call, so a sim leaves it alone while a batch or three
+more sims have work in flight: their two-kernel steps overlap. The results are the same."""
+import threading
+
+import numpy as np
+import pytest
+
+import scenarios as S
+
+pytestmark = pytest.mark.gpu
+
+LONG = 40000    # steps of a small tank: some tenths of a second
+
+
+def _tank(prec="f64"):
+    sim = S.product_sim(S.tunnel_like(radiating=True), precision=prec)
+    sim.init((1.0, 0.02, 0.0))
+    sim.vscale[1], sim.vscale[2] = 0.5, 0.002
+    return sim
+
+
+def _launches(sim, steps):
+    n0 = sim.launch_count()
+    sim.step(steps)
+    return sim.launch_count() - n0
+
+
+def test_fourth_sim_takes_the_two_kernel_step(gpu):
+    a, b, e, c = _tank(), _tank("f32"), _tank(), _tank()
+    ref = _tank()
+    ref.schedule = "concurrent"
+    ref.step(3 * 64)
+    ref.synchronize()
+    assert _launches(c, 64) == 1
+    for s in (a, b, e, c):      # (a kernel's first launch may wait for the device)
+        if s is not c:
+            s.step(64)
+        s.synchronize()
+    for s in (a, b, e):
+        assert _launches(s, LONG) < 20                              # two others in flight at most: still resident
+    assert _launches(c, 64) > 60                                    # three others
+    for s in (a, b, e, c):
+        s.synchronize()
+    assert _launches(c, 64) == 1                                    # none any more
+    assert np.array_equal(c.populations(), ref.populations())
+
+
+def test_sim_beside_a_batch(gpu):
+    from vortexlab_b200.batch import Batch, seeded_tunnels
+    cs = seeded_tunnels(count=4, dmin=15, dmax=20, units=400.0)
+    b = Batch("f32")
+    for t in cs:
+        b.add(t.tunnel.spec_warm(t.body), t.steps)
+    b.build()
+    sim = _tank()
+    b.run_async(8000)
+    assert _launches(sim, 64) > 60
+    b.wait()
+    sim.synchronize()
+    assert _launches(sim, 64) == 1
+    del b
+    assert _launches(sim, 64) == 1
+
+
+def test_sims_come_and_go_on_threads(gpu):
+    ref = _tank()
+    ref.schedule = "concurrent"
+    ref.step(300)
+    want = ref.populations()
+    bad = []
+
+    def work():
+        for _ in range(5):
+            s = _tank()
+            for n in (100, 7, 193):
+                s.step(n)
+            if not np.array_equal(s.populations(), want):
+                bad.append(1)
+
+    ts = [threading.Thread(target=work) for _ in range(6)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad

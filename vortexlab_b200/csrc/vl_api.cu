@@ -14,6 +14,7 @@
 #include "../../include/vortexlab.h"
 #include "vl_device.cuh"
 #include "vl_host.hpp"
+#include "vl_inflight.hpp"
 #include "vl_internal.hpp"
 #include "vl_launch.hpp"
 #include "vl_resident.cuh"
@@ -123,6 +124,50 @@ HostFlags& host_flags() {
 
 }  // namespace
 
+// ==================================================================== work in flight
+vl::InFlight& vl::InFlight::of_process() {
+  static InFlight* f = new InFlight;                            // (outlives every sim and batch)
+  return *f;
+}
+void vl::InFlight::add(Work* w) {
+  std::lock_guard<std::mutex> guard(m_);
+  if (std::find(all_.begin(), all_.end(), w) == all_.end()) all_.push_back(w);
+}
+void vl::InFlight::remove(Work* w) {
+  std::lock_guard<std::mutex> guard(m_);
+  all_.erase(std::remove(all_.begin(), all_.end(), w), all_.end());
+}
+void vl::InFlight::start(Work* w) {
+  std::lock_guard<std::mutex> guard(m_);
+  ++w->calls;
+}
+void vl::InFlight::finish(Work* w) {
+  std::lock_guard<std::mutex> guard(m_);
+  --w->calls;
+  w->queued = true;
+}
+bool vl::InFlight::many_others(const Work* w) {
+  std::lock_guard<std::mutex> guard(m_);
+  // (the query must not end a stream capture that another thread has under way)
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  int n = 0;
+  for (Work* o : all_) {
+    if (o == w || o->device != w->device) continue;
+    if (o->calls == 0) {
+      if (!o->queued) continue;
+      if (cudaEventQuery(o->end) != cudaErrorNotReady) {
+        o->queued = false;
+        continue;
+      }
+    }
+    if ((n += o->weight) >= Work::kMany) break;
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  cudaGetLastError();
+  return n >= Work::kMany;
+}
+
 // ==================================================================== device-resident sim
 struct vl_sim {
   int device = 0;
@@ -177,6 +222,7 @@ struct vl_sim {
   std::vector<int32_t> res_task_first, res_outlets;   // first task / outlet tasks of each block
   void* d_res = nullptr;           // device tables and buffers of the kernel (ResidentParams)
   unsigned res_arrived = 0;        // arrivals of every launch so far
+  vl::Work work;                   // (in the process's list once the sim is built)
   uint64_t t_host = 0;
   uint64_t rec_start = 0, rec_cap = 0;
   bool timed = false;
@@ -184,6 +230,7 @@ struct vl_sim {
   vl::Ctl hctl{};
 
   ~vl_sim() {
+    vl::InFlight::of_process().remove(&work);
     if (device >= 0) cudaSetDevice(device);
     if (gexec) cudaGraphExecDestroy(gexec);
     void* ptrs[] = {buf[0], buf[1], d_flag, d_bidx, d_bfirst, d_links, d_pidx, d_pn, d_ctl,
@@ -524,8 +571,10 @@ struct vl_sim {
   int step(uint64_t steps, Test test = Test::none) {
     VL_CUDA(cudaSetDevice(device));
     if (int rc = check_stall()) return rc;
+    vl::InFlightCall call(&work);
     uint64_t left = steps;
-    if (resident && resident_ok && !P.stream && steps >= (uint64_t)kResidentMinSteps) {
+    if (resident && resident_ok && !P.stream && steps >= (uint64_t)kResidentMinSteps &&
+        !vl::InFlight::of_process().many_others(&work)) {
       if (int rc = step_resident(left, test)) return rc;
       if (left == 0) {
         VL_CUDA(cudaEventRecord(ev1, stream));
@@ -1007,6 +1056,9 @@ vl_sim* make_sim(vl::CompiledDomain&& dom, int precision) {
     fail(VL_ECUDA, "stream/event creation");
     return nullptr;
   }
+  s->work.device = s->device;
+  s->work.end = s->ev1;
+  vl::InFlight::of_process().add(&s->work);
   // Launch geometry: one bulk block per row tile of kBlock cells; one link thread per boundary
   // node, and at least one link block (it runs the end-of-step epilogue).
   const bool forced = d.accel[0] != 0.0 || d.accel[1] != 0.0;

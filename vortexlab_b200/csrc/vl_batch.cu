@@ -17,6 +17,7 @@
 
 #include "../../include/vortexlab.h"
 #include "vl_batch.cuh"
+#include "vl_inflight.hpp"
 #include "vl_internal.hpp"
 #include "vl_launch.hpp"
 
@@ -90,6 +91,7 @@ struct vl_batch {
   bool own_ok = false;                   // d_ownc holds the active tunnels' current boundary nodes
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  vl::Work work;                         // (in the process's list once the batch is built)
   vl::BatchParams P{};
   int ntiles = 0, nchunks = 0;
   int schedule = 0;
@@ -110,6 +112,7 @@ struct vl_batch {
   size_t h_stage_cap = 0;                // doubles
 
   ~vl_batch() {
+    vl::InFlight::of_process().remove(&work);
     cudaSetDevice(device);
     if (gexec) cudaGraphExecDestroy(gexec);
     for (cudaGraphExec_t g : retired) cudaGraphExecDestroy(g);
@@ -265,6 +268,7 @@ struct vl_batch {
   // Enqueues the steps of a run on the stream without waiting for them.
   int enqueue_run(uint64_t max_steps) {
     VB_CUDA(cudaSetDevice(device));
+    vl::InFlightCall call(&work);
     uint64_t end_all = 0;
     for (size_t k = 0; k < tun.size(); ++k) end_all = std::max<uint64_t>(end_all, end_of(k));
     const uint64_t stop = max_steps ? std::min<uint64_t>(end_all, s + max_steps) : end_all;
@@ -509,6 +513,10 @@ int vl_batch_build(vl_batch* b) {
   VB_CUDA(cudaStreamCreateWithFlags(&b->copy, cudaStreamNonBlocking));
   VB_CUDA(cudaEventCreate(&b->ev0));
   VB_CUDA(cudaEventCreate(&b->ev1));
+  b->work.device = b->device;
+  b->work.end = b->ev1;
+  b->work.weight = vl::Work::kMany;      // a batch fills the device by itself
+  vl::InFlight::of_process().add(&b->work);
   // Start states: uniform rest, or the inflow profile when the tunnel has no ramp
   // (src/cases/channel.rs:108-110), into both buffers.
   for (size_t k = 0; k < nt; ++k) {
