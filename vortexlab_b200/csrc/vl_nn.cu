@@ -14,6 +14,7 @@
 #include "../../include/vortexlab.h"
 #include "vl_conv.cuh"
 #include "vl_gemm.cuh"
+#include "vl_groups.hpp"
 #include "vl_launch.hpp"
 
 using bf16 = __nv_bfloat16;
@@ -965,7 +966,7 @@ __global__ void k_up2_bwd(const float* __restrict__ dy, int B, int H, int W, int
 }
 
 // The same moves for channel counts and offsets of whole 16-byte groups (V = 8 BF16 or 4 FP32 values) and fewer
-// than 2^32 groups: one group a thread, 32-bit index arithmetic. (The kernels of one value a thread spend their
+// than 2^31 groups (vl_groups.hpp): one group a thread, 32-bit index arithmetic. (The kernels of one value a thread spend their
 // time on 64-bit divisions: 524,288 pixels x 64 of 96 channels, us: up2 208 -> 26, copy 43 -> 16, slice 46 -> 27,
 // up2_bwd 59 -> 33.) `gc`: groups of C; `gt`, `go`: of ctot and coff.
 __global__ void k_up2_v(const uint4* __restrict__ x, unsigned total, unsigned H, unsigned W, unsigned gc, uint4* __restrict__ y,
@@ -1084,13 +1085,13 @@ __global__ void k_f32_to_bf16(const float* __restrict__ a, long long n, bf16* __
 }
 
 int grid_for(long long n) {
+  constexpr long long most = vl::kMoveThreads / 256;
   long long g = (n + 255) / 256;
-  return (int)(g < 148 * 32 ? (g < 1 ? 1 : g) : 148 * 32);
+  return (int)(g < most ? (g < 1 ? 1 : g) : most);
 }
 
-// Whether channel moves between [.., C] and channels [coff, coff + C) of [.., ctot] go in groups of v values.
 bool grouped(const void* a, const void* b, long long values, int C, int ctot, int coff, int v) {
-  return C % v == 0 && ctot % v == 0 && coff % v == 0 && !(((uintptr_t)a | (uintptr_t)b) & 15) && values / v < 0xffffffffLL;
+  return vl::move_grouped((uintptr_t)a, (uintptr_t)b, values, C, ctot, coff, v);
 }
 
 int launch_check(const char* what) {
