@@ -294,14 +294,12 @@ int launch_rows(const void* x, int B, int H, int W, int C, const void* w, int kp
   // All output channels in one block, their 9 C x bn weights and a ring of five rows in its shared memory;
   // two blocks an SM where both fit. (In two or three parts, 192 -> 64 channels took 53 us as in k_conv, 64 -> 192
   // 47 against 41.)
-  const int row_bytes = p.chunks * p.box_bytes;
-  const auto weight_bytes = [&](int bn) { return (9 * C * bn * 2 + 1023) / 1024 * 1024; };
   constexpr int kMost = 220 * 1024;
   if (N > 256) return VL_OK;
   p.bn = N <= 32 ? 32 : (N + 63) / 64 * 64;
-  if (weight_bytes(p.bn) + 5 * row_bytes + 1024 > kMost) return VL_OK;
+  if ((9LL * C * p.bn * 2 + 1023) / 1024 * 1024 + 5LL * p.chunks * p.box_bytes + 1024 > kMost) return VL_OK;
+  const int row_bytes = p.chunks * p.box_bytes, wb = (9 * C * p.bn * 2 + 1023) / 1024 * 1024;
   p.tmem_cols = p.bn <= 32 ? 32 : (p.bn <= 64 ? 64 : (p.bn <= 128 ? 128 : 256));
-  const int wb = weight_bytes(p.bn);
   const int per_sm = 4 * p.tmem_cols <= 512 && wb + 5 * row_bytes + 1024 <= kMost / 2 ? 2 : 1;
   p.ring = std::min(kRowsMaxRing, (kMost / per_sm - 1024 - wb) / row_bytes);
   p.Ho = H;
