@@ -1670,9 +1670,9 @@ int vl_sim_vorticity(vl_sim* s, float* out) {
   const size_t n = s->n;
   double* tmp = nullptr;
   std::lock_guard<std::mutex> guard(s->scratch_mutex);
-  int rc = s->scratch(3 * n * sizeof(double) + n * sizeof(float), (void**)&tmp);
+  int rc = s->scratch(3 * n * sizeof(double), (void**)&tmp);
   if (rc) return rc;
-  float* w = (float*)(tmp + 3 * n);
+  float* w = (float*)tmp;                                       // (over the density, which the curl does not read)
   cudaError_t e = s->L->macros((int)n, s->ns, s->d_flag, s->dom.accel[0], s->dom.accel[1], s->a(), tmp, tmp + n,
                                tmp + 2 * n, s->stream);
   if (e == cudaSuccess) {
