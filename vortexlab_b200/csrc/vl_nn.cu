@@ -571,23 +571,30 @@ int vl_nn_conv_bf16(const void* x, int B, int H, int W, int C, int stride, int t
   p.bn = (N + parts - 1) / parts;
   p.bn = p.bn <= 32 ? 32 : (p.bn + 63) / 64 * 64;
   // FP32 results of few tiles: the K split of launch_gemm for the same product (there for more blocks),
-  // so that the sums are the same
+  // so that the sums are the same; with accumulation they are formed in the workspace and added as there
   p.kb_split = taps * p.chunks;
+  const long long rows = (long long)B * p.Ho * p.Wo;
+  float* sums = nullptr;
   {
     const int gbn = N <= 32 ? 32 : (N <= 64 ? 64 : (N <= 128 ? 128 : 256)), kb64 = (kp + BK - 1) / BK;
-    const long long gt = (((long long)B * p.Ho * p.Wo + BM - 1) / BM) * ((N + gbn - 1) / gbn);
-    if (gt < 148 && kb64 >= 16 && !(flags & (EPI_BIAS | EPI_RELU | EPI_BF16 | EPI_ACCUM))) {
+    const long long gt = ((rows + BM - 1) / BM) * ((N + gbn - 1) / gbn);
+    if (gt < 148 && kb64 >= 16 && !(flags & (EPI_BIAS | EPI_RELU | EPI_BF16))) {
       const int splits = std::max(1, std::min(kb64 / 8, (int)((296 + gt - 1) / gt)));
       p.kb_split = std::min(p.kb_split, (kb64 + splits - 1) / splits * (BK / kc));
+      if ((flags & EPI_ACCUM) && p.kb_split < taps * p.chunks) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (int rc = workspace(dev, (size_t)rows * N * sizeof(float), (void**)&sums)) return rc;
+      }
     }
   }
   p.tmem_cols = p.bn <= 32 ? 32 : (p.bn <= 64 ? 64 : (p.bn <= 128 ? 128 : 256));
   p.ep = EpiParams{};
-  p.ep.out = out;
-  p.ep.ldc = ldc;
+  p.ep.out = sums ? sums : out;
+  p.ep.ldc = sums ? N : ldc;
   p.ep.bias = bias;
   p.ep.n_valid = N;
-  p.ep.flags = flags & (EPI_ACCUM | EPI_BIAS | EPI_RELU | EPI_BF16);
+  p.ep.flags = sums ? 0 : flags & (EPI_ACCUM | EPI_BIAS | EPI_RELU | EPI_BF16);
   p.ep.err = err;
   p.ep.spin_limit = kSpinLimit;
   // Rows of whole 128-pixel tiles (or nearly: at most a quarter more tiles than the best shape) without a K split
@@ -602,7 +609,8 @@ int vl_nn_conv_bf16(const void* x, int B, int H, int W, int C, int stride, int t
   if (rc) return rc;
   rc = make_map(&tb, w, (uint64_t)N, (uint64_t)kp, (uint64_t)kp, (uint32_t)p.bn, kc);
   if (rc) return rc;
-  return kc == 64 ? launch_conv<64>(ta, tb, p, N, (cudaStream_t)stream) : launch_conv<32>(ta, tb, p, N, (cudaStream_t)stream);
+  rc = kc == 64 ? launch_conv<64>(ta, tb, p, N, (cudaStream_t)stream) : launch_conv<32>(ta, tb, p, N, (cudaStream_t)stream);
+  return rc || !sums ? rc : split_reduce(sums, 1, (int)rows, N, (float*)out, ldc, 1, (cudaStream_t)stream);
 }
 
 int vl_nn_dgrad2_bf16(const void* dz, int B, int H, int W, int C, int N, const void* wt, float* dx, int accumulate, int* err,
