@@ -421,7 +421,7 @@ int vl_nn_gemm_bf16(const void* a, int lda, const void* b, int ldb, int M, int N
  * of stride 1 with kp = 64 and N at most 256; taps 9: 3x3 with padding 1 and
  * stride 1 or 2; taps 1: 1x1): out[pixel, n] = epilogue(sum over (tap, c) x[pixel + tap, c] w[n, (tap, c)]),
  * w BF16 [N][kp] with columns in (ky, kx, c) order, N, kp and ldc in multiples of 8, out 32-byte aligned; flags, bias and err as
- * vl_nn_gemm_bf16, and the same results bit for bit as im2col and that GEMM. */
+ * vl_nn_gemm_bf16 (VL_GEMM_TEST_TIMEOUT too), and the same results bit for bit as im2col and that GEMM. */
 int vl_nn_conv_bf16(const void* x, int B, int H, int W, int C, int stride, int taps, const void* w, int kp, int N,
                     void* out, int ldc, const float* bias, int flags, int* err, void* stream);
 /* Weight gradient of a 3x3 layer without the im2col matrix: gwt [kp][N] FP32 = sum over pixels of
@@ -434,6 +434,12 @@ int vl_nn_wgrad_bf16(const void* x, int B, int H, int W, int C, int stride, cons
  * (ky, kx, c) order), C in multiples of 8, N of 32, dx 32-byte aligned. */
 int vl_nn_dgrad2_bf16(const void* dz, int B, int H, int W, int C, int N, const void* wt, float* dx, int accumulate, int* err,
                       void* stream);
+/* The two gradients with a load left out, as VL_GEMM_TEST_TIMEOUT: the waits run out and *err is set (gwt and dx hold no
+ * result). */
+int vl_nn_wgrad_test_timeout(const void* x, int B, int H, int W, int C, int stride, const void* dz, int N, float* gwt, int kp,
+                             int* err, void* stream);
+int vl_nn_dgrad2_test_timeout(const void* dz, int B, int H, int W, int C, int N, const void* wt, float* dx, int accumulate,
+                              int* err, void* stream);
 int vl_nn_im2col(const void* x, int B, int H, int W, int C, int stride, int kp, void* cols, void* stream);
 int vl_nn_col2im(const float* dcols, int B, int H, int W, int C, int stride, int kp, float* dx, int accumulate,
                  void* stream);

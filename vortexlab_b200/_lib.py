@@ -164,6 +164,8 @@ def _declare(L):
         "vl_nn_conv_bf16": (i, [vp, i, i, i, i, i, i, vp, i, i, vp, i, P(f), i, P(i), vp]),
         "vl_nn_wgrad_bf16": (i, [vp, i, i, i, i, i, vp, i, vp, i, P(i), vp]),
         "vl_nn_dgrad2_bf16": (i, [vp, i, i, i, i, i, vp, vp, i, P(i), vp]),
+        "vl_nn_wgrad_test_timeout": (i, [vp, i, i, i, i, i, vp, i, vp, i, P(i), vp]),
+        "vl_nn_dgrad2_test_timeout": (i, [vp, i, i, i, i, i, vp, vp, i, P(i), vp]),
         "vl_nn_im2col": (i, [vp, i, i, i, i, i, i, vp, vp]),
         "vl_nn_flip_weights": (i, [vp, i, i, i, i, vp, vp]),
         "vl_nn_col2im": (i, [vp, i, i, i, i, i, i, vp, i, vp]),

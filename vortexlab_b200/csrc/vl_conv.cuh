@@ -85,6 +85,9 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t da, uint64_t db
       "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
 }
 
+// Bytes to expect of loads of `bytes`: with the test hook on, more than come, so that the waits for them run out.
+__device__ __forceinline__ uint32_t expected(uint32_t bytes, int drop_load) { return bytes + (drop_load ? 16u : 0u); }
+
 // One lane of the (converged) warp. The issuing loops run on the whole warp, so that descriptors and
 // counters are warp-uniform values (the MMA takes them from uniform registers), and this lane issues.
 __device__ __forceinline__ bool elect_one() {
@@ -213,6 +216,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
   if (threadIdx.x == 0) {
     // loads: the stages of the ring in turn, in tile and K order (the counters are kept, not divided: a
     // division in this loop costs as much as the load it issues)
+    const uint32_t bytes = expected((uint32_t)stage_bytes, ep.drop_load);
     int s = 0, issued = 0;
     uint32_t phase = 1;                         // of the empty barriers: the first round passes at once
     bool ok = true;
@@ -228,7 +232,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const __grid_constant_
           break;
         }
         uint8_t* sa = smem + s * stage_bytes;
-        mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
+        mbar_expect_tx(&full[s], bytes);
         tma_load_4d(&tmA, &full[s], sa, c0, x0 + kx, y0 + ky, b);
         tma_load_2d(&tmB, &full[s], sa + BM * KC * 2, kb * KC, n0);
         ++issued;
@@ -406,6 +410,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv_rows(const __grid_cons
   const uint32_t tmem = tmem_base;
 
   if (threadIdx.x == 0) {
+    const uint32_t bytes = expected((uint32_t)(p.chunks * kRowPixels * KC * 2), ep.drop_load);
     mbar_expect_tx(&wfull, (uint32_t)(9 * p.chunks * wtap_bytes));
     for (int k = 0; k < 9 * p.chunks; ++k) tma_load_2d(&tmB, &wfull, weights + k * wtap_bytes, k * KC, n0);
     int s = 0, issued = 0;
@@ -420,7 +425,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv_rows(const __grid_cons
           ok = false;
           break;
         }
-        mbar_expect_tx(&full[s], (uint32_t)(p.chunks * kRowPixels * KC * 2));
+        mbar_expect_tx(&full[s], bytes);
         for (int c = 0; c < p.chunks; ++c) tma_load_4d(&tmA, &full[s], rows + s * row_bytes + c * p.box_bytes, c * KC, tx * BM - 1, y, b);
         ++issued;
         if (++s == p.ring) {
@@ -591,6 +596,7 @@ __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtens
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_base;
   if (threadIdx.x == 0) {
+    const uint32_t bytes = expected((uint32_t)stage_bytes, ep.drop_load);
     // the KC-wide column blocks of this tile: their tap and first channel (past the last: all zero)
     constexpr int NB = BM / KC;
     int kx[NB], ky[NB], c0[NB];
@@ -609,7 +615,7 @@ __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtens
     for (int kb = 0; kb < kblocks; ++kb) {
       if (!mbar_wait(&empty[s], phase, ep.spin_limit)) { atomicExch(&failed, 1); break; }
       uint8_t* sa = smem + s * stage_bytes;
-      mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
+      mbar_expect_tx(&full[s], bytes);
 #pragma unroll
       for (int i = 0; i < NB; ++i)
         tma_load_4d(&tmA, &full[s], sa + i * (64 * KC * 2), c0[i], x * p.stride - p.pad + kx[i], y * p.stride - p.pad + ky[i], b);
@@ -746,7 +752,7 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_rows(const __grid_constant__ C
     int x = r0 % p.Wo, y = r0 / p.Wo, b = y / p.Ho;
     y -= b * p.Ho;
     const int boxes = (p.bn + 63) / 64;
-    const uint32_t bytes = (uint32_t)(kWgradPixels * KC * 2 + p.bn * 128);
+    const uint32_t bytes = expected((uint32_t)(kWgradPixels * KC * 2 + p.bn * 128), ep.drop_load);
     for (int kb = 0; kb < kblocks; ++kb) {
       if (!mbar_wait(&empty[s], phase, ep.spin_limit)) { atomicExch(&failed, 1); break; }
       uint8_t* sa = smem + s * p.stage_bytes;
@@ -924,7 +930,7 @@ __global__ void __launch_bounds__(288, 1) k_conv_first(const __grid_constant__ C
   } else if (warp == 4) {
     const uint32_t idesc = instr_desc_bf16(p.bn);
     if (elect_one()) {
-      mbar_expect_tx(&wfull, (uint32_t)(p.bn * 128));
+      mbar_expect_tx(&wfull, expected((uint32_t)(p.bn * 128), ep.drop_load));
       tma_load_2d(&tmB, &wfull, weights, 0, 0);
     }
     __syncwarp();
@@ -1036,7 +1042,7 @@ __global__ void __launch_bounds__(160, 1) k_wgrad_first(const __grid_constant__ 
       const int s = kb % kFirstStages;
       if (!mbar_wait(&empty[s], ((uint32_t)(kb / kFirstStages) & 1u) ^ 1u, ep.spin_limit)) return false;
       if (elect_one()) {
-        mbar_expect_tx(&full[s], (uint32_t)(p.bn * 128));
+        mbar_expect_tx(&full[s], expected((uint32_t)(p.bn * 128), ep.drop_load));
         for (int c = 0; c < boxes; ++c)
           tma_load_2d(&tmB, &full[s], smem + s * stage_bytes + 8192 + 8192 * c, 64 * c, (kb_first + kb) * 64);
       }
@@ -1103,6 +1109,7 @@ struct Dgrad2Params {
   int H, W, C, chunks;                  // dx; chunks of KC channels n
   int stages, n_valid;
   int accumulate;
+  int drop_load;                        // test hook, as EpiParams::drop_load
   float* dx;
   int* err;
   unsigned spin_limit;
@@ -1144,6 +1151,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_dgrad2(const __grid_constan
   const int per_class = p.units / 4;            // (the class of four taps first)
 
   if (threadIdx.x == 0) {
+    const uint32_t bytes = expected((uint32_t)STAGE, p.drop_load);
     int s = 0, issued = 0;
     uint32_t phase = 1;
     bool ok = true;
@@ -1161,7 +1169,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_dgrad2(const __grid_constan
               break;
             }
             uint8_t* sa = smem + s * STAGE;
-            mbar_expect_tx(&full[s], (uint32_t)STAGE);
+            mbar_expect_tx(&full[s], bytes);
             tma_load_4d(&tmA, &full[s], sa, c * KC, j0 + dx, i0 + dy, b);
             tma_load_2d(&tmB, &full[s], sa + BM * KC * 2, c * KC, (ky * 3 + kx) * p.C + n0);
             ++issued;

@@ -457,6 +457,13 @@ int launch_dgrad2(const CUtensorMap& ta, const CUtensorMap& tb, vl::gemm::Dgrad2
   return e == cudaSuccess ? VL_OK : fail(VL_ECUDA, std::string("input gradient launch: ") + cudaGetErrorString(e));
 }
 
+// How long a kernel's waits last, and whether a load that they wait for is left out (VL_GEMM_TEST_TIMEOUT).
+constexpr unsigned kTestSpins = 1u << 12;
+void test_timeout(vl::gemm::EpiParams& ep, int flags) {
+  ep.drop_load = (flags & VL_GEMM_TEST_TIMEOUT) ? 1 : 0;
+  ep.spin_limit = ep.drop_load ? kTestSpins : vl::gemm::kSpinLimit;
+}
+
 // The 4-channel layer (x: [B, H, W, 4], 3x3, stride 1).
 int launch_conv_first(const void* x, int B, int H, int W, const void* w, int kp, int N, const vl::gemm::EpiParams& ep,
                       cudaStream_t s) {
@@ -537,7 +544,7 @@ int vl_nn_conv_bf16(const void* x, int B, int H, int W, int C, int stride, int t
     ep.n_valid = N;
     ep.flags = flags & (EPI_BIAS | EPI_RELU | EPI_BF16);
     ep.err = err;
-    ep.spin_limit = kSpinLimit;
+    test_timeout(ep, flags);
     return launch_conv_first(x, B, H, W, w, kp, N, ep, (cudaStream_t)stream);
   }
   const int kc = C % 64 == 0 ? 64 : 32;
@@ -596,7 +603,7 @@ int vl_nn_conv_bf16(const void* x, int B, int H, int W, int C, int stride, int t
   p.ep.n_valid = N;
   p.ep.flags = sums ? 0 : flags & (EPI_ACCUM | EPI_BIAS | EPI_RELU | EPI_BF16);
   p.ep.err = err;
-  p.ep.spin_limit = kSpinLimit;
+  test_timeout(p.ep, flags);
   // Rows of whole 128-pixel tiles (or nearly: at most a quarter more tiles than the best shape) without a K split
   if (stride == 1 && taps == 9 && p.kb_split == taps * p.chunks && 4LL * ((W + BM - 1) / BM) * H <= 5 * best) {
     bool done = false;
@@ -613,8 +620,8 @@ int vl_nn_conv_bf16(const void* x, int B, int H, int W, int C, int stride, int t
   return rc || !sums ? rc : split_reduce(sums, 1, (int)rows, N, (float*)out, ldc, 1, (cudaStream_t)stream);
 }
 
-int vl_nn_dgrad2_bf16(const void* dz, int B, int H, int W, int C, int N, const void* wt, float* dx, int accumulate, int* err,
-                      void* stream) {
+static int dgrad2(const void* dz, int B, int H, int W, int C, int N, const void* wt, float* dx, int accumulate, int* err,
+                  void* stream, int flags) {
   using namespace vl::gemm;
   if (!dz || !wt || !dx || B < 1 || H < 1 || W < 1 || C < 8 || C % 8 || N < 32 || N % 32 || ((uintptr_t)dx & 31))
     return fail(VL_EINVAL, "stride-2 input gradient: C in 8s, N in 32s, 32-byte aligned result");
@@ -626,9 +633,10 @@ int vl_nn_dgrad2_bf16(const void* dz, int B, int H, int W, int C, int N, const v
   p.n_valid = C;
   p.chunks = N / kc;
   p.accumulate = accumulate;
+  p.drop_load = (flags & VL_GEMM_TEST_TIMEOUT) ? 1 : 0;
   p.dx = dx;
   p.err = err;
-  p.spin_limit = kSpinLimit;
+  p.spin_limit = p.drop_load ? kTestSpins : kSpinLimit;
   const int hh = (H + 1) / 2, hw = (W + 1) / 2;                 // dz's grid, and that of the pixels of a class
   long long best = 0;
   for (int lw = 7; lw >= 3; --lw) {
@@ -656,8 +664,8 @@ int vl_nn_dgrad2_bf16(const void* dz, int B, int H, int W, int C, int N, const v
   return bn == 32 ? launch_dgrad2<32, 32>(ta, tb, p, s) : launch_dgrad2<32, 64>(ta, tb, p, s);
 }
 
-int vl_nn_wgrad_bf16(const void* x, int B, int H, int W, int C, int stride, const void* dz, int N, float* gwt, int kp,
-                     int* err, void* stream) {
+static int wgrad(const void* x, int B, int H, int W, int C, int stride, const void* dz, int N, float* gwt, int kp, int* err,
+                 void* stream, int flags) {
   using namespace vl::gemm;
   if (!x || !dz || !gwt || B < 1 || H < 1 || W < 1 || N < 1 || (stride != 1 && stride != 2))
     return fail(VL_EINVAL, "weight gradient: bad arguments");
@@ -668,7 +676,7 @@ int vl_nn_wgrad_bf16(const void* x, int B, int H, int W, int C, int stride, cons
     EpiParams ep{};
     ep.n_valid = N;
     ep.err = err;
-    ep.spin_limit = kSpinLimit;
+    test_timeout(ep, flags);
     return launch_wgrad_first(x, B, H, W, dz, N, kp, gwt, ep, (cudaStream_t)stream);
   }
   if (C < 32 || C % 32 || kp < 9 * C || N % 8 || ((uintptr_t)gwt & 31) || bw > 64 || 64 % bw || Ho % (64 / bw))
@@ -687,7 +695,7 @@ int vl_nn_wgrad_bf16(const void* x, int B, int H, int W, int C, int stride, cons
   p.ep.m_valid = kp;
   p.ep.n_valid = N;
   p.ep.err = err;
-  p.ep.spin_limit = kSpinLimit;
+  test_timeout(p.ep, flags);
   // The three taps of a row as one operand: for chunks of 32 channels (batch 16, 128 x 256 pixels: 32 x 32
   // 67 -> 43 us, 96 x 32 165 -> 79) and many chunks (64 x 128 192 x 64 77 -> 57, 32 x 64 384 x 128 57 -> 49); one or two
   // 64-channel chunks leave it too few blocks (64 x 64 27 -> 30, 128 x 128 23 -> 27), wide N too many dropped products
@@ -702,6 +710,23 @@ int vl_nn_wgrad_bf16(const void* x, int B, int H, int W, int C, int stride, cons
   if (rc) return rc;
   return kc == 64 ? launch_wgrad<64>(ta, tb, p, kp, N, gwt, (cudaStream_t)stream)
                   : launch_wgrad<32>(ta, tb, p, kp, N, gwt, (cudaStream_t)stream);
+}
+
+int vl_nn_dgrad2_bf16(const void* dz, int B, int H, int W, int C, int N, const void* wt, float* dx, int accumulate, int* err,
+                      void* stream) {
+  return dgrad2(dz, B, H, W, C, N, wt, dx, accumulate, err, stream, 0);
+}
+int vl_nn_dgrad2_test_timeout(const void* dz, int B, int H, int W, int C, int N, const void* wt, float* dx, int accumulate,
+                              int* err, void* stream) {
+  return dgrad2(dz, B, H, W, C, N, wt, dx, accumulate, err, stream, VL_GEMM_TEST_TIMEOUT);
+}
+int vl_nn_wgrad_bf16(const void* x, int B, int H, int W, int C, int stride, const void* dz, int N, float* gwt, int kp,
+                     int* err, void* stream) {
+  return wgrad(x, B, H, W, C, stride, dz, N, gwt, kp, err, stream, 0);
+}
+int vl_nn_wgrad_test_timeout(const void* x, int B, int H, int W, int C, int stride, const void* dz, int N, float* gwt, int kp,
+                             int* err, void* stream) {
+  return wgrad(x, B, H, W, C, stride, dz, N, gwt, kp, err, stream, VL_GEMM_TEST_TIMEOUT);
 }
 
 }  // extern "C"
