@@ -113,7 +113,8 @@ int workspace(int dev, size_t bytes, void** out) {
 // A thread's chain of loads is the time where the outputs are few, as they are where the splits are many: the values of
 // AHEAD splits are in flight, the next ones requested before these are added (2,048 outputs of 296 splits 23 us with a
 // wait for each 16, 17 with AHEAD 32, 10 with 64; 9,216 of about 150 10.6, 8.9, 5.9). Where the splits are few, 16 and
-// fewer registers (303,104 outputs and more: 10 us, 13 with 32).
+// fewer registers (303,104 outputs and more: 10 us, 13 with 32), and below 16 as few as there are, in larger blocks (GEMM
+// and reduction, us: 4608 x 512 of 4 splits 47.2 with 16 ahead, 42.7 with 4; 1024 x 1024 of 10 88.1, 84.2 with 8).
 template <int AHEAD>
 __global__ void k_split_reduce(const float* __restrict__ ws, int splits, int M, int N, float* __restrict__ out,
                                int ldc, int accumulate) {
@@ -155,10 +156,15 @@ __global__ void k_split_reduce(const float* __restrict__ ws, int splits, int M, 
 int split_reduce(const float* ws, int splits, int M, int N, float* out, int ldc, int accumulate, cudaStream_t s) {
   const long long total = (long long)M * N;
   const int blocks = (int)std::min<long long>((total + 63) / 64, 148 * 32);
+  const int wide = (int)std::min<long long>((total + 255) / 256, 148 * 8);
   if (splits >= 64)
     k_split_reduce<64><<<blocks, 64, 0, s>>>(ws, splits, M, N, out, ldc, accumulate);
-  else
+  else if (splits >= 16)
     k_split_reduce<16><<<blocks, 64, 0, s>>>(ws, splits, M, N, out, ldc, accumulate);
+  else if (splits >= 8)
+    k_split_reduce<8><<<wide, 256, 0, s>>>(ws, splits, M, N, out, ldc, accumulate);
+  else
+    k_split_reduce<4><<<wide, 256, 0, s>>>(ws, splits, M, N, out, ldc, accumulate);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? VL_OK : fail(VL_ECUDA, std::string("gemm split reduce: ") + cudaGetErrorString(e));
 }
