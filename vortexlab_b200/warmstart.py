@@ -147,7 +147,13 @@ class Conv:
         self.flip = self.k == 3 and self.stride == 1
         if self.flip:       # input gradient as a convolution of dz with mirrored weights
             self.kpf = _kp(9 * self.cout)
-            self.direct_x = self.cout % 32 == 0 and self.cin % 8 == 0
+            # Few pixels and a long contraction (9 cout) leave the direct kernel a few blocks with a serial chain of K
+            # steps, which the GEMM over the matrix splits over the chip. us of the backward pass, direct / matrix: 8 x 16
+            # pixels 64 <- 384 54 / 48, 64 <- 1024 93 / 46, 256 <- 512 69 / 63, 1024 <- 1024 142 / 106, 256 <- 384 60 / 62; 16 x 32
+            # 64 <- 512 64 / 51, 256 <- 1024 104 / 78, 1024 <- 640 96 / 118; 4 x 8 256 <- 512 69 / 73, 256 <- 640 75 / 71.
+            few = self.kpf // 64 >= (54 if self.cin <= 64 else 72 if self.cin <= 128 else 81) and \
+                self.rows <= 1024 and self.rows * self.cin <= 131072
+            self.direct_x = self.cout % 32 == 0 and self.cin % 8 == 0 and not few
             self.dcols = None
             self.wf = torch.zeros(self.cin, self.kpf, **bf)
         elif self.k == 3:   # stride 2: dz W^T gathered by parity of the pixel (or written out, then col2im)
