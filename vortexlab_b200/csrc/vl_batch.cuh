@@ -372,8 +372,14 @@ constexpr int batch_step_tiles() {
 // populations were complete before it began). 24 tunnels of 300 x 150 to 800 x 400 cells, microseconds a step: FP32 68.5
 // -> 59.5, FP64 115 -> 103, 16-bit 65 -> 58; two of 240 x 120 15.6 -> 14.9. Taking warp segments by a counter in memory
 // instead of by block was slower (71 to 92: one address takes an addition every few clocks).
-template <class S, int PAIRS>
-__global__ void __launch_bounds__(kBlock, PAIRS ? batch_pair_min_blocks<S>() : 4) k_batch_step(
+// FEW (FP64, at most kBatchFewTiles tiles): two blocks an SM in place of four, so that nothing of a link chunk is spilled
+// (164 bytes at 64 registers). Its chain is the step where the tiles are few, us a step, before this kernel / four blocks /
+// two: a tunnel of D = 15 14.1 / 15.5 / 13.4, of 60 31.4 / 32.8 / 29.7, two of 40 26.3 / 27.2 / 23.5, four of 15 to 40 (3,300
+// tiles) 26.8 / 28.2 / 25.3; with more the tiles want the other two: six of 15 to 40 (4,800) 38.3 / 37.1 / 40.3, 24 112 / 102 /
+// 141.
+constexpr int kBatchFewTiles = 3800;
+template <class S, int PAIRS, int FEW = 0>
+__global__ void __launch_bounds__(kBlock, PAIRS ? batch_pair_min_blocks<S>() : (FEW ? 2 : 4)) k_batch_step(
     const __grid_constant__ BatchParams p, const S* __restrict__ A, S* __restrict__ B, int nchunks) {
   const int k = (int)blockIdx.x - nchunks;
   if (k < 0) {

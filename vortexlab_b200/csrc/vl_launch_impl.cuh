@@ -207,7 +207,9 @@ struct LaunchImpl {
       c.attrs = &at;
       c.numAttrs = p.noutl > 0 ? 1 : 0;
       auto fn = k_batch_step<S, 0>;
-      if constexpr (!std::is_same<S, double>::value) {
+      if constexpr (std::is_same<S, double>::value) {
+        if (ntiles <= kBatchFewTiles) fn = k_batch_step<S, 0, 1>;
+      } else {
         if (pairs) fn = k_batch_step<S, 1>;
       }
       const cudaError_t e = cudaLaunchKernelEx(&c, fn, p, (const S*)a, (S*)b, nchunks);
