@@ -439,19 +439,18 @@ __device__ void record_probe(const StepParams& p, const S* a, long long tstep, c
 
 // Block-wide sum of `count` values spaced `stride` apart: thread t adds values t, t + kBlock, ...
 // in order, then a fixed shared-memory tree. The result is valid in thread 0. Every thread calls it.
-template <class Part = WholeBlock>
-__device__ __forceinline__ double sum_partials(const double* v, int count, int stride, double* red, Part part = Part()) {
-  const int tid = part.tid();
+__device__ __forceinline__ double sum_partials(const double* v, int count, int stride, double* red) {
+  const int tid = (int)threadIdx.x;
   double acc = 0.0;
   for (int k = tid; k < count; k += kBlock) acc += __ldcg(v + (size_t)k * stride);
   red[tid] = acc;
-  part.sync();
+  __syncthreads();
   for (int s = kBlock / 2; s > 0; s >>= 1) {
     if (tid < s) red[tid] += red[tid + s];
-    part.sync();
+    __syncthreads();
   }
   const double out = red[0];
-  part.sync();
+  __syncthreads();
   return out;
 }
 
@@ -764,8 +763,8 @@ __device__ __forceinline__ void force_terms(const LinkView& L, double o, double 
   ty = (double)cy_of(L.dir) * (o + bk) - wuy * (o - bk);
 }
 
-template <class S, int CG = 0, class Put>
-__device__ __forceinline__ void link_rules(const S* a, unsigned ns, const typename Store<S>::R* own,
+template <class S, class Put>
+__device__ __forceinline__ void link_rules(const S* __restrict__ a, unsigned ns, const typename Store<S>::R* own,
                                            int first, int last, const LinkRecDev* __restrict__ links,
                                            const double* vs, double drho, double gx_, double gy_, double sqrt_cs2,
                                            double* acc, Put put) {
@@ -776,7 +775,7 @@ __device__ __forceinline__ void link_rules(const S* a, unsigned ns, const typena
   for (int l = first; l < last; ++l) {
     const LinkView L = load_link(links, l);
     R out, scale;
-    const R bval = uses_behind(L) ? ldp<S, CG>(a + (unsigned)L.dir * ns + (unsigned)L.behind, L.dir) : R(0);
+    const R bval = uses_behind(L) ? Store<S>::ld(a + (unsigned)L.dir * ns + (unsigned)L.behind, L.dir) : R(0);
     const R back = link_back<S>(bval, L, own, vs, drho, gx, gy, sqrt_cs2, have_u, ux, uy, out, scale);
     put(l, opp_of(L.dir), back);
     if (L.fgroup >= 0) {
@@ -791,8 +790,8 @@ __device__ __forceinline__ void link_rules(const S* a, unsigned ns, const typena
 // The link pass for one boundary node (src/sim.rs:456-503): the incoming populations pulled from
 // the neighbours, each one that would come out of the boundary replaced by its link's rule, then
 // the collision. `f` returns the post-collision populations.
-template <class S, int CG = 0>
-__device__ __forceinline__ void link_node(const S* a, unsigned ns, int nx, int ny, int idx, int first,
+template <class S>
+__device__ __forceinline__ void link_node(const S* __restrict__ a, unsigned ns, int nx, int ny, int idx, int first,
                                           int last, const LinkRecDev* __restrict__ links, const double* vs,
                                           double drho, int ck, double op_, double om_, double gx_, double gy_,
                                           double sqrt_cs2, double* acc, typename Store<S>::R* f) {
@@ -800,27 +799,26 @@ __device__ __forceinline__ void link_node(const S* a, unsigned ns, int nx, int n
   const R op = (R)op_, om = (R)om_, gx = (R)gx_, gy = (R)gy_;
   const int y = idx / nx, x = idx - y * nx;
   R own[9];
-  pull<S, CG>(a, ns, nx, ny, x, y, f);
+  pull<S>(a, ns, nx, ny, x, y, f);
 #pragma unroll
-  for (int d = 0; d < 9; ++d) own[d] = ldp<S, CG>(a + (unsigned)d * ns + idx, d);
-  link_rules<S, CG>(a, ns, own, first, last, links, vs, drho, gx_, gy_, sqrt_cs2, acc,
+  for (int d = 0; d < 9; ++d) own[d] = Store<S>::ld(a + (unsigned)d * ns + idx, d);
+  link_rules<S>(a, ns, own, first, last, links, vs, drho, gx_, gy_, sqrt_cs2, acc,
                 [&](int, int i, R back) { set_dir(f, i, back); });
   collide_s<S>(f, ck, op, om, gx, gy);
 }
 
 // Block partial of the first `ncomp` force components: fixed shuffle tree within each warp, then
 // the warps in order. Written by threads 0..ncomp-1 to out[c]. Every thread calls it.
-template <class Part = WholeBlock>
 __device__ __forceinline__ void block_force_partial(const double (*s_acc)[kBlock], int ncomp, double* out,
-                                                    double (*s_red)[kBlock / 32], Part part = Part()) {
-  const int tid = part.tid(), lane = tid & 31, warp = tid >> 5;
+                                                    double (*s_red)[kBlock / 32]) {
+  const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int c = 0; c < ncomp; ++c) {
     double v = s_acc[c][tid];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
     if (lane == 0) s_red[c][warp] = v;
   }
-  part.sync();
+  __syncthreads();
   if (tid < ncomp) {
     double v = 0.0;
     for (int w = 0; w < kBlock / 32; ++w) v += s_red[tid][w];

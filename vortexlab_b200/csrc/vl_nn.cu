@@ -260,6 +260,17 @@ int vl_nn_gemm_bf16(const void* a, int lda, const void* b, int ldb, int M, int N
 // ------------------------------------------------------------------ implicit convolutions
 namespace {
 
+// The shared-memory limit of a kernel, set once a device (`configured`: the kernel's own).
+int smem_limit(const void* fn, int dev, int bytes, bool (&configured)[64], const char* what) {
+  static std::mutex m;
+  std::lock_guard<std::mutex> g(m);
+  if (dev < 64 && configured[dev]) return VL_OK;
+  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return fail(VL_ECUDA, std::string(what) + " smem attribute: " + cudaGetErrorString(e));
+  if (dev < 64) configured[dev] = true;
+  return VL_OK;
+}
+
 template <int KC>
 int launch_conv(const CUtensorMap& ta, const CUtensorMap& tb, vl::gemm::ConvParams& p, int N, cudaStream_t s) {
   using namespace vl::gemm;
@@ -271,16 +282,8 @@ int launch_conv(const CUtensorMap& ta, const CUtensorMap& tb, vl::gemm::ConvPara
   const int per_sm = 4 * p.tmem_cols <= 512 ? 2 : 1;
   p.stages = std::min(kConvMaxStages, (per_sm == 2 ? 104 * 1024 : 208 * 1024) / stage);
   const int smem = p.stages * stage + 1024;
-  static std::mutex m;
   static bool configured[64] = {};
-  {
-    std::lock_guard<std::mutex> g(m);
-    if (dev >= 64 || !configured[dev]) {
-      cudaError_t e = cudaFuncSetAttribute(k_conv<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024);
-      if (e != cudaSuccess) return fail(VL_ECUDA, std::string("convolution smem attribute: ") + cudaGetErrorString(e));
-      if (dev < 64) configured[dev] = true;
-    }
-  }
+  if (int rc = smem_limit((const void*)k_conv<KC>, dev, 210 * 1024, configured, "convolution")) return rc;
   const int gy = (N + p.bn - 1) / p.bn;
   const int gx = std::max(1, std::min(p.tiles, per_sm * sm_count(dev) / gy));
   k_conv<KC><<<dim3((unsigned)gx, (unsigned)gy), kConvThreads, smem, s>>>(ta, tb, p);
@@ -402,16 +405,8 @@ int launch_wgrad_rows(const void* x, int B, int H, int W, int C, const void* dz,
   if (rc) return rc;
   rc = make_map(&tb, dz, (uint64_t)B * H * W, (uint64_t)N, (uint64_t)N, 64u, p.bn == 32 ? 32 : 64);
   if (rc) return rc;
-  static std::mutex m;
   static bool configured[64] = {};
-  {
-    std::lock_guard<std::mutex> g(m);
-    if (dev >= 64 || !configured[dev]) {
-      cudaError_t e = cudaFuncSetAttribute(k_wgrad_rows<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 104 * 1024);
-      if (e != cudaSuccess) return fail(VL_ECUDA, std::string("weight gradient smem attribute: ") + cudaGetErrorString(e));
-      if (dev < 64) configured[dev] = true;
-    }
-  }
+  if (int rc = smem_limit((const void*)k_wgrad_rows<KC>, dev, 104 * 1024, configured, "weight gradient")) return rc;
   const int gy = (N + p.bn - 1) / p.bn;
   k_wgrad_rows<KC><<<dim3((unsigned)(3 * p.chunks), (unsigned)gy, (unsigned)splits), 128, p.stages * p.stage_bytes + 1024, s>>>(ta, tb, p);
   cudaError_t e = cudaGetLastError();
@@ -431,16 +426,8 @@ int launch_wgrad(const CUtensorMap& ta, const CUtensorMap& tb, vl::gemm::WgradPa
   if (rc) return rc;
   const int stage = wgrad_stage_bytes<KC>(p.bn);
   p.stages = std::min(kConvMaxStages, 100 * 1024 / stage);
-  static std::mutex m;
   static bool configured[64] = {};
-  {
-    std::lock_guard<std::mutex> g(m);
-    if (dev >= 64 || !configured[dev]) {
-      cudaError_t e = cudaFuncSetAttribute(k_wgrad<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 104 * 1024);
-      if (e != cudaSuccess) return fail(VL_ECUDA, std::string("weight gradient smem attribute: ") + cudaGetErrorString(e));
-      if (dev < 64) configured[dev] = true;
-    }
-  }
+  if (int rc = smem_limit((const void*)k_wgrad<KC>, dev, 104 * 1024, configured, "weight gradient")) return rc;
   k_wgrad<KC><<<dim3((unsigned)gx, (unsigned)gy, (unsigned)splits), 128, p.stages * stage + 1024, s>>>(ta, tb, p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(VL_ECUDA, std::string("weight gradient launch: ") + cudaGetErrorString(e));
@@ -454,12 +441,12 @@ int launch_dgrad2(const CUtensorMap& ta, const CUtensorMap& tb, vl::gemm::Dgrad2
   cudaGetDevice(&dev);
   constexpr int kStage = conv_stage_bytes<KC>(BN), kStages = std::min(kConvMaxStages, 104 * 1024 / kStage);
   p.stages = kStages;
-  cudaError_t e = cudaFuncSetAttribute(k_dgrad2<KC, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStages * kStage + 1024);
-  if (e != cudaSuccess) return fail(VL_ECUDA, std::string("input gradient smem attribute: ") + cudaGetErrorString(e));
+  static bool configured[64] = {};
+  if (int rc = smem_limit((const void*)k_dgrad2<KC, BN>, dev, kStages * kStage + 1024, configured, "input gradient")) return rc;
   const int gy = (p.n_valid + BN - 1) / BN;
   const int gx = std::max(1, std::min(p.units, 2 * sm_count(dev) / gy));
   k_dgrad2<KC, BN><<<dim3((unsigned)gx, (unsigned)gy), kConvThreads, kStages * kStage + 1024, s>>>(ta, tb, p);
-  e = cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? VL_OK : fail(VL_ECUDA, std::string("input gradient launch: ") + cudaGetErrorString(e));
 }
 
@@ -490,11 +477,11 @@ int launch_conv_first(const void* x, int B, int H, int W, const void* w, int kp,
   int rc = make_map(&tb, w, (uint64_t)N, (uint64_t)kp, (uint64_t)kp, (uint32_t)p.bn);
   if (rc) return rc;
   const int smem = kFirstStages * 16384 + p.bn * 128 + 1024, most = kFirstStages * 16384 + 256 * 128 + 1024;
-  cudaError_t e = cudaFuncSetAttribute(k_conv_first, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  if (e != cudaSuccess) return fail(VL_ECUDA, std::string("convolution smem attribute: ") + cudaGetErrorString(e));
+  static bool configured[64] = {};
+  if (int rc = smem_limit((const void*)k_conv_first, dev, most, configured, "convolution")) return rc;
   const int per_sm = p.bn <= 128 ? 2 : 1;
   k_conv_first<<<(unsigned)std::min(p.tiles, per_sm * sm_count(dev)), 288, smem, s>>>(tb, p);
-  e = cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? VL_OK : fail(VL_ECUDA, std::string("convolution launch: ") + cudaGetErrorString(e));
 }
 
@@ -520,10 +507,10 @@ int launch_wgrad_first(const void* x, int B, int H, int W, const void* dz, int N
   rc = make_map(&tb, dz, (uint64_t)p.pixels, (uint64_t)N, (uint64_t)N, 64u);
   if (rc) return rc;
   const int smem = kFirstStages * (8192 + p.bn * 128) + 1024, most = kFirstStages * (8192 + 256 * 128) + 1024;
-  cudaError_t e = cudaFuncSetAttribute(k_wgrad_first, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  if (e != cudaSuccess) return fail(VL_ECUDA, std::string("weight gradient smem attribute: ") + cudaGetErrorString(e));
+  static bool configured[64] = {};
+  if (int rc = smem_limit((const void*)k_wgrad_first, dev, most, configured, "weight gradient")) return rc;
   k_wgrad_first<<<(unsigned)splits, 160, smem, s>>>(tb, p);
-  e = cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(VL_ECUDA, std::string("weight gradient launch: ") + cudaGetErrorString(e));
   return splits > 1 ? split_reduce((const float*)p.ep.out, splits, kp, N, out, N, 0, s) : VL_OK;
 }

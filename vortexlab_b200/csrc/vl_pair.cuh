@@ -250,10 +250,7 @@ struct PairTask {
   int* bad;
   unsigned long long* bad_t;
   const unsigned long long* t_now;
-  // shared-memory sources (bulk-copy fed kernel): plane i of the row is at stage + i * seg, its
-  // element 0 holding cell x0t - halo
-  const void* stage;
-  int seg, x0t, halo;
+  int x0t;                      // first cell of the tile (bulk-copy fed kernel)
 };
 
 // The pull of plane i for the thread's group from the source row `src`.

@@ -349,8 +349,6 @@ __global__ void __launch_bounds__(stream::kThreads, 2) k_bulk_stream(const __gri
     t.bad = &p.ctl->nonfinite;
     t.bad_t = &p.ctl->nonfinite_t;
     t.t_now = &p.ctl->t;
-    t.seg = G::SEG;
-    t.halo = G::H;
     long long j = 0;
     for (long long u = blockIdx.x; u < units; u += gridDim.x, ++j) {
       const int s = (int)(j % stream::kStages);
