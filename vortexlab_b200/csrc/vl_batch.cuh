@@ -369,8 +369,8 @@ constexpr int batch_step_tiles() {
 // A step's link chunks and tiles in one launch, instead of two kernels on forked streams: the link chunks are a long
 // chain of dependent loads (28 us beside the tiles) and have the first nchunks blocks, so it ends under the tiles. Only
 // they wait for k_batch_outlet, which lets this kernel start beside it (the tiles read nothing that it writes; their
-// populations were complete before it began). 24 tunnels of 300 x 150 to 800 x 400 cells, microseconds a step: FP32 68.5
-// -> 59.5, FP64 115 -> 103, 16-bit 65 -> 58; two of 240 x 120 15.6 -> 14.9. Taking warp segments by a counter in memory
+// populations were complete before it began). 24 tunnels of 300 x 150 to 800 x 400 cells, microseconds a step: FP32 66
+// -> 58, FP64 112 -> 102, 16-bit 64 -> 56; two of 240 x 120 15.8 -> 15.2; 64 of 300 x 150 to 1200 x 600 (FP32) 284 -> 281. Taking warp segments by a counter in memory
 // instead of by block was slower (71 to 92: one address takes an addition every few clocks).
 // FEW (FP64, at most kBatchFewTiles tiles): two blocks an SM in place of four, so that nothing of a link chunk is spilled
 // (164 bytes at 64 registers). Its chain is the step where the tiles are few, us a step, before this kernel / four blocks /
