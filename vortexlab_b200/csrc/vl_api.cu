@@ -160,11 +160,11 @@ bool vl::InFlight::many_others(const Work* w) {
         o->queued = false;
         continue;
       }
+      cudaGetLastError();                                       // (the query's own "not ready")
     }
     if ((n += o->weight) >= Work::kMany) break;
   }
   cudaThreadExchangeStreamCaptureMode(&mode);
-  cudaGetLastError();
   return n >= Work::kMany;
 }
 
