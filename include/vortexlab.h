@@ -223,8 +223,9 @@ int vl_sim_step_profiled(vl_sim* s, uint64_t steps, double* link_ms, double* bul
  * bulk update, beside the outlet offsets.
  * Until a schedule is chosen here, calls of a few steps and more on a small domain (its populations stay
  * in the L2) run in one kernel that takes all the steps of the call, with the same results; so they do
- * after vl_sim_autotune, which then decides for the other calls. Not while a batch or three more sims of the process
- * have work in flight on the device: that kernel takes most of its SMs, and the two-kernel steps overlap. */
+ * after vl_sim_autotune, which then decides for the other calls. Not while a batch, or (below
+ * 200,000 cells) three more sims of the process have work in flight on the device: that kernel takes most of its SMs,
+ * and the two-kernel steps overlap. */
 enum { VL_SCHEDULE_CONCURRENT = 0, VL_SCHEDULE_LINKS_FIRST = 1, VL_SCHEDULE_BULK_FIRST = 2, VL_SCHEDULE_STAGED = 3,
        VL_SCHEDULE_COUNT = 4 };
 int vl_sim_set_schedule(vl_sim* s, int schedule);

@@ -1,5 +1,5 @@
-"""The resident step kernel takes most of the device for a call, so a sim leaves it alone while a batch or three
-more sims have work in flight: their two-kernel steps overlap. The results are the same."""
+"""The resident step kernel takes most of the device for a call, so a sim leaves it alone while a batch or (a small
+sim) three more sims have work in flight: their two-kernel steps overlap. The results are the same."""
 import threading
 
 import numpy as np
@@ -43,6 +43,19 @@ def test_fourth_sim_takes_the_two_kernel_step(gpu):
         s.synchronize()
     assert _launches(c, 64) == 1                                    # none any more
     assert np.array_equal(c.populations(), ref.populations())
+
+
+def test_larger_sim_stays(gpu):
+    small = [_tank(), _tank("f32"), _tank()]
+    big = S.product_sim(S.tunnel_like(nx=702, ny=302, radiating=True))
+    big.init((1.0, 0.02, 0.0))
+    big.vscale[1], big.vscale[2] = 0.5, 0.002
+    for s in small + [big]:
+        s.step(64)
+        s.synchronize()
+    for s in small:
+        assert _launches(s, LONG) < 20
+    assert _launches(big, 64) == 1
 
 
 def test_sim_beside_a_batch(gpu):

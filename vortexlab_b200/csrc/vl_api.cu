@@ -146,14 +146,14 @@ void vl::InFlight::finish(Work* w) {
   --w->calls;
   w->queued = true;
 }
-bool vl::InFlight::many_others(const Work* w) {
+bool vl::InFlight::many_others(const Work* w, bool batches) {
   std::lock_guard<std::mutex> guard(m_);
   // (the query must not end a stream capture that another thread has under way)
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   cudaThreadExchangeStreamCaptureMode(&mode);
   int n = 0;
   for (Work* o : all_) {
-    if (o == w || o->device != w->device) continue;
+    if (o == w || o->device != w->device || (batches && o->weight < Work::kMany)) continue;
     if (o->calls == 0) {
       if (!o->queued) continue;
       if (cudaEventQuery(o->end) != cudaErrorNotReady) {
@@ -574,7 +574,7 @@ struct vl_sim {
     vl::InFlightCall call(&work);
     uint64_t left = steps;
     if (resident && resident_ok && !P.stream && steps >= (uint64_t)kResidentMinSteps &&
-        !vl::InFlight::of_process().many_others(&work)) {
+        !vl::InFlight::of_process().many_others(&work, n >= vl::kOverlapCells)) {
       if (int rc = step_resident(left, test)) return rc;
       if (left == 0) {
         VL_CUDA(cudaEventRecord(ev1, stream));
