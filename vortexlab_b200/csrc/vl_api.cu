@@ -503,10 +503,9 @@ struct vl_sim {
     const int per_row = (P.nx + 32 * v - 1) / (32 * v);
     const long long nseg = (long long)per_row * P.ny;
     const int G = RP.grid;
-    RP.tables = 0;
-    if (L->resident_blocks(P, RP, ck, sms) < G || nseg > 0x7fffffff) { resident_ok = false; return VL_OK; }
     RP.tables = 1;
     if (L->resident_blocks(P, RP, ck, sms) < G) RP.tables = 0;   // too many for the shared memory
+    if ((!RP.tables && L->resident_blocks(P, RP, ck, sms) < G) || nseg > 0x7fffffff) { resident_ok = false; return VL_OK; }
     // Segments that a task, an outlet node's place in the serial sum, the force sums and a chunk of them
     // stand for (a segment is about 150 cycles of a block). Half and twice these move a step by 3 % at
     // most on tunnels of D = 24, 37 and 60 and the rig at 20 and 80 cells per diameter.

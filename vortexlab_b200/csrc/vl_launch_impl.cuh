@@ -126,16 +126,17 @@ struct LaunchImpl {
     const int v = ck == 0 ? group_width<0>(p) : (ck == 1 ? group_width<1>(p) : group_width<2>(p));
     return v < 2 ? v : 2;
   }
+  static size_t resident_base_bytes(const StepParams& p, const ResidentParams& r) {
+    return (size_t)((p.np + 1) / 2 * 2) * sizeof(double) + (size_t)r.max_tasks * sizeof(TaskScratch<typename Store<S>::R>);
+  }
   static size_t resident_bytes(const StepParams& p, const ResidentParams& r) {
-    const size_t base =
-        (size_t)((p.np + 1) / 2 * 2) * sizeof(double) + (size_t)r.max_tasks * sizeof(TaskScratch<typename Store<S>::R>);
-    return r.tables ? base + resident_table_bytes(r) : base;
+    return resident_base_bytes(p, r) + (r.tables ? resident_table_bytes(r) : 0);
   }
   // Blocks of the kernel that fit the device at once (0: it cannot run).
   static int resident_blocks(const StepParams& p, const ResidentParams& r, int ck, int sms) {
     const void* fn = (const void*)resident_fn(p, ck);
     int per = 0;
-    if (resident_bytes(p, r) > (size_t)(r.tables ? kResidentSmemTables : kResidentSmem) ||
+    if (resident_base_bytes(p, r) > (size_t)kResidentSmem || resident_bytes(p, r) > (size_t)kResidentSmemTables ||
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidentSmemTables) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kResidentThreads, resident_bytes(p, r)) != cudaSuccess) {
       cudaGetLastError();
