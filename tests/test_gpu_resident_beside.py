@@ -27,21 +27,24 @@ def _launches(sim, steps):
 
 def test_fourth_sim_takes_the_two_kernel_step(gpu):
     a, b, e, c = _tank(), _tank("f32"), _tank(), _tank()
+    for s in (a, b, e, c):      # (a kernel's first launch may wait for the device)
+        assert _launches(s, 64) == 1
+        s.synchronize()
+    steps = 64
+    for _ in range(5):          # (a host that is held up for as long as the others take may miss them)
+        for s in (a, b, e):
+            assert _launches(s, LONG) < 20                          # two others in flight at most: still resident
+        n = _launches(c, 64)                                        # three others
+        steps += 64
+        for s in (a, b, e, c):
+            s.synchronize()
+        if n > 60:
+            break
+    assert n > 60
+    assert _launches(c, 64) == 1                                    # none any more
     ref = _tank()
     ref.schedule = "concurrent"
-    ref.step(3 * 64)
-    ref.synchronize()
-    assert _launches(c, 64) == 1
-    for s in (a, b, e, c):      # (a kernel's first launch may wait for the device)
-        if s is not c:
-            s.step(64)
-        s.synchronize()
-    for s in (a, b, e):
-        assert _launches(s, LONG) < 20                              # two others in flight at most: still resident
-    assert _launches(c, 64) > 60                                    # three others
-    for s in (a, b, e, c):
-        s.synchronize()
-    assert _launches(c, 64) == 1                                    # none any more
+    ref.step(steps + 64)
     assert np.array_equal(c.populations(), ref.populations())
 
 
@@ -66,10 +69,14 @@ def test_sim_beside_a_batch(gpu):
         b.add(t.tunnel.spec_warm(t.body), t.steps)
     b.build()
     sim = _tank()
-    b.run_async(8000)
-    assert _launches(sim, 64) > 60
-    b.wait()
-    sim.synchronize()
+    for _ in range(5):
+        b.run_async(2000)
+        n = _launches(sim, 64)
+        b.wait()
+        sim.synchronize()
+        if n > 60:
+            break
+    assert n > 60
     assert _launches(sim, 64) == 1
     del b
     assert _launches(sim, 64) == 1
