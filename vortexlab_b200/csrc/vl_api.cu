@@ -819,7 +819,11 @@ vl::LinkRecDev device_link(const vl::LinkRec& h) {
 // of disks, FP64, with force on 29 chunks 640 x 400 10.6 / 12.8, 300 x 200 9.9 / 11.2; on 34 1000 x 600
 // 18.1 / 17.2; on 46 640 x 400 14.7 / 13.2; on 151 45 / 15.6. With an outlet on 39 300 x 200 13.2 / 14.9, on
 // 62 1000 x 600 25.9 / 27.4, on 72 640 x 400 21.9 / 20.1. So: at most 30 chunks with force times groups, 45 with
-// an outlet. Besides, no outlet node may have a link with a force group (its task forms no force terms), at
+// an outlet. A periodic box without a boundary node leaves the link kernel nothing to do, and two kernels are the
+// faster form (50 x 50 FP64 and FP32 3.9 / 3.0, 5000 x 100 11.1 / 8.5, 801 x 799 15.8 / 12.6, FP32 10.2 / 8.6) but where many
+// rows are short for the tiles of the bulk kernel, 256 cells times the cells a thread: FP64 33 x 9000 11.8 / 10.2, 16 x
+// 20000 11.4 / 14.7, 3 x 50000 24.5 / 42.1; FP32 (two cells) 100 x 4000 7.6 / 8.2; 16-bit (four) 100 x 4000 7.8 / 16.8.
+// Besides, no outlet node may have a link with a force group (its task forms no force terms), at
 // most kBlock chunks of boundary nodes (the force sums' shared memory).
 int resident_setup(vl_sim& s) {
   const vl::CompiledDomain& d = s.dom;
@@ -827,6 +831,11 @@ int resident_setup(vl_sim& s) {
   if (bytes > ((size_t)128 << 20) || d.n > (d.pnode_idx.empty() ? (size_t)640000 : (size_t)1700000) || s.P.nlink > vl::kBlock)
     return VL_OK;
   const size_t nb = d.bnode_idx.size(), np = d.pnode_idx.size();
+  if (nb == 0) {
+    const int v = s.prec == VL_F64 || d.nx % 2 ? 1 : (d.nx % 4 == 0 && s.P.pairs >= 4 ? 4 : 2);
+    const bool strip = v > 1 && d.ny >= 2000 && 5 * d.nx < (size_t)(v * vl::kBlock);
+    if (d.nx >= 32 && !strip) return VL_OK;
+  }
   std::vector<int32_t> outlet_of(nb, -1);
   std::vector<size_t> order, open, outlet_nodes(np);
   for (size_t k = 0; k < np; ++k) {
