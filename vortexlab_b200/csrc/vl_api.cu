@@ -823,7 +823,11 @@ vl::LinkRecDev device_link(const vl::LinkRec& h) {
 // faster form (50 x 50 FP64 and FP32 3.9 / 3.0, 5000 x 100 11.1 / 8.5, 801 x 799 15.8 / 12.6, FP32 10.2 / 8.6) but where many
 // rows are short for the tiles of the bulk kernel, 256 cells times the cells a thread: FP64 33 x 9000 11.8 / 10.2, 16 x
 // 20000 11.4 / 14.7, 3 x 50000 24.5 / 42.1; FP32 (two cells) 100 x 4000 7.6 / 8.2; 16-bit (four) 100 x 4000 7.8 / 16.8.
-// Besides, no outlet node may have a link with a force group (its task forms no force terms), at
+// Without force and with few boundary nodes the link kernel is short too. One disk in a box 600 x 500 FP64 7.7 / 8.4,
+// FP32 6.4 / 7.4, 800 x 799 14.6 / 12.5 and 8.9 / 8.2; a cavity (3,200 nodes) 800 x 799 14.2 / 15.4 and 9.2 / 10.7; a
+// channel driven by a body force, whose collision is the longer one for the resident kernel's 64 registers, 400 x 400
+// 6.4 / 8.2 and 5.1 / 7.9, 600 x 500 8.7 / 7.6 and 6.6 / 7.2 (16-bit 7.7 / 7.5), 800 x 799 16.8 / 13.2 and 10.8 / 10.0. So
+// there: at most 0.4 M cells, with a body force 0.25 M (FP32 0.4 M). Besides, no outlet node may have a link with a force group (its task forms no force terms), at
 // most kBlock chunks of boundary nodes (the force sums' shared memory).
 int resident_setup(vl_sim& s) {
   const vl::CompiledDomain& d = s.dom;
@@ -859,6 +863,10 @@ int resident_setup(vl_sim& s) {
   for (size_t c = 0; c < chunk_force.size(); ++c)
     if (chunk_force[c]) force_chunks.push_back((int32_t)c);
   if (force_chunks.size() * (size_t)d.ngroups > (np > 0 ? 45u : 30u)) return VL_OK;
+  if (nb > 0 && np == 0 && force_chunks.empty()) {
+    const size_t most = s.P.forced ? (s.prec == VL_F32 ? 400000 : 250000) : (nb < 3000 ? 400000 : 640000);
+    if (d.n > most) return VL_OK;
+  }
   int sms = 0;
   VL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s.device));
   if (sms < 2) return VL_OK;
